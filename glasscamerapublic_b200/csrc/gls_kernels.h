@@ -100,8 +100,6 @@ __host__ __device__ inline int pca_cov_group(int chunks) {
 int pca_cov_chunks(int w, int h);  // 64-patch chunks of a level
 int pca_cov_rows(int w, int h);    // partial rows of a level: chunks / pca_cov_group(chunks), rounded up
 
-template <class S, int C>
-void launch_downsample(Plane<S, C> in, Plane<S, C> out, cudaStream_t s);
 // a level's image and gradient in one launch (equal sizes)
 template <class S>
 void launch_downsample_pair(Plane<S, 4> img, Plane<S, 4> img_out, Plane<S, 2> grad, Plane<S, 2> grad_out,

@@ -62,13 +62,6 @@ __device__ __forceinline__ void downsample_px(const Plane<S, C>& in, const Plane
     }
 }
 
-template <class S, int C>
-__global__ void __launch_bounds__(256) k_downsample(Plane<S, C> in, Plane<S, C> out, float rx, float ry) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= out.w || y >= out.h) return;
-    downsample_px<S, C>(in, out, rx, ry, x, y);
-}
-
 // The image and the gradient of a pyramid level in one launch (same sizes,
 // same sample positions): PyramidProcessor::denoise's two downsamples
 // (pyramid_processor.cpp:109-110).
@@ -146,13 +139,6 @@ __global__ void __launch_bounds__(256) k_pca_project(Plane<S, 4> img, const floa
 
 // ------------------------------------------------------------------ launchers
 static inline dim3 grid2(int w, int h, dim3 b) { return dim3((w + b.x - 1) / b.x, (h + b.y - 1) / b.y); }
-
-template <class S, int C>
-void launch_downsample(Plane<S, C> in, Plane<S, C> out, cudaStream_t s) {
-    dim3 b(32, 8);
-    k_downsample<S, C><<<grid2(out.w, out.h, b), b, 0, s>>>(in, out, float(in.w) / float(out.w),
-                                                            float(in.h) / float(out.h));
-}
 
 template <class S>
 void launch_downsample_pair(Plane<S, 4> img, Plane<S, 4> img_out, Plane<S, 2> grad, Plane<S, 2> grad_out,
@@ -279,8 +265,6 @@ void host_pca_basis(const double* part, int n_blocks, int n_patches, float* basi
 }
 
 #define GLS_INST(S)                                                                                              \
-    template void launch_downsample<S, 4>(Plane<S, 4>, Plane<S, 4>, cudaStream_t);                              \
-    template void launch_downsample<S, 2>(Plane<S, 2>, Plane<S, 2>, cudaStream_t);                              \
     template void launch_downsample_pair<S>(Plane<S, 4>, Plane<S, 4>, Plane<S, 2>, Plane<S, 2>, cudaStream_t);  \
     template void launch_subtract_noise<S>(Plane<S, 4>, Plane<S, 4>, Plane<S, 4>, Plane<S, 2>, Plane<S, 4>,     \
                                            const SubtractArgs&, cudaStream_t);                                   \

@@ -31,6 +31,7 @@
 #include "gls_common.cuh"
 #include "gls_devbuf.h"
 #include "gls_fmath.h"
+#include "gls_warp.cuh"
 
 namespace gls {
 
@@ -1261,57 +1262,13 @@ struct WarpArgs {
     int count;  // 0: registerImage
 };
 
-template <class S>
-__device__ __forceinline__ float4 rd4(const S* p) {
-    if constexpr (std::is_same<S, float>::value) {
-        return __ldg(reinterpret_cast<const float4*>(p));
-    } else {
-        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-        return make_float4(a.x, a.y, b.x, b.y);
-    }
-}
-
-__device__ __forceinline__ float lerp_(float a, float b, float t) { return fadd(a, fmul(t, fsub(b, a))); }
-
 // registerAndFuse / registerImage (SURF.metal:489-538): pull-warp by H with
 // exact bilinear sampling, clamp-to-edge, and the running mean.
 template <class S>
 __global__ void __launch_bounds__(256) k_register(WarpArgs a) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= a.w || y >= a.h) return;
-    const float fx = float(x), fy = float(y);
-    const float u = fadd(fadd(fmul(a.H[0], fx), fmul(a.H[1], fy)), a.H[2]);
-    const float v = fadd(fadd(fmul(a.H[3], fx), fmul(a.H[4], fy)), a.H[5]);
-    const float ww = fadd(fadd(fmul(a.H[6], fx), fmul(a.H[7], fy)), a.H[8]);
-    const float xx = fminf(fmaxf(fdiv(u, ww), -1.0f), float(a.iw));
-    const float yy = fminf(fmaxf(fdiv(v, ww), -1.0f), float(a.ih));
-    const float x0f = floorf(xx), y0f = floorf(yy);
-    const float ax = fsub(xx, x0f), ay = fsub(yy, y0f);
-    const int x0 = int(x0f), y0 = int(y0f);
-    const int xa = min(max(x0, 0), a.iw - 1), xb = min(max(x0 + 1, 0), a.iw - 1);
-    const int ya = min(max(y0, 0), a.ih - 1), yb = min(max(y0 + 1, 0), a.ih - 1);
-    const S* in = reinterpret_cast<const S*>(a.input);
-    const float4 p00 = rd4(in + size_t(ya) * a.in_pitch + 4 * xa), p10 = rd4(in + size_t(ya) * a.in_pitch + 4 * xb);
-    const float4 p01 = rd4(in + size_t(yb) * a.in_pitch + 4 * xa), p11 = rd4(in + size_t(yb) * a.in_pitch + 4 * xb);
-    float4 s;
-    {
-        const float t = lerp_(p00.x, p10.x, ax), b = lerp_(p01.x, p11.x, ax);
-        s.x = lerp_(t, b, ay);
-    }
-    {
-        const float t = lerp_(p00.y, p10.y, ax), b = lerp_(p01.y, p11.y, ax);
-        s.y = lerp_(t, b, ay);
-    }
-    {
-        const float t = lerp_(p00.z, p10.z, ax), b = lerp_(p01.z, p11.z, ax);
-        s.z = lerp_(t, b, ay);
-    }
-    {
-        const float t = lerp_(p00.w, p10.w, ax), b = lerp_(p01.w, p11.w, ax);
-        s.w = lerp_(t, b, ay);
-    }
+    float4 s = warp_sample(reinterpret_cast<const S*>(a.input), a.in_pitch, warp_pos(a.H, x, y, a.iw, a.ih));
     float4* o = reinterpret_cast<float4*>(a.out + size_t(y) * a.out_pitch + 4 * x);
     if (a.count > 0) {
         const float4 f = *reinterpret_cast<const float4*>(a.fused + size_t(y) * a.fused_pitch + 4 * x);

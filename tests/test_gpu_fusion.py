@@ -131,3 +131,51 @@ def test_robust_weights_reject_an_outlier_frame(ctx):
     e_flat = np.abs(flat.cpu().numpy()[region] - frames[0][region]).mean()
     e_rob = np.abs(robust.cpu().numpy()[region] - frames[0][region]).mean()
     assert e_rob < 0.2 * e_flat, (e_rob, e_flat)
+
+
+@pytest.mark.parametrize("n,w,h,levels,out_dtype,overlap", [
+    (1, 64, 48, 3, torch.float32, False),    # the reference alone
+    (8, 97, 65, 3, torch.float32, False),    # one full group, ragged sizes
+    (9, 96, 64, 4, torch.float32, False),    # the first frame of a second group
+    (17, 70, 50, 2, torch.float16, False),   # three groups, FP16 output
+    (3, 31, 33, 2, torch.float32, False),    # level ratio 31 / 15
+    (3, 33, 32, 2, torch.float32, False),    # level ratio 33 / 16
+    (4, 96, 64, 3, torch.float32, True),     # the output is one of the input frames
+    (2, 40, 40, 1, torch.float32, False),    # no pyramid
+])
+def test_fusion_groups_and_edges(ctx, n, w, h, levels, out_dtype, overlap):
+    frames, Hs = _frames(n, w, h, seed=3)
+    ref = _numpy_fusion(_warped(frames, Hs), levels, 60.0)
+    t = [torch.from_numpy(f).cuda() for f in frames]
+    t[n // 2] = t[n // 2] if overlap or n == 1 else t[n // 2].half()  # one FP16 frame among FP32 ones
+    if t[n // 2].dtype == torch.float16:
+        frames[n // 2] = t[n // 2].float().cpu().numpy()
+        ref = _numpy_fusion(_warped(frames, Hs), levels, 60.0)
+    out = t[1] if overlap else torch.empty((h, w, 4), dtype=out_dtype, device="cuda")
+    fuse_pyramid(ctx, t, Hs, out, levels=levels, robustness=60.0)
+    torch.cuda.synchronize()
+    got = out.float().cpu().numpy()
+    # 1e-4 as above; an FP16 result of magnitude below 2 adds half an ulp, 2^-11
+    assert np.abs(got[..., :3] - ref).max() < 1e-4 + (2 ** -11 if out_dtype == torch.float16 else 0.0)
+    assert (got[..., 3] == 0).all()
+
+
+@pytest.mark.parametrize("H", [
+    [[1, 0, 0.5], [0, 1, -0.25], [0.01, 0, 0.02]],      # the denominator starts near zero
+    [[1, 0, 0], [0, 1, 0], [-0.04, 0.01, 1]],           # a vanishing line through the image
+    [[0, 0, -50], [0, 0, 500], [0, 0, 1]],              # every sample beyond an edge
+    [[1e-3, 0, 12.3], [0, 1e-3, 7.9], [0, 0, 1e-3]],    # a small common scale
+])
+@pytest.mark.parametrize("iw,ih", [(40, 30), (1, 30), (40, 1)])
+def test_fusion_warps_any_homography_and_frame_size(ctx, H, iw, ih):
+    """The fused warp against registerImage (no pyramid: the flat mean)."""
+    rng = np.random.default_rng(7)
+    ref = torch.from_numpy(rng.random((33, 50, 4), np.float32)).cuda()
+    frm = torch.from_numpy(rng.random((ih, iw, 4), np.float32)).cuda()
+    H = np.array(H, np.float32)
+    warped, out = torch.empty_like(ref), torch.empty_like(ref)
+    register_image(frm, warped, H)
+    fuse_pyramid(ctx, [ref, frm], [np.eye(3, dtype=np.float32), H], out, levels=1, robustness=0.0)
+    torch.cuda.synchronize()
+    # positions agree to an ulp (2^-19 at 40 texels, slope up to 1), each lerp to 2^-24
+    assert (out - (ref + warped) / 2)[..., :3].abs().max().item() < 4e-6
