@@ -609,108 +609,204 @@ struct MatchJobs {
     MatchJob j[kMaxJobs];
 };
 
-// matchKeyPoints (SURF.metal:441-487): 24 lanes per query scan the train
-// descriptors j = lane, lane + 24, ...; the L2 norm accumulates in four
-// float lanes (SURF.metal:423-431). One warp per query.
-__global__ void __launch_bounds__(128) k_match(MatchJobs jobs, int cap, gls_match* __restrict__ out_all) {
+// matchKeyPoints (SURF.metal:441-487): the reference scans the train
+// descriptors in 24 lanes, j = lane, lane + 24, ..., each keeping its first
+// smallest distance, and takes the lanes in order, strictly smaller wins: the
+// minimum over (distance, j mod 24, j). The distance is the square root of
+// four float lane sums (SURF.metal:423-431), each in component order.
+//
+// Here a block of 256 threads takes 64 queries and a share of the train set,
+// 64 at a time staged in shared memory, and a thread 4 x 4 pairs: every
+// staged component serves four pairs from registers. Components travel as
+// packed FP32 pairs (two lane sums an instruction; the train values are
+// staged negated, q + (-t) rounds as q - t). The pair keys, distance bits
+// over (j mod 24, j), are reduced by shuffles and one 64-bit atomic minimum
+// per query and block, so the train set can be split over blocks. Bound by
+// the FP32 pipe's subtract, multiply and add (the reference's roundings
+// leave no FMA; 80% busy): 0.25 ms for 14 jobs of 1500 x 1500, 2.11 ms with a
+// warp per query that read whole descriptors per lane.
+typedef unsigned long long u64;
+constexpr int MT = 64, MT_PAD = MT + 1;  // tile edge; padded so that staging stores and reads are conflict-free
+constexpr u64 kOne2 = 0x3f8000003f800000ull;  // (1, 1)
+constexpr u64 kNoMatch = ~0ull;          // no distance below FLT_MAX: reported as train 0 at FLT_MAX
+
+struct MatchSmem {
+    float4 q[16][MT_PAD], t[16][MT_PAD];  // component group, descriptor
+};
+
+__device__ __forceinline__ u64 add_f32x2(u64 a, u64 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 mul_f32x2(u64 a, u64 b) {
+    u64 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 fma_f32x2(u64 a, u64 b, u64 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float2 unpack_f32x2(u64 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+
+// descriptors [first, first + 64) of n, negated if NEG, into a tile (zeros past n)
+template <bool NEG>
+__device__ __forceinline__ void stage_desc(float4 (*tile)[MT_PAD], const float* __restrict__ d, int first, int n) {
+#pragma unroll
+    for (int k = 0; k < MT * 16 / 256; k++) {
+        const int e = threadIdx.x + 256 * k, row = e / 16, g = e % 16;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (first + row < n) v = __ldg(reinterpret_cast<const float4*>(d + size_t(first + row) * 64) + g);
+        tile[g][row] = NEG ? make_float4(-v.x, -v.y, -v.z, -v.w) : v;
+    }
+}
+
+__global__ void __launch_bounds__(256, 2) k_match(MatchJobs jobs, int cap, u64 one, u64* __restrict__ keys) {
+    __shared__ MatchSmem sm;
     const MatchJob& J = jobs.j[blockIdx.y];
-    gls_match* out = out_all + size_t(blockIdx.y) * cap;
-    const float* __restrict__ d1 = J.d1;
-    const float* __restrict__ d2 = J.d2;
-    const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int n1 = *J.n1, n2 = *J.n2;
-    if (i >= n1) return;
-    const float* p1 = d1 + size_t(i) * 64;
-    float dmin = FLT_MAX;
-    int jmin = 0;
-    if (lane < 24) {
-        for (int j = 0; j + lane < n2; j += 24) {
-            const float4* p2 = reinterpret_cast<const float4*>(d2 + size_t(j + lane) * 64);
-            const float4* q1 = reinterpret_cast<const float4*>(p1);
-            float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-#pragma unroll 4
-            for (int g = 0; g < 16; g++) {
-                const float4 u = __ldg(q1 + g), v = __ldg(p2 + g);
-                const float e0 = fsub(u.x, v.x), e1 = fsub(u.y, v.y), e2 = fsub(u.z, v.z), e3 = fsub(u.w, v.w);
-                s0 = fadd(s0, fmul(e0, e0));
-                s1 = fadd(s1, fmul(e1, e1));
-                s2 = fadd(s2, fmul(e2, e2));
-                s3 = fadd(s3, fmul(e3, e3));
+    const int q0 = blockIdx.x * MT;
+    if (q0 >= n1) return;
+    const int tiles = (n2 + MT - 1) / MT;
+    const int t0 = int(int64_t(tiles) * blockIdx.z / gridDim.z), t1 = int(int64_t(tiles) * (blockIdx.z + 1) / gridDim.z);
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    stage_desc<false>(sm.q, J.d1, q0, n1);
+    u64 best[4] = {kNoMatch, kNoMatch, kNoMatch, kNoMatch};
+    for (int tile = t0; tile < t1; tile++) {
+        __syncthreads();  // the previous tile is read
+        stage_desc<true>(sm.t, J.d2, tile * MT, n2);
+        __syncthreads();
+        u64 s01[4][4], s23[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) s01[i][j] = s23[i][j] = 0;
+#pragma unroll 2
+        for (int g = 0; g < 16; g++) {
+            ulonglong2 q[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) q[i] = *reinterpret_cast<const ulonglong2*>(&sm.q[g][ty + 16 * i]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&sm.t[g][tx + 16 * j]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const u64 e01 = add_f32x2(q[i].x, t.x), e23 = add_f32x2(q[i].y, t.y);
+                    // 1 x + s rounds as the sum; `one` comes from the launch,
+                    // since a packed multiply and add, or a multiply-add by a
+                    // known 1, is contracted into one rounding
+                    s01[i][j] = fma_f32x2(mul_f32x2(e01, e01), one, s01[i][j]);
+                    s23[i][j] = fma_f32x2(mul_f32x2(e23, e23), one, s23[i][j]);
+                }
             }
-            const float d = fsqrt(fadd(fadd(fadd(s0, s1), s2), s3));
-            if (d < dmin) {
-                dmin = d;
-                jmin = j + lane;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int jt = tile * MT + tx + 16 * j;
+            const unsigned low = (unsigned(jt % 24) << 27) | unsigned(jt);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 a = unpack_f32x2(s01[i][j]), b = unpack_f32x2(s23[i][j]);
+                const float d = fsqrt(fadd(fadd(fadd(a.x, a.y), b.x), b.y));
+                if (jt < n2 && d < FLT_MAX) {
+                    const u64 key = (u64(__float_as_uint(d)) << 32) | low;
+                    best[i] = key < best[i] ? key : best[i];
+                }
             }
         }
     }
-    // lane 0 takes the lanes in order, strictly smaller wins
-    float best = __shfl_sync(0xffffffffu, dmin, 0);
-    int bj = __shfl_sync(0xffffffffu, jmin, 0);
-    for (int l = 1; l < 24; l++) {
-        const float dl = __shfl_sync(0xffffffffu, dmin, l);
-        const int jl = __shfl_sync(0xffffffffu, jmin, l);
-        if (dl < best) {
-            best = dl;
-            bj = jl;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {  // over the 16 threads of a query
+            const u64 v = __shfl_xor_sync(0xffffffffu, best[i], o);
+            best[i] = v < best[i] ? v : best[i];
         }
+        const int q = q0 + ty + 16 * i;
+        if (tx == 0 && q < n1 && best[i] != kNoMatch) atomicMin(keys + size_t(blockIdx.y) * cap + q, best[i]);
     }
-    if (lane == 0) out[i] = {i, bj, best};
 }
 
 // refineMatch order (SURF.cpp:917-929): distance, then query index; the
 // sorted matches become point pairs (query pt, train pt) as findMatches
-// builds them (SURF.hpp:65-75).
-__global__ void __launch_bounds__(256) k_match_rank(MatchJobs jobs, int cap, const gls_match* __restrict__ m_all,
+// builds them (SURF.hpp:65-75). A block ranks 64 matches, four threads each
+// scanning a quarter of the others ((distance bits, query index) as one
+// 64-bit key: distances are not negative).
+constexpr int MR_N = 64;
+__global__ void __launch_bounds__(256) k_match_rank(MatchJobs jobs, int cap, const u64* __restrict__ keys_all,
                                                     gls_match* __restrict__ sorted_all, float4* __restrict__ pairs_all) {
-    __shared__ gls_match tile[256];
+    __shared__ u64 tile[1024];
     const MatchJob& J = jobs.j[blockIdx.y];
-    const gls_match* __restrict__ m = m_all + size_t(blockIdx.y) * cap;
+    const u64* __restrict__ keys = keys_all + size_t(blockIdx.y) * cap;
     gls_match* __restrict__ sorted = sorted_all + size_t(blockIdx.y) * cap;
     float4* __restrict__ pairs = pairs_all + size_t(blockIdx.y) * cap;
-    const gls_keypoint* __restrict__ k1 = J.k1;
-    const gls_keypoint* __restrict__ k2 = J.k2;
     const int n = *J.n1;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.x * blockDim.x >= n) return;
-    gls_match me{};
-    if (i < n) me = m[i];
+    const int i = blockIdx.x * MR_N + (threadIdx.x >> 2), part = threadIdx.x & 3;
+    if (blockIdx.x * MR_N >= n) return;
+    auto distance = [](u64 key) { return key == kNoMatch ? FLT_MAX : __uint_as_float(unsigned(key >> 32)); };
+    auto rank_key = [&](u64 key, int q) { return (u64(__float_as_uint(distance(key))) << 32) | unsigned(q); };
+    const u64 mine = i < n ? keys[i] : 0, me = rank_key(mine, i);
     int rank = 0;
-    for (int j0 = 0; j0 < n; j0 += 256) {
+    for (int j0 = 0; j0 < n; j0 += 1024) {
         __syncthreads();
-        if (j0 + threadIdx.x < n) tile[threadIdx.x] = m[j0 + threadIdx.x];
+        for (int j = threadIdx.x; j < 1024; j += 256) tile[j] = j0 + j < n ? rank_key(keys[j0 + j], j0 + j) : kNoMatch;
         __syncthreads();
-        const int c = min(256, n - j0);
-        if (i < n)
-            for (int j = 0; j < c; j++) {
-                const gls_match& o = tile[j];
-                rank += (o.distance < me.distance || (o.distance == me.distance && o.query_idx < me.query_idx)) ? 1 : 0;
-            }
+        const int c = min(1024, n - j0);
+#pragma unroll 8
+        for (int j = part; j < c; j += 4) rank += tile[j] < me ? 1 : 0;
     }
-    if (i < n) {
-        sorted[rank] = me;
-        const gls_keypoint a = k1[me.query_idx], b = k2[me.train_idx];
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+    if (i < n && part == 0) {
+        const int train = mine == kNoMatch ? 0 : int(mine & ((1u << 27) - 1));
+        sorted[rank] = {i, train, distance(mine)};
+        const gls_keypoint a = J.k1[i], b = J.k2[train];
         pairs[rank] = make_float4(a.x, a.y, b.x, b.y);
     }
 }
 
 // ------------------------------------------------------------ homography
 // FindLeastSquaresHomography (LeastSquaresHomography.cpp:355-423) with the
-// Jacobi solver of :218-353; hypot(p, q) is sqrt(p^2 + q^2). One warp
-// solves one system: the rotations of a Jacobi step update disjoint element
-// pairs, one pair per lane, so the warp produces the sequential loop's
-// results bit for bit.
+// Jacobi solver of :218-353; hypot(p, q) is sqrt(p^2 + q^2). Every value is
+// the sequential loop's, bit for bit: a Jacobi step's rotations update disjoint
+// element pairs, and the scans for the next pivot compare the same values in
+// an order whose result does not depend on it.
+//
+// Ten lanes solve one system, three systems to a warp (lanes 30 and 31 idle
+// along with the third): lane r of a group owns row r. The pivot choice is a
+// 9-lane tournament, the rotation parameters (two square roots, three
+// divisions, most of a step's instructions) are formed by all lanes of the
+// three groups at once, and lanes k and l rescan their rows together. A
+// 4-point fit takes about 136 steps; a step costs a warp about 490 issue
+// slots for three systems where a warp per system, with its serial scans on
+// one lane, took about 660 for one: 2.16 -> 0.74 ms for 14 x 2000 fits (73%
+// of the issue slots, FP64 pipe 34%).
 __device__ __forceinline__ double hypot_d(double a, double b) { return dsqrt(dadd(dmul(a, a), dmul(b, b))); }
 
 constexpr unsigned kFull = 0xffffffffu;
+constexpr int LS_LANES = 10, LS_GROUPS = 3;
 
-struct LsWarp {  // shared scratch of one warp
-    double a[81], V[81], W[9], T[9];
+struct LsGroup {  // shared scratch of one system
+    double a[9][10];        // the symmetric matrix, both triangles (destroyed)
+    double V[9][9];         // eigenvectors as rows, in the order before sorting
+    double T[9];
     double cen[4], mad[4];  // (cm0, cm1, cM0, cM1) and (sm0, sm1, sM0, sM1)
-    double nrm[4][4];       // the 4 sample points, normalised (a0, a1, b0, b1)
-    int indR[9], indC[9];
 };
+
+// a lane's place: its group's first lane and its row (9 and more: idle)
+struct LsLane {
+    int base, r;
+};
+__device__ __forceinline__ LsLane ls_lane() {
+    const int lane = threadIdx.x & 31, g = min(lane / LS_LANES, LS_GROUPS - 1);
+    return {g * LS_LANES, lane - g * LS_LANES};
+}
 
 __device__ __forceinline__ void jac_rot(double& v0, double& v1, double c, double s) {
     const double a0 = v0, b0 = v1;
@@ -718,139 +814,131 @@ __device__ __forceinline__ void jac_rot(double& v0, double& v1, double c, double
     v1 = dadd(dmul(a0, s), dmul(b0, c));
 }
 
-// column m > k of the largest |a[k][m]| (the first on ties)
-__device__ __forceinline__ int max_in_row(const double* a, int k) {
-    int m = k + 1;
-    double mv = fabs(a[k * 9 + m]);
-    for (int i = k + 2; i < 9; i++) {
-        const double val = fabs(a[k * 9 + i]);
-        if (mv < val) mv = val, m = i;
+// of row r of the symmetric matrix: the column right of the diagonal and the
+// one left of it with the largest magnitude, the first on ties (indR, indC)
+__device__ __forceinline__ void row_maxima(const double* row, int r, int& right, int& left) {
+    double mr = 0.0, ml = 0.0;
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+        const double v = fabs(row[j]);
+        if (j > r && (j == r + 1 || mr < v)) mr = v, right = j;
+        if (j < r && (j == 0 || ml < v)) ml = v, left = j;
     }
-    return m;
 }
 
-// row m < k of the largest |a[m][k]| (the first on ties)
-__device__ __forceinline__ int max_in_col(const double* a, int k) {
-    int m = 0;
-    double mv = fabs(a[k]);
-    for (int i = 1; i < k; i++) {
-        const double val = fabs(a[i * 9 + k]);
-        if (mv < val) mv = val, m = i;
-    }
-    return m;
-}
-
-// Jacobi eigen-solve of the symmetric S.a (destroyed): eigenvalues S.W
-// sorted descending, eigenvectors as the rows of S.V. Called by a whole warp.
-__device__ void jacobi9_warp(LsWarp& S) {
+// Jacobi eigen-solve of the group's S.a: returns the row of S.V that the
+// reference's sort (descending eigenvalues) puts last. Called by a whole
+// warp; groups with run = false only take part in the shuffles.
+__device__ int jacobi9(LsGroup& S, LsLane L, bool run) {
     constexpr int N = 9;
-    const int lane = threadIdx.x & 31;
-    double* a = S.a;
-    if (lane < N) {
-        for (int i = 0; i < N; i++) S.V[lane * N + i] = i == lane ? 1.0 : 0.0;
-        S.W[lane] = a[lane * N + lane];
-        if (lane < N - 1) S.indR[lane] = max_in_row(a, lane);
-        if (lane > 0) S.indC[lane] = max_in_col(a, lane);
+    const int r = L.r, row = min(r, N - 1);
+    const bool lane_on = run && r < N;
+    double* mine = S.a[row];
+    double W = 0.0;
+    int indR = N - 1, indC = 0;
+    if (lane_on) {
+#pragma unroll
+        for (int i = 0; i < N; i++) S.V[row][i] = i == row ? 1.0 : 0.0;
+        W = mine[row];
+        row_maxima(mine, row, indR, indC);
     }
     __syncwarp();
+    bool active = run;
     for (int it = 0; it < N * N * 30; it++) {
-        int k = 0, l = 0, stop = 0;
-        double c = 0.0, s = 0.0;
-        if (lane == 0) {
-            double mv = fabs(a[S.indR[0]]);
-            for (int i = 1; i < N - 1; i++) {
-                const double val = fabs(a[i * N + S.indR[i]]);
-                if (mv < val) mv = val, k = i;
+        // the pivot: the largest |a[i][indR[i]]| (i = 0..7), then
+        // |a[indC[i]][i]| (i = 1..8), the first of equals; a NaN in the very
+        // first place is kept, elsewhere it never wins
+        double v = -1.0;
+        int code = 31;
+        if (lane_on && active) {
+            if (r < N - 1) {
+                v = fabs(mine[indR]);
+                code = r;
+                if (isnan(v)) v = r == 0 ? __longlong_as_double(0x7ff0000000000000ll) : -1.0;
             }
-            l = S.indR[k];
-            for (int i = 1; i < N; i++) {
-                const double val = fabs(a[S.indC[i] * N + i]);
-                if (mv < val) mv = val, k = S.indC[i], l = i;
+            if (r > 0) {
+                const double vc = fabs(mine[indC]);
+                if (v < vc) v = vc, code = 16 + r;
             }
-            const double p = a[k * N + l];
-            if (fabs(p) <= DBL_EPSILON) {
-                stop = 1;
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            const double ov = __shfl_down_sync(kFull, v, o);
+            const int oc = __shfl_down_sync(kFull, code, o);
+            if (r + o < N && r < o && (v < ov || (v == ov && oc < code))) v = ov, code = oc;
+        }
+        code = __shfl_sync(kFull, code, L.base) & 31;
+        const int from = code & 15, ind = __shfl_sync(kFull, indR | (indC << 8), L.base + min(from, N - 1));
+        int k = code < 16 ? from : ind >> 8, l = code < 16 ? ind & 255 : from;
+        k = min(k, N - 1);
+        l = min(l, N - 1);
+        const double Wk = __shfl_sync(kFull, W, L.base + k), Wl = __shfl_sync(kFull, W, L.base + l);
+        const double p = S.a[k][l];
+        active = active && !(fabs(p) <= DBL_EPSILON);
+        if (!__any_sync(kFull, active)) break;
+        const double y = dmul(dsub(Wl, Wk), 0.5);
+        double t = dadd(fabs(y), hypot_d(p, y));
+        double s = hypot_d(p, t);
+        const double c = ddiv(t, s);
+        s = ddiv(p, s);
+        t = dmul(ddiv(p, t), p);
+        if (y < 0) {
+            s = -s;
+            t = -t;
+        }
+        __syncwarp();  // p is read by every lane
+        if (lane_on && active) {
+            if (r == k) {
+                W = dsub(W, t);
+                mine[l] = 0.0;
+            } else if (r == l) {
+                W = dadd(W, t);
+                mine[k] = 0.0;
             } else {
-                const double y = dmul(dsub(S.W[l], S.W[k]), 0.5);
-                double t = dadd(fabs(y), hypot_d(p, y));
-                s = hypot_d(p, t);
-                c = ddiv(t, s);
-                s = ddiv(p, s);
-                t = dmul(ddiv(p, t), p);
-                if (y < 0) {
-                    s = -s;
-                    t = -t;
-                }
-                a[k * N + l] = 0.0;
-                S.W[k] = dsub(S.W[k], t);
-                S.W[l] = dadd(S.W[l], t);
+                double ek = mine[k], el = mine[l];
+                jac_rot(ek, el, c, s);
+                mine[k] = ek;
+                mine[l] = el;
+                S.a[k][r] = ek;
+                S.a[l][r] = el;
             }
-        }
-        stop = __shfl_sync(kFull, stop, 0);
-        if (stop) break;
-        k = __shfl_sync(kFull, k, 0);
-        l = __shfl_sync(kFull, l, 0);
-        c = __shfl_sync(kFull, c, 0);
-        s = __shfl_sync(kFull, s, 0);
-        __syncwarp();
-        if (lane < N) {  // k < l always: indR points right, indC points up
-            if (lane != k && lane != l) {
-                if (lane < k) jac_rot(a[lane * N + k], a[lane * N + l], c, s);
-                else if (lane < l) jac_rot(a[k * N + lane], a[lane * N + l], c, s);
-                else jac_rot(a[k * N + lane], a[l * N + lane], c, s);
-            }
-            jac_rot(S.V[k * N + lane], S.V[l * N + lane], c, s);
+            jac_rot(S.V[k][r], S.V[l][r], c, s);
         }
         __syncwarp();
-        if (lane < 2) {
-            const int idx = lane == 0 ? k : l;
-            if (idx < N - 1) S.indR[idx] = max_in_row(a, idx);
-            if (idx > 0) S.indC[idx] = max_in_col(a, idx);
-        }
-        __syncwarp();
+        if (lane_on && active && (r == k || r == l)) row_maxima(mine, row, indR, indC);
     }
-    if (lane == 0) {
-        for (int k = 0; k < N - 1; k++) {
-            int m = k;
-            for (int i = k + 1; i < N; i++)
-                if (S.W[m] < S.W[i]) m = i;
-            if (k != m) {
-                const double tw = S.W[m];
-                S.W[m] = S.W[k];
-                S.W[k] = tw;
-                for (int i = 0; i < N; i++) {
-                    const double tv = S.V[m * N + i];
-                    S.V[m * N + i] = S.V[k * N + i];
-                    S.V[k * N + i] = tv;
-                }
-            }
-        }
+    // the selection sort of the eigenvalues, every lane of the group alike
+    double w[N];
+    int perm[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        w[i] = __shfl_sync(kFull, W, L.base + i);
+        perm[i] = i;
+    }
+#pragma unroll
+    for (int k = 0; k < N - 1; k++) {
+        int m = k, pm = perm[k];
+        double wm = w[k];
+#pragma unroll
+        for (int i = k + 1; i < N; i++)
+            if (wm < w[i]) wm = w[i], pm = perm[i], m = i;
+#pragma unroll
+        for (int i = k + 1; i < N; i++)
+            if (i == m) w[i] = w[k], perm[i] = perm[k];
+        w[k] = wm;
+        perm[k] = pm;
     }
     __syncwarp();
+    return perm[N - 1];
 }
 
-// entry j of the rows Lx, Ly of LeastSquaresHomography.cpp:396-397
-__device__ __forceinline__ double lx_entry(int j, double a0, double a1, double b0) {
-    switch (j) {
-        case 0: return a0;
-        case 1: return a1;
-        case 2: return 1.0;
-        case 6: return dmul(-b0, a0);
-        case 7: return dmul(-b0, a1);
-        case 8: return -b0;
-        default: return 0.0;
-    }
-}
-__device__ __forceinline__ double ly_entry(int j, double a0, double a1, double b1) {
-    switch (j) {
-        case 3: return a0;
-        case 4: return a1;
-        case 5: return 1.0;
-        case 6: return dmul(-b1, a0);
-        case 7: return dmul(-b1, a1);
-        case 8: return -b1;
-        default: return 0.0;
-    }
+// the rows Lx, Ly of LeastSquaresHomography.cpp:396-397 for a normalised
+// point pair (a0, a1) -> (b0, b1)
+__device__ __forceinline__ void ls_rows(double a0, double a1, double b0, double b1, double* lx, double* ly) {
+    lx[0] = a0, lx[1] = a1, lx[2] = 1.0, lx[3] = lx[4] = lx[5] = 0.0;
+    lx[6] = dmul(-b0, a0), lx[7] = dmul(-b0, a1), lx[8] = -b0;
+    ly[0] = ly[1] = ly[2] = 0.0, ly[3] = a0, ly[4] = a1, ly[5] = 1.0;
+    ly[6] = dmul(-b1, a0), ly[7] = dmul(-b1, a1), ly[8] = -b1;
 }
 
 // upper-triangle entry e (0..44) -> (j, k), j <= k
@@ -863,76 +951,85 @@ __device__ __forceinline__ void tri_index(int e, int& j, int& k) {
     k = j + e;
 }
 
-// The tail of the normalised DLT on S.a (full symmetric LtL), S.cen and
-// S.mad: least eigenvector, de-normalisation, scale to H[2][2] = 1. Warp.
-__device__ void ls_finish_warp(LsWarp& S, float* H) {
-    const int lane = threadIdx.x & 31;
-    jacobi9_warp(S);
-    const double* h0 = &S.V[72];
-    const double cm0 = S.cen[0], cm1 = S.cen[1], cM0 = S.cen[2], cM1 = S.cen[3];
-    const double sm0 = S.mad[0], sm1 = S.mad[1], sM0 = S.mad[2], sM1 = S.mad[3];
-    if (lane < 9) {
+// The tail of the normalised DLT on S.a, S.cen and S.mad: least
+// eigenvector, de-normalisation, scale to H[2][2] = 1. Warp.
+__device__ void ls_finish(LsGroup& S, LsLane L, bool run, float* H) {
+    const double* h0 = S.V[jacobi9(S, L, run)];
+    const int r = min(L.r, 8), i = r / 3, j = r % 3;
+    double q = 0.0;
+    if (run) {
+        const double cm0 = S.cen[0], cm1 = S.cen[1], sm0 = S.mad[0], sm1 = S.mad[1];
         const double inv[9] = {sm0, 0, cm0, 0, sm1, cm1, 0, 0, 1};
-        const int i = lane / 3, j = lane % 3;
         double acc = 0.0;
-        for (int k = 0; k < 3; k++) acc = dadd(acc, dmul(inv[i * 3 + k], h0[k * 3 + j]));
-        S.T[lane] = acc;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const double e = i == 0 ? inv[k] : i == 1 ? inv[3 + k] : inv[6 + k];
+            acc = dadd(acc, dmul(e, h0[k * 3 + j]));
+        }
+        if (L.r < 9) S.T[r] = acc;
     }
     __syncwarp();
-    double r = 0.0;
-    if (lane < 9) {
+    if (run) {
+        const double cM0 = S.cen[2], cM1 = S.cen[3], sM0 = S.mad[2], sM1 = S.mad[3];
         const double nrm[9] = {ddiv(1.0, sM0), 0, ddiv(-cM0, sM0), 0, ddiv(1.0, sM1), ddiv(-cM1, sM1), 0, 0, 1};
-        const int i = lane / 3, j = lane % 3;
-        for (int k = 0; k < 3; k++) r = dadd(r, dmul(S.T[i * 3 + k], nrm[k * 3 + j]));
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const double e = j == 0 ? nrm[3 * k] : j == 1 ? nrm[3 * k + 1] : nrm[3 * k + 2];
+            q = dadd(q, dmul(S.T[i * 3 + k], e));
+        }
     }
-    const double r8 = __shfl_sync(kFull, r, 8);
-    if (lane < 9) H[lane] = fdiv(__double2float_rn(r), __double2float_rn(r8));
+    const double q8 = __shfl_sync(kFull, q, L.base + 8);
+    if (run && L.r < 9) H[r] = fdiv(__double2float_rn(q), __double2float_rn(q8));
     __syncwarp();
 }
 
-// The 4-point model of one RANSAC sample; false where the reference throws
-// (a degenerate spread). Warp.
-__device__ bool ls4_warp(LsWarp& S, const float4* __restrict__ P, const int* __restrict__ idx, float* H) {
-    const int lane = threadIdx.x & 31;
+// The 4-point models of the RANSAC samples idx of a warp's groups; a group
+// whose spread is degenerate (where the reference throws) gets the identity.
+__device__ void ls4(LsGroup& S, LsLane L, bool run, const float4* __restrict__ P, const int* __restrict__ idx,
+                    float* H) {
+    const int r = L.r;
     auto comp = [](const float4& p, int c) { return c == 0 ? p.z : c == 1 ? p.w : c == 2 ? p.x : p.y; };
-    if (lane < 4) {
+    // the rows of the four points, in the place of V (built after them)
+    double(*lx)[9] = S.V, (*ly)[9] = S.V + 4;
+    if (run && r < 4) {
         double acc = 0.0;
-        for (int i = 0; i < 4; i++) acc = dadd(acc, double(comp(P[idx[i]], lane)));
-        S.cen[lane] = ddiv(acc, 4.0);
+        for (int i = 0; i < 4; i++) acc = dadd(acc, double(comp(P[idx[i]], r)));
+        const double cen = ddiv(acc, 4.0);
+        acc = 0.0;
+        for (int i = 0; i < 4; i++) acc = dadd(acc, fabs(dsub(double(comp(P[idx[i]], r)), cen)));
+        S.cen[r] = cen;
+        S.mad[r] = ddiv(acc, 4.0);
     }
     __syncwarp();
-    if (lane < 4) {
-        double acc = 0.0;
-        for (int i = 0; i < 4; i++) acc = dadd(acc, fabs(dsub(double(comp(P[idx[i]], lane)), S.cen[lane])));
-        S.mad[lane] = ddiv(acc, 4.0);
+    bool degenerate = false;
+    if (run) {
+        const double eps = DBL_EPSILON;
+        degenerate =
+            fabs(S.mad[0]) < eps || fabs(S.mad[1]) < eps || fabs(S.mad[2]) < eps || fabs(S.mad[3]) < eps;
+    }
+    const bool fit = run && !degenerate;
+    if (fit && r < 4) {
+        const float4 p = P[idx[r]];
+        ls_rows(ddiv(dsub(double(p.x), S.cen[2]), S.mad[2]), ddiv(dsub(double(p.y), S.cen[3]), S.mad[3]),
+                ddiv(dsub(double(p.z), S.cen[0]), S.mad[0]), ddiv(dsub(double(p.w), S.cen[1]), S.mad[1]), lx[r],
+                ly[r]);
     }
     __syncwarp();
-    const double eps = DBL_EPSILON;
-    if (fabs(S.mad[0]) < eps || fabs(S.mad[1]) < eps || fabs(S.mad[2]) < eps || fabs(S.mad[3]) < eps) return false;
-    if (lane < 4) {
-        const float4 p = P[idx[lane]];
-        S.nrm[lane][0] = ddiv(dsub(double(p.x), S.cen[2]), S.mad[2]);
-        S.nrm[lane][1] = ddiv(dsub(double(p.y), S.cen[3]), S.mad[3]);
-        S.nrm[lane][2] = ddiv(dsub(double(p.z), S.cen[0]), S.mad[0]);
-        S.nrm[lane][3] = ddiv(dsub(double(p.w), S.cen[1]), S.mad[1]);
-    }
-    __syncwarp();
-    for (int e = lane; e < 45; e += 32) {
-        int j, k;
-        tri_index(e, j, k);
-        double acc = 0.0;
-        for (int q = 0; q < 4; q++) {
-            const double* v = S.nrm[q];
-            const double xj = lx_entry(j, v[0], v[1], v[2]), xk = lx_entry(k, v[0], v[1], v[2]);
-            const double yj = ly_entry(j, v[0], v[1], v[3]), yk = ly_entry(k, v[0], v[1], v[3]);
-            acc = dadd(acc, dadd(dmul(xj, xk), dmul(yj, yk)));
+    if (fit && r < 9) {
+        for (int e = r; e < 45; e += 9) {
+            int j, k;
+            tri_index(e, j, k);
+            double acc = 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc = dadd(acc, dadd(dmul(lx[q][j], lx[q][k]), dmul(ly[q][j], ly[q][k])));
+            S.a[j][k] = acc;
+            S.a[k][j] = acc;  // completeSymm
         }
-        S.a[j * 9 + k] = acc;
-        S.a[k * 9 + j] = acc;  // completeSymm
     }
     __syncwarp();
-    ls_finish_warp(S, H);
-    return true;
+    ls_finish(S, L, fit, H);
+    if (run && degenerate && r < 9) H[r] = (r % 4 == 0) ? 1.0f : 0.0f;
+    __syncwarp();
 }
 
 // applyHomography + squared error (Homography.cpp:65-70)
@@ -955,41 +1052,52 @@ struct RansacJobs {
     RansacJob j[kMaxJobs];
 };
 
-// RANSAC hypotheses (RTL/RANSAC.hpp:47-66, 101-108): one warp per
-// iteration fits its sample and counts the errors above the threshold.
-constexpr int kHypWarps = 4;
+// RANSAC hypotheses (RTL/RANSAC.hpp:47-66, 101-108): a warp fits three
+// iterations' samples and counts the errors above the threshold of the three
+// models in one pass over the pairs.
+constexpr int kHypWarps = 4, kHypModels = kHypWarps * LS_GROUPS;
 __global__ void __launch_bounds__(32 * kHypWarps) k_ransac_models(RansacJobs jobs, int iters, float threshold,
                                                                   float* __restrict__ models_all,
                                                                   int* __restrict__ losses_all) {
-    __shared__ LsWarp S[kHypWarps];
-    __shared__ float Hs[kHypWarps][9];
+    __shared__ LsGroup S[kHypWarps][LS_GROUPS];
+    __shared__ float Hs[kHypWarps][LS_GROUPS][9];
     const RansacJob& J = jobs.j[blockIdx.y];
     const float4* __restrict__ pairs = J.pairs;
-    const int* __restrict__ samples = J.samples;
     const int n = J.n;
     float* __restrict__ models = models_all + size_t(blockIdx.y) * iters * 9;
     int* __restrict__ losses = losses_all + size_t(blockIdx.y) * iters;
     const int w = threadIdx.x / 32, lane = threadIdx.x & 31;
-    const int it = blockIdx.x * kHypWarps + w;
-    if (it >= iters) return;  // warp-uniform
-    float* H = Hs[w];
-    if (!ls4_warp(S[w], pairs, samples + 4 * it, H)) {
-        if (lane < 9) H[lane] = (lane % 4 == 0) ? 1.0f : 0.0f;
-        __syncwarp();
+    const LsLane L = ls_lane();
+    const int g = L.base / LS_LANES, it0 = (blockIdx.x * kHypWarps + w) * LS_GROUPS, it = it0 + g;
+    if (it0 >= iters) return;  // warp-uniform
+    ls4(S[w][g], L, it < iters, pairs, J.samples + 4 * min(it, iters - 1), Hs[w][g]);
+    const int ng = min(LS_GROUPS, iters - it0);
+    float H[LS_GROUPS][9];
+#pragma unroll
+    for (int m = 0; m < LS_GROUPS; m++)
+#pragma unroll
+        for (int e = 0; e < 9; e++) H[m][e] = Hs[w][min(m, ng - 1)][e];
+    int c[LS_GROUPS] = {0, 0, 0};
+    for (int i = lane; i < n; i += 32) {
+        const float4 p = pairs[i];
+#pragma unroll
+        for (int m = 0; m < LS_GROUPS; m++) c[m] += fabsf(h_error(H[m], p)) > threshold ? 1 : 0;
     }
-    int c = 0;
-    for (int i = lane; i < n; i += 32) c += fabsf(h_error(H, pairs[i])) > threshold ? 1 : 0;
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
-    if (lane == 0) losses[it] = c;
-    if (lane < 9) models[it * 9 + lane] = H[lane];
+#pragma unroll
+    for (int m = 0; m < LS_GROUPS; m++) {
+        for (int o = 16; o > 0; o >>= 1) c[m] += __shfl_xor_sync(kFull, c[m], o);
+        if (m < ng && lane == 0) losses[it0 + m] = c[m];
+    }
+    for (int e = lane; e < 9 * ng; e += 32) models[it0 * 9 + e] = Hs[w][e / 9][e % 9];
 }
 
 // The first model with the least loss, its inliers (|error| < threshold,
 // in index order) and, with 4 or more, their least-squares refit
-// (Homography.cpp:90-113). One block; the sequential sums read the inliers
-// staged in shared memory.
+// (Homography.cpp:90-113). One block a job: bound by the serial FP64 additions
+// and the Jacobi steps; the terms of the sums are formed by all threads into
+// shared memory, off the chains (0.70 -> 0.20 ms at about 1000 inliers).
 constexpr int kFinalThreads = 256;
-constexpr int kStage = 512;
+constexpr int kStage = 512, kRows = 32;  // inliers staged: for the sums, for the normal matrix
 __global__ void __launch_bounds__(kFinalThreads) k_ransac_final(RansacJobs jobs, int cap,
                                                                  const float* __restrict__ models_all,
                                                                  const int* __restrict__ losses_all, int iters,
@@ -1009,12 +1117,17 @@ __global__ void __launch_bounds__(kFinalThreads) k_ransac_final(RansacJobs jobs,
     __shared__ int best_s, base_s;
     __shared__ float H[9], Hf[9];
     __shared__ int wsum[kFinalThreads / 32];
-    __shared__ LsWarp S;
-    __shared__ float4 stage[kStage];
-    __shared__ double4 nstage[kStage];
-    __shared__ double L[81];
+    __shared__ LsGroup S[LS_GROUPS];  // the first is the refit's, the others idle along
+    __shared__ double stage[4][kStage];
+    __shared__ double lx[kRows][9], ly[kRows][9], prod[kRows][45];
     __shared__ int red_loss[kFinalThreads / 32], red_idx[kFinalThreads / 32];
+    __shared__ int tri[45];  // upper-triangle entry -> 9 j + k
     const int t = threadIdx.x;
+    if (t < 45) {
+        int j, k;
+        tri_index(t, j, k);
+        tri[t] = 9 * j + k;
+    }
     {  // the first iteration with the least loss: (loss, index) minimum
         int bl = INT_MAX, bi = INT_MAX;
         for (int i = t; i < iters; i += kFinalThreads) {
@@ -1067,62 +1180,81 @@ __global__ void __launch_bounds__(kFinalThreads) k_ransac_final(RansacJobs jobs,
     bool refit = false;
     if (m >= 4) {
         // centroids, then mean absolute deviations: sequential sums over the
-        // inliers in index order
+        // inliers in index order, a thread per component; the terms are formed
+        // by all threads, so the serial path is one FP64 addition an inlier
         for (int pass = 0; pass < 2; pass++) {
             double acc = 0.0;
             for (int c0 = 0; c0 < m; c0 += kStage) {
                 const int cnt = min(kStage, m - c0);
                 __syncthreads();
-                for (int i = t; i < cnt; i += kFinalThreads) stage[i] = pairs[inliers[c0 + i]];
+                for (int i = t; i < cnt; i += kFinalThreads) {
+                    const float4 p = pairs[inliers[c0 + i]];
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        const double v = double(comp(p, c));
+                        stage[c][i] = pass == 0 ? v : fabs(dsub(v, S[0].cen[c]));
+                    }
+                }
                 __syncthreads();
                 if (t < 4) {
-                    if (pass == 0)
-                        for (int i = 0; i < cnt; i++) acc = dadd(acc, double(comp(stage[i], t)));
-                    else
-                        for (int i = 0; i < cnt; i++) acc = dadd(acc, fabs(dsub(double(comp(stage[i], t)), S.cen[t])));
+                    int i = 0;
+                    for (; i + 16 <= cnt; i += 16) {
+#pragma unroll
+                        for (int u = 0; u < 16; u++) acc = dadd(acc, stage[t][i + u]);
+                    }
+                    for (; i < cnt; i++) acc = dadd(acc, stage[t][i]);
                 }
             }
             if (t < 4) {
-                if (pass == 0) S.cen[t] = ddiv(acc, double(m));
-                else S.mad[t] = ddiv(acc, double(m));
+                if (pass == 0) S[0].cen[t] = ddiv(acc, double(m));
+                else S[0].mad[t] = ddiv(acc, double(m));
             }
             __syncthreads();
         }
         const double eps = DBL_EPSILON;
         const bool degenerate =
-            fabs(S.mad[0]) < eps || fabs(S.mad[1]) < eps || fabs(S.mad[2]) < eps || fabs(S.mad[3]) < eps;
+            fabs(S[0].mad[0]) < eps || fabs(S[0].mad[1]) < eps || fabs(S[0].mad[2]) < eps || fabs(S[0].mad[3]) < eps;
         if (!degenerate) {
+            // the normal matrix, entry by entry in inlier order: a thread per
+            // inlier forms its rows, all threads the 45 products of each
+            // inlier, and 45 threads add them up, one FP64 addition an inlier
+            // on the serial path
             double acc = 0.0;
-            int j = 0, k = 0;
-            if (t < 45) tri_index(t, j, k);
-            for (int c0 = 0; c0 < m; c0 += kStage) {
-                const int cnt = min(kStage, m - c0);
+            for (int c0 = 0; c0 < m; c0 += kRows) {
+                const int cnt = min(kRows, m - c0);
                 __syncthreads();
                 for (int i = t; i < cnt; i += kFinalThreads) {
                     const float4 p = pairs[inliers[c0 + i]];
-                    nstage[i] = make_double4(ddiv(dsub(double(p.x), S.cen[2]), S.mad[2]),
-                                             ddiv(dsub(double(p.y), S.cen[3]), S.mad[3]),
-                                             ddiv(dsub(double(p.z), S.cen[0]), S.mad[0]),
-                                             ddiv(dsub(double(p.w), S.cen[1]), S.mad[1]));
+                    ls_rows(ddiv(dsub(double(p.x), S[0].cen[2]), S[0].mad[2]),
+                            ddiv(dsub(double(p.y), S[0].cen[3]), S[0].mad[3]),
+                            ddiv(dsub(double(p.z), S[0].cen[0]), S[0].mad[0]),
+                            ddiv(dsub(double(p.w), S[0].cen[1]), S[0].mad[1]), lx[i], ly[i]);
                 }
                 __syncthreads();
-                if (t < 45)
-                    for (int q = 0; q < cnt; q++) {
-                        const double4 v = nstage[q];
-                        const double xj = lx_entry(j, v.x, v.y, v.z), xk = lx_entry(k, v.x, v.y, v.z);
-                        const double yj = ly_entry(j, v.x, v.y, v.w), yk = ly_entry(k, v.x, v.y, v.w);
-                        acc = dadd(acc, dadd(dmul(xj, xk), dmul(yj, yk)));
+                for (int e = t; e < cnt * 45; e += kFinalThreads) {
+                    const int i = e / 45;
+                    const int jk = tri[e % 45], j = jk / 9, k = jk % 9;
+                    prod[i][e % 45] = dadd(dmul(lx[i][j], lx[i][k]), dmul(ly[i][j], ly[i][k]));
+                }
+                __syncthreads();
+                if (t < 45) {
+                    if (cnt == kRows) {
+#pragma unroll
+                        for (int i = 0; i < kRows; i++) acc = dadd(acc, prod[i][t]);
+                    } else {
+                        for (int i = 0; i < cnt; i++) acc = dadd(acc, prod[i][t]);
                     }
+                }
             }
             if (t < 45) {
-                L[j * 9 + k] = acc;
-                L[k * 9 + j] = acc;  // completeSymm
+                const int j = tri[t] / 9, k = tri[t] % 9;
+                S[0].a[j][k] = acc;
+                S[0].a[k][j] = acc;  // completeSymm
             }
             __syncthreads();
             if (t < 32) {
-                for (int i = t; i < 81; i += 32) S.a[i] = L[i];
-                __syncwarp();
-                ls_finish_warp(S, Hf);
+                const LsLane L = ls_lane();
+                ls_finish(S[L.base / LS_LANES], L, L.base == 0, Hf);
             }
             refit = true;
             __syncthreads();
@@ -1436,7 +1568,7 @@ gls_status run_ransac(gls_surf* s, const std::vector<int>& ns, float threshold, 
     GLS_TRY(s->n_inliers.ensure(size_t(J) * sizeof(int)));
     GLS_TRY(s->Hdev.ensure(size_t(J) * 9 * sizeof(float)));
     GLS_TRY(s->loss.ensure(size_t(J) * sizeof(float)));
-    k_ransac_models<<<dim3((iters + kHypWarps - 1) / kHypWarps, J), 32 * kHypWarps, 0, st>>>(
+    k_ransac_models<<<dim3((iters + kHypModels - 1) / kHypModels, J), 32 * kHypWarps, 0, st>>>(
         rj, iters, threshold, reinterpret_cast<float*>(s->models.p), reinterpret_cast<int*>(s->losses.p));
     GLS_TRY(launch_check(s, "k_ransac_models"));
     k_ransac_final<<<J, kFinalThreads, 0, st>>>(rj, int(cap), reinterpret_cast<const float*>(s->models.p),
@@ -1463,7 +1595,7 @@ gls_status ransac_result(gls_surf* s, float* H, int32_t* inliers, int32_t* n_inl
 gls_status ensure_pairs(gls_surf* s, int jobs, int cap) {
     s->pair_cap = std::max(s->pair_cap, cap);
     const size_t c = size_t(std::max(s->pair_cap, 1));
-    GLS_TRY(s->matches.ensure(size_t(jobs) * c * sizeof(gls_match)));
+    GLS_TRY(s->matches.ensure(size_t(jobs) * c * sizeof(u64)));
     GLS_TRY(s->matches_sorted.ensure(size_t(jobs) * c * sizeof(gls_match)));
     GLS_TRY(s->pairs.ensure(size_t(jobs) * c * sizeof(float4)));
     return GLS_OK;
@@ -1482,13 +1614,16 @@ gls_status run_match(gls_surf* s, const std::vector<std::pair<int, int>>& qt, cu
                    reinterpret_cast<const int*>(t.count.p), reinterpret_cast<const gls_keypoint*>(t.kps.p)};
     }
     const int cap = s->pair_cap;
-    const int warps = 4;
-    k_match<<<dim3((s->capacity + warps - 1) / warps, J), 32 * warps, 0, st>>>(
-        mj, cap, reinterpret_cast<gls_match*>(s->matches.p));
+    u64* keys = reinterpret_cast<u64*>(s->matches.p);
+    GLS_CUDA(cudaMemsetAsync(keys, 0xff, size_t(J) * cap * sizeof(u64), st));
+    // the train set split so that the blocks fill about eight rounds of two
+    // per SM (148): the last round's idle share stays near a tenth
+    const int tiles = (s->capacity + MT - 1) / MT;
+    const int split = std::clamp(8 * 296 / std::max(tiles * J, 1), 1, std::max(tiles, 1));
+    k_match<<<dim3(tiles, J, split), 256, 0, st>>>(mj, cap, kOne2, keys);
     GLS_TRY(launch_check(s, "k_match"));
-    k_match_rank<<<dim3((s->capacity + 255) / 256, J), 256, 0, st>>>(
-        mj, cap, reinterpret_cast<const gls_match*>(s->matches.p), reinterpret_cast<gls_match*>(s->matches_sorted.p),
-        reinterpret_cast<float4*>(s->pairs.p));
+    k_match_rank<<<dim3((s->capacity + MR_N - 1) / MR_N, J), 256, 0, st>>>(
+        mj, cap, keys, reinterpret_cast<gls_match*>(s->matches_sorted.p), reinterpret_cast<float4*>(s->pairs.p));
     GLS_TRY(launch_check(s, "k_match_rank"));
     return GLS_OK;
 }

@@ -282,3 +282,50 @@ def test_register_frames_batch_equals_single_jobs():
             assert scene.corner_error(Hb[f - 1], Hs[f], 1024, 768) < 1.0
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("n1,n2", [(1, 1), (63, 24), (64, 64), (65, 129), (300, 25), (7, 0), (130, 500)])
+def test_match_edges_and_ties_bit_exact(n1, n2):
+    """Tile edges, split train sets, and equal distances (repeated and zero
+    descriptors), where the reference's lane order decides."""
+    rng = np.random.default_rng(n1 * 1000 + n2)
+    def feats(n):
+        d = rng.standard_normal((n, 64)).astype(np.float32)
+        d[rng.random(n) < 0.3] = 0.0
+        if n > 4:
+            d[n // 2:] = d[rng.integers(0, n // 2, n - n // 2)]
+        k = np.zeros(n, g.KEYPOINT_DTYPE)
+        k["x"], k["y"] = np.arange(n), 2 * np.arange(n)
+        return k, d
+    (k1, d1), (k2, d2) = feats(n1), feats(n2)
+    s = SURF(64, 64, max_features=600)
+    try:
+        s.load_features(0, k1, d1)
+        s.load_features(1, k2, d2)
+        m = s.match_slots(0, 1)
+        assert len(m) == n1
+        if n2 == 0:  # nothing to match: train 0 at the largest distance
+            assert (m["train_idx"] == 0).all() and (m["distance"] == np.finfo(np.float32).max).all()
+        else:
+            assert np.array_equal(m, R.match(d1, d2))
+    finally:
+        s.close()
+
+
+@pytest.mark.parametrize("n,iters", [(4, 1), (5, 2), (9, 3), (40, 4), (200, 100), (513, 37)])
+def test_ransac_partial_warps_bit_exact(n, iters):
+    """Iteration counts that leave groups of a warp empty, degenerate samples
+    among them, and inlier counts around the staged chunks."""
+    rng = np.random.default_rng(n)
+    a = rng.uniform(0, 500, (n, 2)).astype(np.float32)
+    if n > 8:
+        a[: n // 4] = a[0]  # repeated points: some samples have no spread
+    b = (a @ np.array([[1.01, 0.02], [-0.01, 0.99]]) + [3, -2] + rng.normal(0, 0.3, (n, 2))).astype(np.float32)
+    b[:: 7] += 40
+    s = SURF(64, 64, max_features=10)
+    try:
+        H, inl = FindHomography(s, np.concatenate([a, b], 1), 1.0, iters)
+        rH, rinl = R.find_homography(a, b, 1.0, iters)[:2]
+        assert np.array_equal(H, rH) and np.array_equal(inl, rinl)
+    finally:
+        s.close()
