@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(352, 3) k_pca_cov(Plane<S, 4> img, double* __r
     pca_cov_row<S>(img, part + size_t(blockIdx.x) * kPcaAcc, c0, min(c0 + group, n_chunks), sm);
 }
 
-constexpr int EJ_THREADS = 704;  // 22 warps: the prologue's 700 partial sums at once
+constexpr int EJ_THREADS = 384;  // the prologue's 700 partial sums in two rounds, 168 registers for the one-warp phases
 
 __global__ void __launch_bounds__(EJ_THREADS) k_pca_eigen(const double* __restrict__ part, int n_blocks,
                                                          int n_patches, float* __restrict__ basis, int* status) {

@@ -179,36 +179,40 @@ __device__ __forceinline__ void pca_cov_row(Plane<S, 4> img, double* __restrict_
 // Van Loan (Matrix Computations, 4th ed.): section 8.3.1 and the
 // bisection / inverse-iteration methods of sections 8.4.1 and 8.2.2
 // (the tred2 / tridiagonal bisection / tinvit sequence of EISPACK):
-//   1. Householder tridiagonalisation, A = Q T Q^T, Q = H_0 ... H_22: 23
-//      reflector steps, each a column norm, the product p = beta A v (a
-//      thread per row), and the rank-2 update of the trailing block by all
-//      threads (matrix in shared memory);
+//   1. Householder tridiagonalisation, A = Q T Q^T, Q = H_0 ... H_22, by
+//      seven warps, the matrix in shared memory: eight lanes to a row form
+//      its sums (three terms a lane, three shuffles), every row for itself, and
+//      update it; three barriers a step;
 //   2. the 8 largest eigenvalues of T by Sturm-sequence multisection:
 //      warp w brackets eigenvalue 24 - w (ascending order); its 32 lanes
 //      count the eigenvalues below 32 points of the bracket, which shrinks
-//      33-fold per round (7 rounds: 2.4e-11 of the spectrum width);
-//   3. each eigenvector of T by inverse iteration: the tridiagonal
-//      T - lambda I is factored once with partial pivoting (lane 0 of the
-//      eigenvalue's warp) and solved three times from a start vector of its
+//      33-fold per round (9 rounds: 2e-14 of the spectrum width). The counts
+//      are the sign changes of the leading principal minors' recurrence on T
+//      scaled by a power of two, one FMA a term on the serial path; a
+//      recurrence that ends at zero is counted by its pivots;
+//   3. the eigenvectors of T by inverse iteration, lane c of one warp for
+//      eigenvector c: T - lambda I is factored once with partial pivoting by
+//      selects (no divergence) and solved twice from a start vector of its
 //      own; tiny pivots are raised to eps ||T|| so the solve stays finite;
-//   4. the back-transform z = H_0 (H_1 (... H_22 y)), one reflector at a
-//      time for all 8 vectors (a thread per dot product, then the block),
-//      and Gram-Schmidt of the 8 vectors in eigenvalue order, the classical
-//      form applied twice (exactly equal eigenvalues give an orthonormal
-//      basis of their eigenspace; distinct ones are already orthogonal).
-//      FP64 warp shuffles are slow on this part (about 15 lanes per SM per
-//      cycle), so no step reduces across a warp's lanes.
+//   4. the back-transform z = H_0 (H_1 (... H_22 y)) in the same lanes, the
+//      vector in registers, the reflectors read by broadcast;
+//   5. Gram-Schmidt (modified, twice) of the 8 vectors in eigenvalue order if
+//      two eigenvalues lie close together (exactly equal ones give an
+//      orthonormal basis of their eigenspace; distinct ones are orthogonal
+//      already).
 // The top-8 eigenvectors (descending eigenvalue, each signed so its
 // largest-magnitude entry is positive; eigenvalues <= 1e-9 of the largest
 // completed as in select_pca_basis) are written as a row-major 25x8 FP32
 // basis. Every reduction has a fixed order, so the result is deterministic.
-// status receives the number of inverse-iteration solves per vector (3), or
+// status receives the number of inverse-iteration solves per vector (2), or
 // -1 when a vector came out non-finite (the basis is then still written).
-// 7 multisection rounds bracket each eigenvalue to 33^-7 (2.4e-11) of the
-// spectrum's width: inverse iteration from such a shift converges in its
-// three solves (the error shrinks by shift error / gap per solve), and the
-// eigenvalue itself only orders the vectors and sets the rank threshold
-constexpr int EJ_N = 25, EJ_TOP = 8, EJ_INV_ITERS = 3, EJ_MSEC_ROUNDS = 7;
+// Bound by the serial chain on one SM: 29 us (tridiagonalisation 14, Sturm 4.5,
+// inverse iteration to the basis 6, the launch and the row sums 4), 68 us with
+// block-wide phases for every step and the pivot form of the Sturm sequence.
+// Matrix rows in registers (one warp with a row per lane; eight lanes with
+// two barriers a step) were no faster: 22 and 16 us for the tridiagonalisation.
+constexpr int EJ_N = 25, EJ_TOP = 8, EJ_INV_ITERS = 2, EJ_MSEC_ROUNDS = 9;
+constexpr int EJ_HH = 224;  // threads of the tridiagonalisation: eight to a row
 
 // 1 / x to FP64 accuracy: the hardware approximation refined by two
 // Newton-Raphson steps r <- r + r (1 - x r), each doubling the correct bits.
@@ -235,11 +239,11 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
 // Number of eigenvalues of the symmetric tridiagonal (d, e) below x: the
 // signs of the pivots of T - x I (Sturm sequence); a pivot smaller than
 // pivmin in magnitude is replaced by -pivmin.
-__device__ __forceinline__ int sturm_count(const double* d, const double* ee, double x, double pivmin) {
+static __device__ __noinline__ int sturm_count_pivots(const double* d, const double* ee, double x, double pivmin) {
     double q = d[0] - x;
     if (fabs(q) < pivmin) q = -pivmin;
     int cnt = q < 0.0;
-#pragma unroll 8
+#pragma unroll 1
     for (int i = 1; i < EJ_N; i++) {
         q = fma(-ee[i - 1], rcp_nr(q), d[i] - x);
         if (fabs(q) < pivmin) q = -pivmin;
@@ -248,39 +252,66 @@ __device__ __forceinline__ int sturm_count(const double* d, const double* ee, do
     return cnt;
 }
 
-// sum_{i in [i0, i1)} a[i * sa] * b[i * sb] in four interleaved partial
-// FP64 chains (i - i0 mod 4), added in a fixed order: a quarter of the
-// latency of one chain
-__device__ __forceinline__ double dot4(const double* a, int sa, const double* b, int sb, int i0, int i1) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int i = i0;
-    for (; i + 4 <= i1; i += 4) {
-        s0 = fma(a[i * sa], b[i * sb], s0);
-        s1 = fma(a[(i + 1) * sa], b[(i + 1) * sb], s1);
-        s2 = fma(a[(i + 2) * sa], b[(i + 2) * sb], s2);
-        s3 = fma(a[(i + 3) * sa], b[(i + 3) * sb], s3);
+// The same as the sign changes of the leading minors p_i of T - x I,
+// p_i = (d_i - x) p_(i-1) - e_(i-1)^2 p_(i-2), for entries of T of at most 1 in
+// size (24 factors below 4 cannot overflow; both terms are rescaled by a power
+// of two every 8 steps against underflow). A zero minor between nonzero ones
+// counts once whichever sign it is given; a sequence that has run to zero is
+// counted by its pivots.
+__device__ __forceinline__ int sturm_count(const double* d, const double* ee, double x, double pivmin) {
+    double p0 = 1.0, p1 = d[0] - x;
+    unsigned cnt = unsigned(__double2hiint(p1)) >> 31;  // sign bits: the FP64 pipe is the limit here
+#pragma unroll 1  // a body of 8 steps stays in the instruction cache
+    for (int i0 = 1; i0 < EJ_N; i0 += 8) {
+#pragma unroll
+        for (int i = i0; i < i0 + 8; i++) {
+            const double p2 = fma(d[i] - x, p1, -(ee[i - 1] * p0));
+            cnt += unsigned(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+            p0 = p1;
+            p1 = p2;
+        }
+        const int ex = max(__double2hiint(p0) & 0x7fffffff, __double2hiint(p1) & 0x7fffffff) >> 20;  // biased exponent
+        const double sc = __hiloint2double((2046 - min(ex, 2045)) << 20, 0);                        // 2^(1023 - ex)
+        p0 *= sc;
+        p1 *= sc;
     }
-    if (i < i1) s0 = fma(a[i * sa], b[i * sb], s0);
-    if (i + 1 < i1) s1 = fma(a[(i + 1) * sa], b[(i + 1) * sb], s1);
-    if (i + 2 < i1) s2 = fma(a[(i + 2) * sa], b[(i + 2) * sb], s2);
-    return (s0 + s1) + (s2 + s3);
+    return p1 != 0.0 ? int(cnt) : sturm_count_pivots(d, ee, x, pivmin);
+}
+
+// sum_{j = 1..24} a[j] b[j] in four interleaved partial FP64 chains, added in
+// a fixed order: a quarter of the latency of one chain
+__device__ __forceinline__ double dot24(const double (&a)[EJ_N], const double (&b)[EJ_N]) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int j = 1; j < EJ_N; j++) s[j & 3] = fma(a[j], b[j], s[j & 3]);
+    return (s[1] + s[2]) + (s[3] + s[0]);
+}
+
+// the 25 values of a 16-byte aligned shared vector
+__device__ __forceinline__ void load25(const double* p, double (&v)[EJ_N]) {
+#pragma unroll
+    for (int j = 0; j < EJ_N - 1; j += 2) {
+        const double2 t = *reinterpret_cast<const double2*>(p + j);
+        v[j] = t.x;
+        v[j + 1] = t.y;
+    }
+    v[EJ_N - 1] = p[EJ_N - 1];
 }
 
 struct EigenSmem {
-    double acc[kPcaAcc];
-    double A[EJ_N][EJ_N + 1];       // covariance, reduced in place
-    double V[EJ_N - 2][EJ_N];       // Householder vectors (zero above k + 1)
-    double beta[EJ_N - 2], vk1[EJ_N - 2];
+    alignas(16) double V[EJ_N - 2][EJ_N + 1];  // Householder vectors (zero above k + 1)
+    double ax[EJ_N], w[EJ_N];                  // a tridiagonalisation step's vectors
+    alignas(16) double q[EJ_N + 1];            // the vector that Gram-Schmidt broadcasts
+    double A[EJ_N][EJ_N + 1];                  // covariance
+    double beta[EJ_N - 2];
     double d[EJ_N], e[EJ_N], ee[EJ_N];
-    double p[EJ_N], w[EJ_N];
-    double lam[EJ_TOP];
-    // inverse iteration, per eigenvector: the pivoted LU of T - lambda I
-    double u0[EJ_TOP][EJ_N], u1[EJ_TOP][EJ_N], u2[EJ_TOP][EJ_N], l[EJ_TOP][EJ_N], ru0[EJ_TOP][EJ_N];
-    double y[EJ_TOP][EJ_N];
-    unsigned char piv[EJ_TOP][EJ_N];
-    double Z[EJ_N][EJ_TOP + 1];     // eigenvectors of A, column c = the c-th largest
+    double lam[EJ_TOP], tnorm;
+    // inverse iteration, lane c for eigenvector c: the pivoted LU of T - lambda I
+    double ru0[EJ_N][EJ_TOP], u1[EJ_N][EJ_TOP], u2[EJ_N][EJ_TOP], l[EJ_N][EJ_TOP];
+    unsigned char piv[EJ_N][EJ_TOP];
+    double Z[EJ_N][EJ_TOP + 1];                // eigenvectors of A, column c = the c-th largest
     double work[200];
-    double part1[kPcaAcc], part2[kPcaAcc];
+    double acc[kPcaAcc], part1[kPcaAcc], part2[kPcaAcc];
     int bad;
 };
 
@@ -296,7 +327,7 @@ __device__ inline void pca_eigen_block(const double* __restrict__ part, int n_bl
         return;
     }
     // ---- partial rows summed in a fixed order: two halves of the row range
-    //      per accumulator, sixteen loads in flight each, then added
+    //      per accumulator, 32 loads in flight each, then added
     {
         const int half = (n_blocks + 1) / 2;
         for (int q = t; q < 2 * kPcaAcc; q += nth) {
@@ -304,13 +335,14 @@ __device__ inline void pca_eigen_block(const double* __restrict__ part, int n_bl
             const int b0 = h == 0 ? 0 : half, b1 = h == 0 ? half : n_blocks;
             double v = 0.0;
             int b = b0;
-            for (; b + 16 <= b1; b += 16) {  // sixteen loads in flight
-                double x[16];
+            for (; b + 32 <= b1; b += 32) {  // 32 loads in flight
+                double x[32];
 #pragma unroll
-                for (int k = 0; k < 16; k++) x[k] = part[size_t(b + k) * kPcaAcc + a];
+                for (int k = 0; k < 32; k++) x[k] = part[size_t(b + k) * kPcaAcc + a];
 #pragma unroll
-                for (int k = 0; k < 16; k++) v += x[k];
+                for (int k = 0; k < 32; k++) v += x[k];
             }
+#pragma unroll 4
             for (; b < b1; b++) v += part[size_t(b) * kPcaAcc + a];
             (h == 0 ? sm.part1 : sm.part2)[a] = v;
         }
@@ -329,87 +361,108 @@ __device__ inline void pca_eigen_block(const double* __restrict__ part, int n_bl
     }
     __syncthreads();
 
-    // ---- 1. Householder tridiagonalisation. Per step: thread 0 forms the
-    //         reflector from column k (a sequential FP64 norm); thread j > k
-    //         forms p_j = beta sum_i A[j][i] v_i; every thread forms
-    //         K = (beta / 2) p.v and updates its entries of the trailing
-    //         block, A' -= v w^T + w v^T with w = p - K v. v is column k below
-    //         the diagonal with its first entry replaced (vk1), read from A
-    //         itself; column k is outside every later trailing block.
-    for (int k = 0; k < EJ_N - 2; k++) {
-        if (t == 0) {
+    // ---- 1. Householder tridiagonalisation, eight lanes to a row. With x
+    //         column k below the diagonal, v = x - alpha e1, beta = 2 / v.v:
+    //         p = beta A v = beta (A x - alpha A e1), and v.A v = x.A x -
+    //         2 alpha (A x)_1 + alpha^2 A_11 (x.A e1 is (A x)_1), so A x and w are
+    //         the only vectors exchanged; w = p - (beta / 2) (p.v) v, then
+    //         A -= v w^T + w v^T on the trailing block.
+    if (t < EJ_HH) {
+        const int i = t >> 3, s8 = t & 7, row = min(i, EJ_N - 1);
+        auto bar = [] { asm volatile("bar.sync 1, %0;" ::"n"(EJ_HH) : "memory"); };
+        auto sum8 = [](double v) {  // over the row's eight lanes
+            v += __shfl_xor_sync(0xffffffffu, v, 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            return v + __shfl_xor_sync(0xffffffffu, v, 1);
+        };
+#pragma unroll 1
+        for (int k = 0; k < EJ_N - 2; k++) {
+            const bool below = i > k && i < EJ_N;
+            double x[3], a[3];
+#pragma unroll
+            for (int m = 0; m < 3; m++) {
+                const int j = k + 1 + s8 + 8 * m;
+                x[m] = j < EJ_N ? sm.A[j][k] : 0.0;
+                a[m] = j < EJ_N ? sm.A[row][j] : 0.0;
+            }
+            const double x1 = sm.A[k + 1][k], xi = sm.A[row][k], ai1 = sm.A[row][k + 1], a11 = sm.A[k + 1][k + 1];
+            const double n2 = sum8(fma(x[2], x[2], fma(x[1], x[1], x[0] * x[0])));
+            const double ax = sum8(fma(a[2], x[2], fma(a[1], x[1], a[0] * x[0])));
+            if (s8 == 0 && below) sm.ax[i] = ax;
             // the norm and 1 / (v.v / 2) by refined hardware approximations:
             // the IEEE square root and division are long serial sequences
-            // on this single thread's path
-            const double nrm2 = dot4(&sm.A[0][k], EJ_N + 1, &sm.A[0][k], EJ_N + 1, k + 1, EJ_N);
-            const double x1 = sm.A[k + 1][k];
-            const bool skip = !(nrm2 > 1e-280);
-            const double nrm = skip ? 0.0 : nrm2 * rsqrt_nr(nrm2);
+            const bool skip = !(n2 > 1e-280);  // the column is already reduced
+            const double nrm = skip ? 0.0 : n2 * rsqrt_nr(n2);
             const double alpha = x1 >= 0.0 ? -nrm : nrm;
-            const double den = nrm2 - alpha * x1;  // v.v / 2 > 0 unless the column is zero
-            sm.beta[k] = skip ? 0.0 : rcp_nr(den);
-            sm.vk1[k] = skip ? 0.0 : x1 - alpha;
-            sm.d[k] = sm.A[k][k];
-            sm.e[k] = skip ? x1 : alpha;
+            const double beta = skip ? 0.0 : rcp_nr(n2 - alpha * x1);  // v.v / 2 > 0 unless the column is zero
+            const double v1 = skip ? 0.0 : x1 - alpha;
+            bar();
+            double xy = 0.0;
+#pragma unroll
+            for (int m = 0; m < 3; m++) {
+                const int j = k + 1 + s8 + 8 * m;
+                if (j < EJ_N) xy = fma(x[m], sm.ax[j], xy);
+            }
+            const double vav = fma(alpha * alpha, a11, fma(-2.0 * alpha, sm.ax[k + 1], sum8(xy)));
+            const double K = 0.5 * beta * beta * vav;  // (beta / 2) p.v
+            const double v = skip || !below ? 0.0 : (i == k + 1 ? v1 : xi);
+            const double w = skip || !below ? 0.0 : beta * (ax - alpha * ai1) - K * v;
+            if (s8 == 0 && i < EJ_N) {
+                sm.w[i] = w;
+                sm.V[k][i] = v;
+            }
+            if (t == 0) {
+                sm.beta[k] = beta;
+                sm.d[k] = sm.A[k][k];
+                sm.e[k] = skip ? x1 : alpha;
+            }
+            bar();
+            if (below && !skip) {
+#pragma unroll
+                for (int m = 0; m < 3; m++) {
+                    const int j = k + 1 + s8 + 8 * m;
+                    if (j < EJ_N) sm.A[i][j] = a[m] - fma(v, sm.w[j], w * (j == k + 1 ? v1 : x[m]));
+                }
+            }
+            bar();
         }
-        __syncthreads();
-        const double beta = sm.beta[k];
-        if (t < EJ_N) sm.V[k][t] = beta == 0.0 || t <= k ? 0.0 : (t == k + 1 ? sm.vk1[k] : sm.A[t][k]);
-        if (beta == 0.0) continue;  // uniform: the column is already reduced
-        const double v1 = sm.vk1[k];
-        if (t > k && t < EJ_N)
-            sm.p[t] = beta * fma(sm.A[t][k + 1], v1, dot4(&sm.A[t][0], 1, &sm.A[0][k], EJ_N + 1, k + 2, EJ_N));
-        __syncthreads();
-        const double K = 0.5 * beta * fma(sm.p[k + 1], v1, dot4(sm.p, 1, &sm.A[0][k], EJ_N + 1, k + 2, EJ_N));
-        const int m = EJ_N - k - 1;
-        for (int q = t; q < m * m; q += nth) {
-            const int i = k + 1 + q / m, j = k + 1 + q % m;
-            const double vi = i == k + 1 ? v1 : sm.A[i][k], vj = j == k + 1 ? v1 : sm.A[j][k];
-            const double wi = sm.p[i] - K * vi, wj = sm.p[j] - K * vj;
-            sm.A[i][j] -= vi * wj + wi * vj;
+    }
+    if (warp == 0) {
+        if (lane == 0) {
+            sm.d[EJ_N - 2] = sm.A[EJ_N - 2][EJ_N - 2];
+            sm.d[EJ_N - 1] = sm.A[EJ_N - 1][EJ_N - 1];
+            sm.e[EJ_N - 2] = sm.A[EJ_N - 1][EJ_N - 2];
+            sm.e[EJ_N - 1] = 0.0;
         }
-        __syncthreads();
+        __syncwarp();
+        // T scaled by a power of two to a Gershgorin bound in [1/2, 1): exact, and
+        // neither the eigenvectors nor the rank threshold depend on it. Only the
+        // bound's exponent is needed: the largest high word
+        double b = 0.0;
+        if (lane < EJ_N) b = fabs(sm.d[lane]) + fabs(sm.e[lane]) + (lane > 0 ? fabs(sm.e[lane - 1]) : 0.0);
+        const unsigned ex = __reduce_max_sync(0xffffffffu, unsigned(__double2hiint(b))) >> 20;
+        const double sc = ex > 64 && ex < 2000 ? __hiloint2double((2045 - ex) << 20, 0) : 1.0;
+        if (lane < EJ_N) {
+            const double e = sm.e[lane] * sc;
+            sm.d[lane] *= sc;
+            sm.ee[lane] = e * e;
+            sm.e[lane] = e;
+        }
+        if (lane == 0) sm.tnorm = ex > 64 && ex < 2000 ? 1.0 : 0.0;  // 0: no eigenvalue to find
     }
-    if (t == 0) {
-        sm.d[EJ_N - 2] = sm.A[EJ_N - 2][EJ_N - 2];
-        sm.d[EJ_N - 1] = sm.A[EJ_N - 1][EJ_N - 1];
-        sm.e[EJ_N - 2] = sm.A[EJ_N - 1][EJ_N - 2];
-        sm.e[EJ_N - 1] = 0.0;
-    }
-    __syncthreads();
-    if (t < EJ_N) sm.ee[t] = sm.e[t] * sm.e[t];
     __syncthreads();
 
     // ---- 2. the 8 largest eigenvalues by Sturm multisection, warp w for
     //         eigenvalue index 24 - w (ascending)
-    double tnorm = 0.0, lo = 0.0, hi = 0.0;
-    {
-        double a = 0.0, b = 0.0, s = 0.0;
-        if (lane < EJ_N) {
-            const double r = fabs(sm.e[lane]) + (lane > 0 ? fabs(sm.e[lane - 1]) : 0.0);
-            a = sm.d[lane] - r;
-            b = sm.d[lane] + r;
-            s = fabs(sm.d[lane]) + r;
-        } else {
-            a = b = sm.d[0];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
-            b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-            s = fmax(s, __shfl_xor_sync(0xffffffffu, s, o));
-        }
-        tnorm = s;
-        const double pad = 2.2e-16 * fmax(tnorm, 1e-300) * EJ_N;
-        lo = a - pad;
-        hi = b + pad;
-    }
-    const double pivmin = fmax(1e-290, 1e-290 * tnorm * tnorm);
+    const double tnorm = sm.tnorm;
     if (warp < EJ_TOP) {
+        double lo = -tnorm, hi = tnorm;
+        constexpr double pivmin = 1e-290;
         const int m = EJ_N - 1 - warp;
+#pragma unroll 1
         for (int r = 0; r < EJ_MSEC_ROUNDS; r++) {
             if (!(hi - lo > 4.4e-16 * fmax(fabs(lo), fabs(hi)) + pivmin)) break;  // warp-uniform
-            const double x = lo + (hi - lo) * (double(lane + 1) / 33.0);
+            const double x = lo + (hi - lo) * (double(lane + 1) * (1.0 / 33.0));
             const int c = sturm_count(sm.d, sm.ee, x, pivmin);
             const unsigned above = __ballot_sync(0xffffffffu, c > m);
             const int first = above ? __ffs(above) - 1 : 32;
@@ -421,137 +474,143 @@ __device__ inline void pca_eigen_block(const double* __restrict__ part, int n_bl
         if (lane == 0) sm.lam[warp] = 0.5 * (lo + hi);
     }
     __syncthreads();
+    if (warp != 0) return;
 
-    // ---- 3. inverse iteration on T for eigenvector `warp` (lane 0)
-    if (warp < EJ_TOP && lane == 0) {
-        const int c = warp;
+    // ---- 3. inverse iteration on T, lane c for eigenvector c
+    const int c = min(lane, EJ_TOP - 1);
+    double y[EJ_N];
+    {
         const double lam = sm.lam[c];
         const double tiny = fmax(2.2e-16 * tnorm, 1e-290);
         // factor T - lam I = P L U (Gaussian elimination, partial pivoting);
-        // U has the diagonal u0 and two super-diagonals u1, u2
+        // U has the diagonal u0 (kept as 1 / u0) and two super-diagonals
         double a = sm.d[0] - lam, b = sm.e[0];
-        for (int k = 0; k < EJ_N - 1; k++) {
-            const double cl = sm.e[k];                 // sub-diagonal entry of row k + 1
-            const double an = sm.d[k + 1] - lam;       // diagonal of row k + 1
-            const double bn = k + 1 < EJ_N - 1 ? sm.e[k + 1] : 0.0;
-            if (fabs(a) >= fabs(cl)) {                 // no interchange
-                double piv = a;
+        if (lane < EJ_TOP) {
+#pragma unroll 4
+            for (int k = 0; k < EJ_N - 1; k++) {
+                const double cl = sm.e[k];                 // sub-diagonal entry of row k + 1
+                const double an = sm.d[k + 1] - lam;       // diagonal of row k + 1
+                const double bn = sm.e[k + 1];             // 0 for the last row
+                const bool swap = fabs(a) < fabs(cl);      // rows k and k + 1 interchanged
+                double piv = swap ? cl : a;
                 if (fabs(piv) < tiny) piv = piv < 0.0 ? -tiny : tiny;
                 const double rp = rcp_nr(piv);
-                const double mult = cl * rp;
-                sm.u0[c][k] = piv; sm.ru0[c][k] = rp; sm.u1[c][k] = b; sm.u2[c][k] = 0.0;
-                sm.l[c][k] = mult; sm.piv[c][k] = 0;
-                a = an - mult * b;
-                b = bn;
-            } else {                                   // rows k and k + 1 interchanged
-                const double pc = fabs(cl) < tiny ? (cl < 0.0 ? -tiny : tiny) : cl;
-                const double rp = rcp_nr(pc);
-                const double mult = a * rp;
-                sm.u0[c][k] = pc; sm.ru0[c][k] = rp; sm.u1[c][k] = an; sm.u2[c][k] = bn;
-                sm.l[c][k] = mult; sm.piv[c][k] = 1;
-                a = b - mult * an;
-                b = -mult * bn;
+                const double mult = (swap ? a : cl) * rp;
+                const double u1 = swap ? an : b, u2 = swap ? bn : 0.0;
+                sm.ru0[k][c] = rp;
+                sm.u1[k][c] = u1;
+                sm.u2[k][c] = u2;
+                sm.l[k][c] = mult;
+                sm.piv[k][c] = swap;
+                a = (swap ? b : an) - mult * u1;
+                b = (swap ? 0.0 : bn) - mult * u2;
             }
+            if (fabs(a) < tiny) a = a < 0.0 ? -tiny : tiny;
+            sm.ru0[EJ_N - 1][c] = rcp_nr(a);
         }
-        double piv = a;
-        if (fabs(piv) < tiny) piv = piv < 0.0 ? -tiny : tiny;
-        sm.u0[c][EJ_N - 1] = piv;
-        sm.ru0[c][EJ_N - 1] = rcp_nr(piv);
-        sm.u1[c][EJ_N - 1] = sm.u2[c][EJ_N - 1] = 0.0;
         // start vector of its own per eigenvector (deterministic)
-        double* y = sm.y[c];
-        for (int i = 0; i < EJ_N; i++) y[i] = 1.0 + 0.25 * double(((i + 1) * (7 + 4 * c)) % 13) / 13.0;
+#pragma unroll
+        for (int i = 0; i < EJ_N; i++) y[i] = 1.0 + (0.25 / 13.0) * double(((i + 1) * (7 + 4 * c)) % 13);
+        __syncwarp();
+#pragma unroll 1
         for (int it = 0; it < EJ_INV_ITERS; it++) {
-            for (int k = 0; k < EJ_N - 1; k++) {       // apply P and L^-1
-                if (sm.piv[c][k]) {
-                    const double tmp = y[k];
-                    y[k] = y[k + 1];
-                    y[k + 1] = tmp - sm.l[c][k] * y[k];
-                } else {
-                    y[k + 1] -= sm.l[c][k] * y[k];
-                }
+#pragma unroll
+            for (int k = 0; k < EJ_N - 1; k++) {           // apply P and L^-1
+                const bool swap = sm.piv[k][c];
+                const double up = swap ? y[k + 1] : y[k], dn = swap ? y[k] : y[k + 1];
+                y[k] = up;
+                y[k + 1] = dn - sm.l[k][c] * up;
             }
-            for (int k = EJ_N - 1; k >= 0; k--) {      // U^-1
-                double s = y[k];
-                if (k + 1 < EJ_N) s -= sm.u1[c][k] * y[k + 1];
-                if (k + 2 < EJ_N) s -= sm.u2[c][k] * y[k + 2];
-                y[k] = s * sm.ru0[c][k];
-            }
-            double mx = 0.0;                            // rescale by the largest entry
-            for (int i = 0; i < EJ_N; i++) mx = fmax(mx, fabs(y[i]));
+            y[EJ_N - 1] *= sm.ru0[EJ_N - 1][c];            // U^-1
+            y[EJ_N - 2] = (y[EJ_N - 2] - sm.u1[EJ_N - 2][c] * y[EJ_N - 1]) * sm.ru0[EJ_N - 2][c];
+#pragma unroll
+            for (int k = EJ_N - 3; k >= 0; k--)
+                y[k] = (fma(-sm.u2[k][c], y[k + 2], y[k]) - sm.u1[k][c] * y[k + 1]) * sm.ru0[k][c];
+            double m[4] = {0.0, 0.0, 0.0, 0.0};            // rescale by the largest entry
+#pragma unroll
+            for (int i = 0; i < EJ_N; i++) m[i & 3] = fmax(m[i & 3], fabs(y[i]));
+            const double mx = fmax(fmax(m[0], m[1]), fmax(m[2], m[3]));
             const double inv = mx > 1e-290 && mx < 1e300 ? rcp_nr(mx) : 0.0;
+#pragma unroll
             for (int i = 0; i < EJ_N; i++) y[i] *= inv;
         }
     }
-    __syncthreads();
-    // ---- 4. back-transform z = H_0 (H_1 (... H_22 y)), one reflector at a
-    //         time for the 8 vectors: thread c forms the dot product of
-    //         reflector k with vector c (a sequential FP64 chain, no warp
-    //         reduction), then the block updates the vectors
+    // ---- 4. back-transform z = H_0 (H_1 (... H_22 y)), lane c for vector c
+#pragma unroll 1
     for (int k = EJ_N - 3; k >= 0; k--) {
-        if (sm.beta[k] == 0.0) continue;  // uniform: the reflector is the identity
-        if (t < EJ_TOP) sm.p[t] = sm.beta[k] * dot4(sm.V[k], 1, sm.y[t], 1, k + 1, EJ_N);  // V[k][i] = 0 for i <= k
-        __syncthreads();
-        for (int q = t; q < EJ_TOP * EJ_N; q += nth) {
-            const int c = q / EJ_N, i = q % EJ_N;
-            if (i > k) sm.y[c][i] -= sm.p[c] * sm.V[k][i];
-        }
-        __syncthreads();
+        double v[EJ_N];
+        load25(sm.V[k], v);  // zero for entries <= k, all zero for a skipped column
+        const double s = sm.beta[k] * dot24(v, y);
+#pragma unroll
+        for (int i = 1; i < EJ_N; i++) y[i] = fma(-s, v[i], y[i]);
     }
-    // ---- 5. Gram-Schmidt in eigenvalue order, classical, twice per vector
-    //         (as stable as the modified form): the dot products of vector c
-    //         with the earlier ones by c threads at once, then the update by
-    //         row; exactly equal eigenvalues give an orthonormal basis of
-    //         their eigenspace, distinct ones are already orthogonal
-    for (int c = 0; c < EJ_TOP; c++) {
-        for (int pass = 0; pass < 2; pass++) {
-            if (c == 0) break;
-            if (t < c) sm.w[t] = dot4(sm.y[t], 1, sm.y[c], 1, 0, EJ_N);
-            __syncthreads();
-            if (t < EJ_N) {
-                double v = sm.y[c][t];
-                for (int k2 = 0; k2 < c; k2++) v -= sm.w[k2] * sm.y[k2][t];
-                sm.y[c][t] = v;
-            }
-            __syncthreads();
-        }
-        if (t == 0) {
-            const double nn = dot4(sm.y[c], 1, sm.y[c], 1, 0, EJ_N);
+    // ---- 5. normalisation; a non-finite vector is zeroed. Vectors of
+    //         eigenvalues 1e-7 of ||T|| apart are orthogonal to 2e-9 as they
+    //         are (rounding over the gap, below FP32); closer ones go through
+    //         Gram-Schmidt in eigenvalue order, vector g subtracted from the
+    //         later ones, twice
+    bool close = false;
+#pragma unroll
+    for (int k = 0; k + 1 < EJ_TOP; k++) close = close || !(sm.lam[k] - sm.lam[k + 1] > 1e-7);
+    const int steps = close ? 2 * EJ_TOP : 0;
+#pragma unroll 1
+    for (int step = -1; step < steps; step++) {
+        const int g = step < 0 ? -1 : step % EJ_TOP;
+        if (step < 0 || lane == g) {  // the first round normalises every vector
+            const double nn = fma(y[0], y[0], dot24(y, y));
             const bool ok = nn > 1e-290 && nn < 1e300;
-            sm.w[EJ_TOP] = ok ? rsqrt_nr(nn) : 0.0;
+            const double r = ok ? rsqrt_nr(nn) : 0.0;
             if (!ok) sm.bad = 1;
+#pragma unroll
+            for (int i = 0; i < EJ_N; i++) y[i] = ok ? y[i] * r : 0.0;
+            if (step >= 0) {
+#pragma unroll
+                for (int i = 0; i < EJ_N; i++) sm.q[i] = y[i];
+            }
         }
-        __syncthreads();
-        if (t < EJ_N) sm.y[c][t] = sm.w[EJ_TOP] != 0.0 ? sm.y[c][t] * sm.w[EJ_TOP] : 0.0;  // a non-finite vector is zeroed
-        __syncthreads();
+        if (step < 0) continue;
+        __syncwarp();
+        double q[EJ_N];
+        load25(sm.q, q);
+        const double s = lane > g ? fma(q[0], y[0], dot24(q, y)) : 0.0;
+#pragma unroll
+        for (int i = 0; i < EJ_N; i++) y[i] = fma(-s, q[i], y[i]);
+        __syncwarp();
     }
-    for (int q = t; q < EJ_TOP * EJ_N; q += nth) sm.Z[q % EJ_N][q / EJ_N] = sm.y[q / EJ_N][q % EJ_N];
-    __syncthreads();
     // ---- 6. select_pca_basis. When every eigenvalue is kept (the usual
     //         case) it reduces to signing each column by its largest-magnitude
-    //         entry (first on ties): thread c scans column c, then the block
-    //         writes the basis, with the same result
+    //         entry (first on ties), with the same result
     const double lam0 = sm.lam[0] > 0.0 ? sm.lam[0] : 0.0;
     bool all_kept = lam0 > 0.0;
-    for (int c = 0; c < EJ_TOP; c++) all_kept = all_kept && sm.lam[c] > 1e-9 * lam0;
+#pragma unroll
+    for (int k = 0; k < EJ_TOP; k++) all_kept = all_kept && sm.lam[k] > 1e-9 * lam0;
     if (all_kept) {
-        if (t < EJ_TOP) {
-            int amax = 0;
-            for (int r = 1; r < EJ_N; r++)
-                if (fabs(sm.y[t][r]) > fabs(sm.y[t][amax])) amax = r;
-            sm.w[t] = sm.y[t][amax] < 0 ? -1.0 : 1.0;
+        double mx = fabs(y[0]);
+        bool neg = y[0] < 0.0;
+#pragma unroll
+        for (int r = 1; r < EJ_N; r++)
+            if (fabs(y[r]) > mx) {
+                mx = fabs(y[r]);
+                neg = y[r] < 0.0;
+            }
+        if (lane < EJ_TOP) {
+#pragma unroll
+            for (int r = 0; r < EJ_N; r++) basis[r * EJ_TOP + lane] = float(neg ? -y[r] : y[r]);
         }
-        __syncthreads();
-        for (int q = t; q < EJ_N * EJ_TOP; q += nth) {
-            const int r = q / EJ_TOP, c = q % EJ_TOP;
-            basis[q] = float(sm.y[c][r] * sm.w[c]);
+    } else {
+        if (lane < EJ_TOP) {
+#pragma unroll
+            for (int r = 0; r < EJ_N; r++) sm.Z[r][lane] = y[r];
         }
-    } else if (t == 0) {
-        double ev[EJ_TOP];
-        for (int c = 0; c < EJ_TOP; c++) ev[c] = sm.lam[c];
-        select_pca_basis(ev, &sm.Z[0][0], EJ_TOP + 1, sm.work, basis);
+        __syncwarp();
+        if (lane == 0) {
+            double ev[EJ_TOP];
+            for (int k = 0; k < EJ_TOP; k++) ev[k] = sm.lam[k];
+            select_pca_basis(ev, &sm.Z[0][0], EJ_TOP + 1, sm.work, basis);
+        }
     }
-    if (t == 0 && status) *status = sm.bad ? -1 : EJ_INV_ITERS;
+    __syncwarp();
+    if (lane == 0 && status) *status = sm.bad ? -1 : EJ_INV_ITERS;
 }
 
 
