@@ -6,13 +6,11 @@
 //   w  = gaussian(0.1 |(i, j)|) * (lw, cw, cw)
 // accumulated in FP32; output (Y, Cb, Cr, sum of luma weights).
 //
-// Both kernels stage the tile's window region (halo 10) in shared memory
-// and give each thread a column of vertically adjacent pixels, which share
-// all but one of their window rows: one staged neighbour feeds several
-// taps. The kernel for the FP32 plain path evaluates the formula directly
-// with correctly rounded exponentials (parity with the oracle's FP32 run);
-// the FP16-storage path's kernel is arranged for the fewest FMA-pipe and
-// shared-memory operations per tap.
+// The kernels stage the tile's window region (halo 10) in shared memory. The
+// one for the FP32 plain path evaluates the formula directly with correctly
+// rounded exponentials (parity with the oracle's FP32 run), two vertically
+// adjacent pixels a thread; the FP16-storage path's forms the distances on the
+// tensor cores and the weights and sums in packed FP32.
 #include <cmath>
 
 #include <cstdlib>
@@ -65,6 +63,31 @@ __device__ __forceinline__ BmConst bm_const(const BlockMatchArgs& a, Plane<S, 2>
     k.s = dm0 / (1.f + a.gradient_boost * edge);
     k.c1 = dm1 / a.chroma_boost;
     k.c2 = dm2 / a.chroma_boost;
+    return k;
+}
+
+// The same for the FP16-storage path: reciprocals and square roots by rsqrtf
+// and __fdividef (a few 2^-24 each, FP32 throughout), inv[c] = 1 / a.tm[c] and
+// ib = 1 / chroma_boost formed once per thread: about 50 instructions a pixel
+// where the IEEE sequences take 200.
+__device__ __forceinline__ BmConst bm_const_h(const BlockMatchArgs& a, const float (&inv)[3], float ib,
+                                              Plane<__half, 2> grad, int w, int h, int px, int py, float y) {
+    BmConst k{};
+    float ls = 1.f;
+    if (a.lsc > 0.f) {  // lensShading, demosaic.metal:91-93, at the pixel
+        const float cx = float(w / 2), cy = float(h / 2);
+        const float dx = float(px) - cx, dy = float(py) - cy;
+        ls = 1.f + a.lsc * __fdividef(dx * dx + dy * dy, cx * cx + cy * cy);
+    }
+    const float r0 = rsqrtf(a.var_a[0] + a.var_b[0] * ls * y);
+    const float r1 = rsqrtf(a.var_a[1] + a.var_b[1] * ls * y);
+    const float r2 = rsqrtf(a.var_a[2] + a.var_b[2] * ls * y);
+    const f2 g = ld2<__half>(grad.px(px, py));
+    const float mag = sqrtf(g.x * g.x + g.y * g.y);
+    const float t = clampf((a.gradient_threshold * mag * r0 - 2.f) * (1.f / 14.f), 0.f, 1.f);  // smoothstep(2, 16, .)
+    k.s = __fdividef(inv[0] * r0, 1.f + a.gradient_boost * (t * t * (3.f - 2.f * t)));
+    k.c1 = inv[1] * r1 * ib;
+    k.c2 = inv[2] * r2 * ib;
     return k;
 }
 
@@ -183,41 +206,52 @@ __global__ void __launch_bounds__(256) k_block_match_plain(Plane<S, 4> img, Plan
 }
 
 // ============================================================ FP16-storage path
-// Four vertically adjacent pixels per thread (they share 18 of 24 window
-// rows; a staged neighbour feeds 3.5 taps on average), tile 32 x 32, 256
-// threads. Shared memory per window position: the PCA coefficients minus
-// the tile-centre pixel's, as 8 halves, and (Y, Cb, Cr, |q'|^2) in FP32.
-//   * |p - q|^2 = |p'|^2 + |q'|^2 - 2 p'.q' (an 8-FMA dot product, the
-//     -2 kl luma scale folded into the centre's coefficients); the
-//     centring keeps the cancellation error at FP32 rounding of the local
-//     variation of the coefficients;
-//   * lw is carried scaled by sqrt(2 log2 e), so the chroma exponent is
-//     three FMAs with log2(sw) folded in as the addend, and the luma weight
-//     is sw / sqrt(2 log2 e) times it;
-//   * both exponentials are ex2.approx (the reference uses half-precision
-//     exp under fast math here).
+// Distances on the tensor cores, weights and sums in packed FP32. A warp takes
+// a group of 4 x 2 pixels: the union of their windows is 24 x 22 positions, of
+// which each pixel's 21 x 21 window is 83.5%, walked as 33 tiles of 16
+// neighbours (2 rows x 8 columns). Per tile
+//   * S = |q'|^2 - 2 p'.q' for 16 neighbours x 8 pixels by one mma.sync
+//     m16n8k8: A holds the neighbours' centred coefficients (8 halves), B the
+//     pixels' times -2 (exact), C the neighbours' |q'|^2 in FP32. Products of
+//     halves are exact in FP32 and the sum is an FP32 sum, as the scalar form's;
+//     centring on the tile-centre pixel's coefficients keeps the cancellation
+//     error at FP32 rounding of the local variation of the coefficients;
+//   * a lane gets S of two horizontally adjacent pixels for each of two
+//     neighbours and evaluates both pixels' weights as packed FP32 pairs
+//     (fma/mul/add .rn.f32x2), the neighbour's values staged twice so that one
+//     load gives the broadcast pair: lw scaled by sqrt(2 log2 e) =
+//     exp2(kl S + base), chroma weight exp2(-(lw^2 + d1^2 + d2^2 - log2 sw)),
+//     both by ex2.approx.f32 (the reference uses half-precision exp under fast
+//     math here), then the five FP32 sums;
+//   * the spatial weight is separable. Its row part comes from a 23-entry table
+//     (weight 0, log-weight -inf outside the window's rows); its column part is
+//     fixed for a lane and column segment, so the sums are kept per segment
+//     and multiplied by it once at the end (0 outside the window's columns).
+// The lanes' sums are added over the 8 neighbour columns at the end.
+//
+// What bounds it: per tile and warp 8 ex2 (64 cycles of the sub-partition's
+// MUFU), 24 packed FP32 instructions (56 cycles of its FMA pipe) and about 46
+// issue slots, so the MUFU's 3.69 ms per 12 MP frame (5 levels) is the floor.
+// Measured: level 0 of a 2016x1512 image 1.25 ms (1.64 ms with the scalar
+// distance in packed FP32, four pixels a thread), 83 cycles a tile in the loop
+// (the mix of 8 ex2 and 24 packed FMA alone runs at about 70) and a quarter of
+// the time in staging, projection and the groups' ends; XU pipe 64% busy, issue
+// slots 59%. A 12 MP frame in a 6-frame batch: 8.35 -> 7.71 ms.
 constexpr int BX_TX = 32, BX_W = BX_TX + 20;
-// tile variants: TY thread rows of NP vertically adjacent pixels (NP = 4:
-// two pixel pairs per thread, NP = 2: one), tiles of 32 x (NP TY) = 32 x 32
-// or 32 x 16 pixels; the autotuner picks one per level size
-// (launch_block_match). Variant code 10 TY + NP: 84, 44, 82, 162.
+// tile variants: TY warps of 32 NP pixels, tiles of 32 x (NP TY) = 32 x 32 or
+// 32 x 16 pixels (bm_tile_variant chooses).
+// Variant code 10 TY + NP: 84, 44, 82, 162. A 32 x 32 tile's staging takes an
+// SM's shared memory alone, a 32 x 16 tile's half of it.
 template <int TY, int NP>
 struct BxTile {
-    static constexpr int H = NP * TY + 20;  // window rows staged
+    static constexpr int ROWS = NP * TY;
+    static constexpr int H = ROWS + 20;     // window rows staged
     static constexpr int LH = H + 4;        // luma rows staged
     static constexpr int THREADS = BX_TX * TY;
-    static constexpr int MIN_BLOCKS = THREADS >= 512 ? 1 : (NP == 4 && TY == 8 ? 2 : 3);
-    static_assert(NP == 2 || NP == 4, "one or two pixel pairs per thread");
-    static_assert(NP * TY == 16 || NP * TY == 32, "tile heights divide the 32-row centring tiles");
+    static constexpr int MIN_BLOCKS = ROWS == 16 ? 2 : 1;
+    static_assert(ROWS == 16 || ROWS == 32, "tile heights divide the 32-row centring tiles");
+    static_assert((BX_W * H) % 16 == 0, "the projection takes 16 positions at a time");
 };
-
-// ---------------------------------------------------------------- FFMA2 form
-// The four pixels of a thread are taken as two pairs, (p0, p1) and
-// (p2, p3), and every per-pixel FP32 operation of a pair is issued as one
-// packed FP32x2 instruction (fma/mul/add .rn.f32x2, sm_100a). The neighbour's values enter as broadcast pairs. A pair's
-// spatial weights come from one float4 of a 22 x 21 table indexed by the
-// pair's first window row (rows outside a pixel's window carry weight 0 and
-// log-weight -inf, which zero both of its weights).
 typedef unsigned long long u64;
 
 __device__ __forceinline__ u64 pk2(float a, float b) {
@@ -241,174 +275,293 @@ __device__ __forceinline__ u64 add2(u64 a, u64 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-
-template <int H>
-struct BmPairSmem {
-    uint4 pca[H * BX_W];   // q - c, 8 halves
-    float4 ycc[H * BX_W];  // Y, Cb, Cr, |q - c|^2
-    float4 sp[22 * 21];       // (sw(j)/sqrt(lk), sw(j-1)/sqrt(lk), -log2 sw(j), -log2 sw(j-1)), j = table row
-};
-
-struct BmPair {  // two pixels, each member of a pair register = one pixel
-    u64 p[8];             // -2 kl (p - c), per component
-    u64 kl, base;         // luma exponent terms
-    u64 c1, c2, no1, no2; // chroma: e = c * v - o  (no = -o)
-};
-
-template <bool A, bool B, class Sm>
-__device__ __forceinline__ void bmp2_row(const Sm& sm, int base, int r, const BmPair& pa, const BmPair& pb,
-                                         u64 (&acc)[2][5]) {
-    // unrolled 3 of the row's 21 taps: 0.9% faster per 12 MP frame than 7,
-    // 1.2% than 1, 1.6% than all 21 (which spills)
-#pragma unroll 3
-    for (int i = 0; i < 21; i++) {
-        const uint4 u = sm.pca[base + i];
-        const float2 a0 = __half22float2(u2h_(u.x)), a1 = __half22float2(u2h_(u.y));
-        const float2 a2 = __half22float2(u2h_(u.z)), a3 = __half22float2(u2h_(u.w));
-        const float4 y = sm.ycc[base + i];
-        const u64 q[8] = {pk2(a0.x, a0.x), pk2(a0.y, a0.y), pk2(a1.x, a1.x), pk2(a1.y, a1.y),
-                          pk2(a2.x, a2.x), pk2(a2.y, a2.y), pk2(a3.x, a3.x), pk2(a3.y, a3.y)};
-        const u64 yy = pk2(y.x, y.x), cb = pk2(y.y, y.y), cr = pk2(y.z, y.z), nn = pk2(y.w, y.w);
-        auto pair = [&](const BmPair& P, const float4 s, u64 (&ac)[5]) {
-            // ex = kl |q'|^2 - 2 kl p'.q' + base: the -2 kl scale rides in the
-            // stored coefficients and base starts the dot-product chain
-            u64 dot = fma2(q[0], P.p[0], P.base);
-#pragma unroll
-            for (int c = 1; c < 8; c++) dot = fma2(q[c], P.p[c], dot);
-            const u64 ex = fma2(P.kl, nn, dot);
-            float e0, e1;
-            upk2(ex, e0, e1);
-            float l0, l1;
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(l0) : "f"(fminf(e0, 2.f)));
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(l1) : "f"(fminf(e1, 2.f)));
-            const u64 lws = pk2(l0, l1);
-            const u64 d1 = fma2(P.c1, cb, P.no1), d2 = fma2(P.c2, cr, P.no2);
-            // q = lws^2 + d1^2 + d2^2 - log2 sw;  wc = exp2(-q)
-            const u64 q = fma2(lws, lws, fma2(d1, d1, fma2(d2, d2, pk2(s.z, s.w))));
-            float n0, n1;
-            upk2(q, n0, n1);
-            const float w0 = ex2_approx(-n0), w1 = ex2_approx(-n1);
-            const u64 wc = pk2(w0, w1);
-            const u64 wy = mul2(pk2(s.x, s.y), lws);
-            ac[0] = fma2(wy, yy, ac[0]);
-            ac[1] = fma2(wc, cb, ac[1]);
-            ac[2] = fma2(wc, cr, ac[2]);
-            ac[3] = add2(ac[3], wy);
-            ac[4] = add2(ac[4], wc);
-        };
-        if (A) pair(pa, sm.sp[r * 21 + i], acc[0]);
-        if (B) pair(pb, sm.sp[(r - 2) * 21 + i], acc[1]);
-    }
+__device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+__device__ __forceinline__ uint32_t hmul2_u(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0, float c0, float c1,
+                                        float c2, float c3) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(b0), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 
-// pcaProjection (demosaic.metal:774-796) fused into the tile producer: the
-// 5x5 luma patch of every window position times the 25 x 8 basis, as FP16
-// tensor-core MMAs (mma.sync m16n8k16, FP32 accumulate). 52 x 52 = 2704
-// positions = 169 chunks of 16 rows; K = 25 padded to 32 (two k-steps);
-// N = the 8 components. The luma tile (window region + 2) is staged once.
 constexpr int BX_LW = BX_W + 4;  // luma tile width, origin (x0 - 12, y0 - 12)
 
-__device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+enum { BK_KL, BK_BASE, BK_C1, BK_C2, BK_NO1, BK_NO2, BK_COUNT };
 
-// shared memory of one pair-form tile: the staged window region, the
-// centring vector and basis, then the luma tile (BX_LH x BX_LW halves)
+// shared memory of a tile
 template <int TY, int NP>
-struct BmPairTileSmem {
-    BmPairSmem<BxTile<TY, NP>::H> w;
+struct BmTileSmem {
+    using T = BxTile<TY, NP>;
+    uint4 q[T::H * BX_W];                  // q - c, 8 halves
+    float4 yb[T::H * BX_W];                // (Y, Y, Cb, Cb)
+    float2 cr[T::H * BX_W];                // (Cr, Cr)
+    float2 nn[T::H * BX_W];                // (|q - c|^2, the same)
+    float4 wrow[24];                       // row part of the spatial weight, dy = -11 .. 11: (-log2, -log2, w / sqrt(lk) twice)
+    float wcol[28];                        // column part, dx = -13 .. 13
     float cen[8];
     float bsm[25][8];
+    float k[BK_COUNT][T::ROWS * BX_TX];    // per pixel: kl, base, c1, c2, -c1 Cb, -c2 Cr
+    __half luma[2][T::LH * BX_LW];         // the luma tile, and the same shifted left by one
+    unsigned nn_max, kl_max;               // bits of the largest |q - c|^2 and |kl|
 };
-template <int TY, int NP>
-constexpr size_t bm_pair_smem_bytes() {
-    return sizeof(BmPairTileSmem<TY, NP>) + sizeof(__half) * BX_LW * BxTile<TY, NP>::LH;
+
+// a lane's view of a group: two adjacent pixels' constants as pairs
+struct BmPair {
+    u64 kl, base, c1, c2, no1, no2;
+};
+
+// The weights of a pixel pair for one neighbour and the five sums. S: the
+// pair's distances; yy, cb, cr: the neighbour's values; ly, sy: the row part of
+// the spatial weight, -log2 and over sqrt(lk).
+template <bool CLAMP>
+__device__ __forceinline__ void bm_accumulate(const BmPair& P, u64 S, u64 yy, u64 cb, u64 cr, u64 ly, u64 sy,
+                                              u64 (&acc)[5]) {
+    float e0, e1, l0, l1, n0, n1;
+    upk2(fma2(P.kl, S, P.base), e0, e1);
+    // the exponent is at most log2 sqrt(lk) but for rounding, held below 2
+    l0 = ex2_approx(CLAMP ? fminf(e0, 2.f) : e0);
+    l1 = ex2_approx(CLAMP ? fminf(e1, 2.f) : e1);
+    const u64 lws = pk2(l0, l1);
+    const u64 d1 = fma2(P.c1, cb, P.no1), d2 = fma2(P.c2, cr, P.no2);
+    upk2(fma2(lws, lws, fma2(d1, d1, fma2(d2, d2, ly))), n0, n1);
+    const u64 wc = pk2(ex2_approx(-n0), ex2_approx(-n1));
+    const u64 wy = mul2(sy, lws);
+    acc[0] = fma2(wy, yy, acc[0]);
+    acc[1] = fma2(wc, cb, acc[1]);
+    acc[2] = fma2(wc, cr, acc[2]);
+    acc[3] = add2(acc[3], wy);
+    acc[4] = add2(acc[4], wc);
 }
 
-// One tile (origin x0, y0) of the pair form by TY x 32 threads; the thread
-// is (tcol, trow) of the tile. Shared by the stream kernel and the
+__device__ __forceinline__ u64 as_u64(float2 v) { return pk2(v.x, v.y); }
+
+// The sums of one group (pixel origin gx, gy in the tile). SAFE: positions
+// outside a pixel's window are read as 0, so that a value that is not finite
+// reaches the pixels whose windows hold it and no others. CLAMP: the luma
+// exponents may round past their limit.
+template <bool SAFE, bool CLAMP, class Sm>
+__device__ __forceinline__ void bm_group(const Sm& sm, int gx, int gy, u64 (&acc)[3][5]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    BmPair P;
+    {
+        const int i = (gy + (t >> 1)) * BX_TX + gx + 2 * (t & 1);
+        auto pair = [&](int c) { return as_u64(*reinterpret_cast<const float2*>(&sm.k[c][i])); };
+        P = {pair(BK_KL), pair(BK_BASE), pair(BK_C1), pair(BK_C2), pair(BK_NO1), pair(BK_NO2)};
+    }
+    // B: pixel g's coefficients 2t, 2t + 1 times -2
+    const uint32_t* q32 = reinterpret_cast<const uint32_t*>(sm.q);
+    const uint32_t bq = hmul2_u(q32[((gy + (g >> 2) + 10) * BX_W + gx + (g & 3) + 10) * 4 + t], 0xc000c000u);
+#pragma unroll
+    for (int k = 0; k < 15; k++) acc[k / 5][k % 5] = 0;
+    // neighbour g of a tile's first row; ldmatrix: lanes 0-7 the first row's
+    // eight positions, lanes 8-15 the second row's
+    int pos = gy * BX_W + gx + g;
+    uint32_t lda = uint32_t(__cvta_generic_to_shared(&sm.q[(gy + ((lane >> 3) & 1)) * BX_W + gx + (lane & 7)]));
+    const float4* wr = &sm.wrow[1 - (t >> 1)];
+#pragma unroll 1
+    for (int r = 0; r < 11; r++, pos += 2 * BX_W, lda += 2 * BX_W * 16, wr += 2) {
+        const float4 w0 = wr[0], w1 = wr[1];
+#pragma unroll
+        for (int s = 0; s < 3; s++) {
+            uint32_t a0, a1;
+            asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];"
+                         : "=r"(a0), "=r"(a1)
+                         : "r"(lda + 8 * 16 * s));
+            const int p0 = pos + 8 * s, p1 = p0 + BX_W;
+            const float2 m0 = sm.nn[p0], m1 = sm.nn[p1];
+            float S[4];
+            mma1688(S, a0, a1, bq, m0.x, m0.y, m1.x, m1.y);
+            float4 y0 = sm.yb[p0], y1 = sm.yb[p1];
+            float2 c0 = sm.cr[p0], c1 = sm.cr[p1];
+            if constexpr (SAFE) {
+                const int dx = 8 * s + g - 2 * (t & 1) - 10, dy = 2 * r - (t >> 1) - 10;
+                auto zero = [&](float4& y, float2& c, float& s0, float& s1, int d) {
+                    const bool row = d >= -10 && d <= 10, in0 = row && dx >= -10 && dx <= 10,
+                               in1 = row && dx - 1 >= -10 && dx - 1 <= 10;
+                    y.x = in0 ? y.x : 0.f, y.z = in0 ? y.z : 0.f, c.x = in0 ? c.x : 0.f, s0 = in0 ? s0 : 0.f;
+                    y.y = in1 ? y.y : 0.f, y.w = in1 ? y.w : 0.f, c.y = in1 ? c.y : 0.f, s1 = in1 ? s1 : 0.f;
+                };
+                zero(y0, c0, S[0], S[1], dy);
+                zero(y1, c1, S[2], S[3], dy + 1);
+            }
+            bm_accumulate<CLAMP>(P, pk2(S[0], S[1]), pk2(y0.x, y0.y), pk2(y0.z, y0.w), as_u64(c0),
+                                 pk2(w0.x, w0.y), pk2(w0.z, w0.w), acc[s]);
+            bm_accumulate<CLAMP>(P, pk2(S[2], S[3]), pk2(y1.x, y1.y), pk2(y1.z, y1.w), as_u64(c1),
+                                 pk2(w1.x, w1.y), pk2(w1.z, w1.w), acc[s]);
+        }
+    }
+}
+
+// A warp's share of the tile's groups, the results into shared memory.
+template <bool SAFE, bool CLAMP, int TY, class Sm>
+__device__ __forceinline__ void bm_groups(Sm& sm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    constexpr int GROUPS = (BX_TX / 4) * (Sm::T::ROWS / 2);
+    // the column part of the spatial weight: neighbour g of each segment,
+    // pixel columns 2 (t & 1) and 2 (t & 1) + 1
+    u64 sx[3];
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+        const float* w = &sm.wcol[8 * s + g - 2 * (t & 1) - 10 + 13];
+        sx[s] = pk2(w[0], w[-1]);
+    }
+    const bool second = lane & 16;
+#pragma unroll 1
+    for (int grp = warp; grp < GROUPS; grp += TY) {
+        const int gx = (grp % (BX_TX / 4)) * 4, gy = (grp / (BX_TX / 4)) * 2;
+        u64 part[3][5];
+        bm_group<SAFE, CLAMP>(sm, gx, gy, part);
+        // over the eight neighbour columns: lanes of the lower half keep the
+        // first pixel of their pair, those of the upper half the second
+        float v[5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            float u0, u1;
+            upk2(fma2(sx[2], part[2][k], fma2(sx[1], part[1][k], mul2(sx[0], part[0][k]))), u0, u1);
+            v[k] = (second ? u1 : u0) + __shfl_xor_sync(0xffffffffu, second ? u0 : u1, 16);
+        }
+#pragma unroll
+        for (int k = 0; k < 5; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], 8);
+#pragma unroll
+        for (int k = 0; k < 5; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], 4);
+        // into the place of the pixel's constants, which only this group reads
+        if ((lane & 12) == 0) {
+            const int i = (gy + (t >> 1)) * BX_TX + gx + 2 * (t & 1) + second;
+#pragma unroll
+            for (int k = 0; k < 5; k++) sm.k[k][i] = v[k];
+        }
+    }
+}
+
+// One tile (origin x0, y0) by TY warps. Shared by the stream kernel and the
 // persistent kernel's block-matching tasks.
 template <int TY, int NP>
-__device__ __forceinline__ void bm_pair_tile(int x0, int y0, int tcol, int trow, const Plane<__half, 4>& img,
-                                             const Plane<__half, 2>& grad, const float* __restrict__ basis,
-                                             const Plane<__half, 4>& out, const BlockMatchArgs& a,
-                                             unsigned char* smem_raw) {
+__device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& img, const Plane<__half, 2>& grad,
+                                        const float* __restrict__ basis, const Plane<__half, 4>& out,
+                                        const BlockMatchArgs& a, BmTileSmem<TY, NP>& sm) {
     using T = BxTile<TY, NP>;
-    constexpr int BX_H = T::H, BX_LH = T::LH, NT = T::THREADS, BX_NP = NP;
-    BmPairTileSmem<TY, NP>& st = *reinterpret_cast<BmPairTileSmem<TY, NP>*>(smem_raw);
-    BmPairSmem<BX_H>& sm = st.w;
-    __half* luma = reinterpret_cast<__half*>(smem_raw + sizeof(BmPairTileSmem<TY, NP>));  // BX_LH x BX_LW
-    float* cen = st.cen;
-    float (*bsm)[8] = st.bsm;
-    const int tid = trow * BX_TX + tcol;
+    constexpr int NT = T::THREADS, NPOS = BX_W * T::H;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const float kLog2e = 1.4426950408889634f, lk = 2.f * kLog2e, isq = rsqrtf(lk);
-    for (int k = tid; k < 22 * 21; k += NT) {
-        const int j = k / 21, i = k % 21 - 10;
-        // window row j of the pair's first pixel, j - 1 of its second
-        const float w0 = j <= 20 ? spatial_weight(i, j - 10) : 0.f;
-        const float w1 = j >= 1 ? spatial_weight(i, j - 11) : 0.f;
-        sm.sp[k] = make_float4(w0 * isq, w1 * isq, -log2f(w0), -log2f(w1));
+    const float inf = __int_as_float(0x7f800000);
+    if (tid < 27) {
+        const int d = tid - 13;
+        sm.wcol[tid] = d >= -10 && d <= 10 ? spatial_weight(d, 0) : 0.f;
+    } else if (tid >= 32 && tid < 32 + 23) {
+        const int d = tid - 32 - 11;
+        const float w = d >= -10 && d <= 10 ? spatial_weight(0, d) : 0.f, l = w > 0.f ? -log2f(w) : inf;
+        sm.wrow[tid - 32] = make_float4(l, l, w * isq, w * isq);
     }
-    for (int k = tid; k < 200; k += NT) bsm[k / 8][k % 8] = basis[k];
-    for (int k = tid; k < BX_LW * BX_LH; k += NT) {
-        const int ty = k / BX_LW, tx = k % BX_LW;
-        luma[k] = *img.pxc(x0 - 12 + tx, y0 - 12 + ty);
-    }
-    for (int k = tid; k < BX_W * BX_H; k += NT) {
-        const int ty = k / BX_W, tx = k % BX_W;
-        const f4 p = ld4<__half>(img.pxc(x0 - 10 + tx, y0 - 10 + ty));
-        sm.ycc[k] = make_float4(p.x, p.y, p.z, 0.f);
+    for (int k = tid; k < 200; k += NT) sm.bsm[k / 8][k % 8] = basis[k];
+    if (tid == 0) sm.nn_max = sm.kl_max = 0;
+    // the window region plus the patches' margin of 2, a warp per row
+    bool bad = false;  // a staged value that is not finite
+#pragma unroll
+    for (int i = 0; i < (T::LH + TY - 1) / TY; i++) {  // unrolled: all of a warp's loads in flight
+        const int ty = warp + i * TY;
+        if (ty >= T::LH) break;
+        const __half* row = img.px(0, clampi(y0 - 12 + ty, 0, img.h - 1));
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int tx = lane + 32 * h;
+            if (tx >= BX_LW) break;
+            const __half* src = row + 4 * clampi(x0 - 12 + tx, 0, img.w - 1);
+            const __half y = *src;
+            const f4 p = ld4<__half>(src);
+            const int l = ty * BX_LW + tx, k = (ty - 2) * BX_W + tx - 2;
+            sm.luma[0][l] = y;
+            if (tx > 0) sm.luma[1][l - 1] = y;
+            bad = bad || !(fabsf(p.x) + fabsf(p.y) + fabsf(p.z) < inf);
+            if (ty >= 2 && ty < T::H + 2 && tx >= 2 && tx < BX_W + 2) {
+                sm.yb[k] = make_float4(p.x, p.x, p.y, p.y);
+                sm.cr[k] = make_float2(p.z, p.z);
+            }
+        }
     }
     __syncthreads();
     if (tid < 8) {  // centring vector: the coefficients (FP32) of the centre pixel of the
                     // enclosing 32 x 32 tile, so that both tile heights centre and round alike
         const int cx = BX_TX / 2 + 12, cy = 16 + 12 - (y0 % 32);  // luma-tile coordinates
         float c = 0.f;
-        for (int k = 0; k < 25; k++) c += bsm[k][tid] * __half2float(luma[(cy + k / 5 - 2) * BX_LW + cx + k % 5 - 2]);
-        cen[tid] = c;
+        for (int k = 0; k < 25; k++)
+            c += sm.bsm[k][tid] * __half2float(sm.luma[0][(cy + k / 5 - 2) * BX_LW + cx + k % 5 - 2]);
+        sm.cen[tid] = c;
     }
-    // B fragments (basis, k x n, "col" layout): rows 2t, 2t+1, 2t+8, 2t+9 of column g, per k-step
-    const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    uint32_t bf[2][2];
+    // pcaProjection (demosaic.metal:774-796) fused into the tile producer: the
+    // 5x5 luma patch of every window position times the 25 x 8 basis, as FP16
+    // tensor-core MMAs (mma.sync m16n8k16, FP32 accumulate), 16 positions at a
+    // time. K runs over the patch rows padded to 6 (15 pairs, and one of
+    // zeros): an A register is two adjacent luma values, one aligned 32-bit
+    // load from the copy of the tile that suits the position's parity. The
+    // padding is masked, not only multiplied by 0. B fragments (basis, k x n,
+    // "col" layout): rows 2t, 2t+1, 2t+8, 2t+9 of column g, per k-step
+    uint32_t bf[2][2], mask[4];
+    int off[4];
 #pragma unroll
-    for (int s = 0; s < 2; s++) {
-        auto bk = [&](int k) { return k < 25 ? bsm[k][g] : 0.f; };
-        const int k0 = 16 * s + 2 * t;
-        bf[s][0] = h2u(__floats2half2_rn(bk(k0), bk(k0 + 1)));
-        bf[s][1] = h2u(__floats2half2_rn(bk(k0 + 8), bk(k0 + 9)));
+    for (int n = 0; n < 4; n++) {
+        const int pr = 4 * n + t, dy = pr / 3, j = pr % 3;  // the lane's pairs t, 4 + t, 8 + t, 12 + t
+        const bool in = pr < 15;
+        off[n] = in ? 2 * (dy * BX_LW + 2 * j) : 0;  // bytes
+        mask[n] = in ? (j == 2 ? 0x0000ffffu : 0xffffffffu) : 0u;
+        const float b0 = in ? sm.bsm[5 * dy + 2 * j][g] : 0.f, b1 = in && j < 2 ? sm.bsm[5 * dy + 2 * j + 1][g] : 0.f;
+        bf[n >> 1][n & 1] = h2u(__floats2half2_rn(b0, b1));
     }
     __syncthreads();
-    uint32_t* pca32 = reinterpret_cast<uint32_t*>(sm.pca);  // [position][4] half2
-    for (int ch = warp; ch < (BX_W * BX_H) / 16; ch += TY) {
+    uint32_t* q32 = reinterpret_cast<uint32_t*>(sm.q);  // [position][4] half2
+    const float cen0 = sm.cen[2 * t], cen1 = sm.cen[2 * t + 1];
+    float nmax = 0.f;
+    // window positions that lie outside the image take its edge's patches
+    const bool inner = x0 >= 10 && y0 >= 10 && x0 + BX_W - 10 <= img.w && y0 + T::H - 10 <= img.h;
+    int mx[2], my[2];  // window column and row of this thread's two positions of a chunk
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        mx[e] = (warp * 16 + g + 8 * e) % BX_W;
+        my[e] = (warp * 16 + g + 8 * e) / BX_W;
+    }
+    const uint32_t luma0 = uint32_t(__cvta_generic_to_shared(sm.luma[0]));
+    for (int ch = warp; ch < NPOS / 16; ch += TY) {
         const int m0 = ch * 16 + g, m1 = m0 + 8;  // the two rows of this thread
-        // patch centre in the luma tile: the clamped image position of the
-        // window position, as a clamped read of a projected plane would see
-        auto lidx = [&](int m) {
-            const int px = clampi(x0 - 10 + m % BX_W, 0, img.w - 1) - (x0 - 12);
-            const int py = clampi(y0 - 10 + m / BX_W, 0, img.h - 1) - (y0 - 12);
-            return py * BX_LW + px;
+        // first pair of the patch in the luma tile, around the clamped image
+        // position of the window position, as a clamped read of a projected
+        // plane would see
+        auto first = [&](int e) {
+            int px = mx[e], py = my[e];
+            if (!inner) {
+                px = clampi(x0 - 10 + px, 0, img.w - 1) - (x0 - 10);
+                py = clampi(y0 - 10 + py, 0, img.h - 1) - (y0 - 10);
+            }
+            mx[e] += 16 * TY % BX_W;  // on to the next chunk
+            my[e] += 16 * TY / BX_W;
+            if (mx[e] >= BX_W) mx[e] -= BX_W, my[e]++;
+            // odd columns: the second copy, one half lower
+            return luma0 + uint32_t((px & 1) * (T::LH * BX_LW - 1) + py * BX_LW + px) * 2;
         };
-        const int l0 = lidx(m0), l1 = lidx(m1);
-        auto av = [&](int l, int k) {  // patch element k of the position at luma index l
-            return k < 25 ? luma[l + (k / 5 - 2) * BX_LW + (k % 5 - 2)] : __float2half(0.f);
+        const uint32_t l0 = first(0), l1 = first(1);
+        auto av = [&](uint32_t l, int n) {
+            uint32_t v;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(l + off[n]));
+            return v & mask[n];
         };
         float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int s = 0; s < 2; s++) {
-            const int k0 = 16 * s + 2 * t;
-            const uint32_t a0 = h2u(__halves2half2(av(l0, k0), av(l0, k0 + 1)));
-            const uint32_t a1 = h2u(__halves2half2(av(l1, k0), av(l1, k0 + 1)));
-            const uint32_t a2 = h2u(__halves2half2(av(l0, k0 + 8), av(l0, k0 + 9)));
-            const uint32_t a3 = h2u(__halves2half2(av(l1, k0 + 8), av(l1, k0 + 9)));
             asm volatile(
                 "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                 "{%0,%1,%2,%3};"
                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(bf[s][0]), "r"(bf[s][1]));
+                : "r"(av(l0, 2 * s)), "r"(av(l1, 2 * s)), "r"(av(l0, 2 * s + 1)), "r"(av(l1, 2 * s + 1)),
+                  "r"(bf[s][0]), "r"(bf[s][1]));
         }
         // rows m0 (c0, c1) and m1 (c2, c3), components 2t, 2t+1; centre, round, store
-        const __half2 h0 = __floats2half2_rn(c[0] - cen[2 * t], c[1] - cen[2 * t + 1]);
-        const __half2 h1 = __floats2half2_rn(c[2] - cen[2 * t], c[3] - cen[2 * t + 1]);
-        pca32[m0 * 4 + t] = h2u(h0);
-        pca32[m1 * 4 + t] = h2u(h1);
+        const __half2 h0 = __floats2half2_rn(c[0] - cen0, c[1] - cen1);
+        const __half2 h1 = __floats2half2_rn(c[2] - cen0, c[3] - cen1);
+        q32[m0 * 4 + t] = h2u(h0);
+        q32[m1 * 4 + t] = h2u(h1);
         const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
         float n0 = f0.x * f0.x + f0.y * f0.y, n1 = f1.x * f1.x + f1.y * f1.y;
         n0 += __shfl_xor_sync(0xffffffffu, n0, 1);
@@ -416,93 +569,83 @@ __device__ __forceinline__ void bm_pair_tile(int x0, int y0, int tcol, int trow,
         n1 += __shfl_xor_sync(0xffffffffu, n1, 1);
         n1 += __shfl_xor_sync(0xffffffffu, n1, 2);
         if (t == 0) {
-            sm.ycc[m0].w = n0;
-            sm.ycc[m1].w = n1;
+            sm.nn[m0] = make_float2(n0, n0);
+            sm.nn[m1] = make_float2(n1, n1);
         }
+        nmax = fmaxf(nmax, n0 + n1);
+        bad = bad || !(n0 + n1 < inf);
+    }
+    {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(nmax));  // not negative
+        if (lane == 0) atomicMax(&sm.nn_max, m);
     }
     __syncthreads();
-    const int x = x0 + tcol, y = y0 + BX_NP * trow;
-    float pc[BX_NP][8], kl[BX_NP], base[BX_NP], c1[BX_NP], c2[BX_NP], o1[BX_NP], o2[BX_NP];
-#pragma unroll
-    for (int p = 0; p < BX_NP; p++) {
-        const int c = (BX_NP * trow + p + 10) * BX_W + tcol + 10;
-        const float4 in = sm.ycc[c];
-        const uint4 u = sm.pca[c];
-        const float2 a0 = __half22float2(u2h_(u.x)), a1 = __half22float2(u2h_(u.y));
-        const float2 a2 = __half22float2(u2h_(u.z)), a3 = __half22float2(u2h_(u.w));
-        pc[p][0] = a0.x; pc[p][1] = a0.y; pc[p][2] = a1.x; pc[p][3] = a1.y;
-        pc[p][4] = a2.x; pc[p][5] = a2.y; pc[p][6] = a3.x; pc[p][7] = a3.y;
+    // the pixels' constants, once each
+    const float inv[3] = {1.f / a.tm[0], 1.f / a.tm[1], 1.f / a.tm[2]}, ib = 1.f / a.chroma_boost;
+    float kmax = 0.f;
+    for (int i = tid; i < T::ROWS * BX_TX; i += NT) {
+        const int px = i % BX_TX, py = i / BX_TX;
+        const int c = (py + 10) * BX_W + px + 10;
+        const float4 yb = sm.yb[c];
+        const float cr = sm.cr[c].x;
         const BmConst k =
-            bm_const<__half>(a, grad, img.w, img.h, min(x, img.w - 1), min(y + p, img.h - 1), in.x, in.y, in.z);
-        kl[p] = fmaxf(-2.f * kLog2e * k.s * k.s, -1e30f);
-        base[p] = fmaf(kl[p], in.w, 0.5f * log2f(lk));
-        const float sq = sqrtf(lk);
-        c1[p] = sq * k.c1;
-        c2[p] = sq * k.c2;
-        o1[p] = c1[p] * in.y;
-        o2[p] = c2[p] * in.z;
+            bm_const_h(a, inv, ib, grad, img.w, img.h, min(x0 + px, img.w - 1), min(y0 + py, img.h - 1), yb.x);
+        const float kl = fmaxf(-2.f * kLog2e * k.s * k.s, -1e30f), sq = sqrtf(lk);
+        const float c1 = sq * k.c1, c2 = sq * k.c2;
+        sm.k[BK_KL][i] = kl;
+        sm.k[BK_BASE][i] = fmaf(kl, sm.nn[c].x, 0.5f * log2f(lk));
+        sm.k[BK_C1][i] = c1;
+        sm.k[BK_C2][i] = c2;
+        sm.k[BK_NO1][i] = -c1 * yb.z;
+        sm.k[BK_NO2][i] = -c2 * cr;
+        kmax = fmaxf(kmax, -kl);
+        bad = bad || !(kl <= 0.f);
     }
-    BmPair PP[NP / 2];
-#pragma unroll
-    for (int q = 0; q < NP / 2; q++) {
-        for (int c = 0; c < 8; c++) PP[q].p[c] = pk2(-2.f * kl[2 * q] * pc[2 * q][c], -2.f * kl[2 * q + 1] * pc[2 * q + 1][c]);
-        PP[q].kl = pk2(kl[2 * q], kl[2 * q + 1]);
-        PP[q].base = pk2(base[2 * q], base[2 * q + 1]);
-        PP[q].c1 = pk2(c1[2 * q], c1[2 * q + 1]);
-        PP[q].c2 = pk2(c2[2 * q], c2[2 * q + 1]);
-        PP[q].no1 = pk2(-o1[2 * q], -o1[2 * q + 1]);
-        PP[q].no2 = pk2(-o2[2 * q], -o2[2 * q + 1]);
+    {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(kmax));
+        if (lane == 0) atomicMax(&sm.kl_max, m);
     }
-    u64 acc[2][5];
-    for (int k = 0; k < 5; k++) acc[0][k] = acc[1][k] = pk2(0.f, 0.f);
-    const int col = tcol, row0 = BX_NP * trow;
-    auto rb = [&](int r) { return (row0 + r) * BX_W + col; };
-    const BmPair& PA = PP[0];
-    const BmPair& PB = PP[NP / 2 - 1];  // the second pair (unused when NP = 2)
-    if constexpr (NP == 4) {
-        bmp2_row<true, false>(sm, rb(0), 0, PA, PB, acc);
-        bmp2_row<true, false>(sm, rb(1), 1, PA, PB, acc);
-        for (int r = 2; r <= 21; r++) bmp2_row<true, true>(sm, rb(r), r, PA, PB, acc);
-        bmp2_row<false, true>(sm, rb(22), 22, PA, PB, acc);
-        bmp2_row<false, true>(sm, rb(23), 23, PA, PB, acc);
-    } else {
-        for (int r = 0; r <= 21; r++) bmp2_row<true, false>(sm, rb(r), r, PA, PB, acc);
-    }
-    float v[2][5][2];
-    for (int q = 0; q < 2; q++)
-        for (int k = 0; k < 5; k++) upk2(acc[q][k], v[q][k][0], v[q][k][1]);
-    if (x < out.w) {
-#pragma unroll
-        for (int p = 0; p < BX_NP; p++) {
-            const int q = p >> 1, m = p & 1;
-            if (y + p < out.h)
-                st4<__half>(out.px(x, y + p), f4{v[q][0][m] / v[q][3][m], v[q][1][m] / v[q][4][m],
-                                                 v[q][2][m] / v[q][4][m], v[q][3][m]});
-        }
+    const bool safe = __syncthreads_or(bad);
+    // S is not negative but for the rounding of its terms, below 2^-18 of the
+    // largest |q'|^2: the exponents stay below log2 sqrt(lk) + 1 < 2 unasked
+    // unless the tile's kl are extreme
+    const bool clamp = !(__uint_as_float(sm.nn_max) * __uint_as_float(sm.kl_max) < 0x1p18f);
+    if (safe) bm_groups<true, true, TY>(sm);
+    else if (clamp) bm_groups<false, true, TY>(sm);
+    else bm_groups<false, false, TY>(sm);
+    __syncthreads();
+    for (int i = tid; i < T::ROWS * BX_TX; i += NT) {
+        const int x = x0 + i % BX_TX, y = y0 + i / BX_TX;
+        if (x >= out.w || y >= out.h) continue;
+        const float ny = sm.k[3][i], nc = sm.k[4][i];
+        // sums that vanish: at scales where the distance's rounding alone
+        // exceeds the exponent's range even the pixel's own weight is lost
+        const int c = (i / BX_TX + 10) * BX_W + i % BX_TX + 10;
+        const float vy = ny != 0.f ? sm.k[0][i] / ny : sm.yb[c].x;
+        const float vb = nc != 0.f ? sm.k[1][i] / nc : sm.yb[c].z, vr = nc != 0.f ? sm.k[2][i] / nc : sm.cr[c].x;
+        st4<__half>(out.px(x, y), f4{vy, vb, vr, ny});
     }
 }
-
 
 template <int TY, int NP>
 __global__ void __launch_bounds__(BxTile<TY, NP>::THREADS, BxTile<TY, NP>::MIN_BLOCKS)
     k_block_match_pair(Plane<__half, 4> img, Plane<__half, 2> grad, const float* __restrict__ basis,
                        Plane<__half, 4> out, BlockMatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    bm_pair_tile<TY, NP>(blockIdx.x * BX_TX, blockIdx.y * (NP * TY), threadIdx.x, threadIdx.y, img, grad, basis, out,
-                         a, smem_raw);
+    bm_tile<TY, NP>(blockIdx.x * BX_TX, blockIdx.y * (NP * TY), img, grad, basis, out, a,
+                    *reinterpret_cast<BmTileSmem<TY, NP>*>(smem_raw));
 }
 
 template <int TY, int NP>
 static void launch_pair(Plane<__half, 4> img, Plane<__half, 2> grad, const float* basis, Plane<__half, 4> out,
                         const BlockMatchArgs& a, cudaStream_t s) {
-    const size_t smem = bm_pair_smem_bytes<TY, NP>();
+    const size_t smem = sizeof(BmTileSmem<TY, NP>);
     ensure_dynamic_smem(reinterpret_cast<const void*>(k_block_match_pair<TY, NP>), int(smem));
-    dim3 b(BX_TX, TY);
     dim3 g((img.w + BX_TX - 1) / BX_TX, (img.h + NP * TY - 1) / (NP * TY));
-    k_block_match_pair<TY, NP><<<g, b, smem, s>>>(img, grad, basis, out, a);
+    k_block_match_pair<TY, NP><<<g, BxTile<TY, NP>::THREADS, smem, s>>>(img, grad, basis, out, a);
 }
 
-// the pair kernel's variants by code (10 TY + NP)
+// the variants by code (10 TY + NP)
 static constexpr int kBmVariants[4] = {84, 44, 82, 162};
 
 static void launch_pair_variant(int code, Plane<__half, 4> img, Plane<__half, 2> grad, const float* basis,
@@ -563,21 +706,9 @@ __device__ __forceinline__ uint32_t ex2_h2(uint32_t x) {
     asm("ex2.approx.f16x2 %0, %1;" : "=r"(r) : "r"(x));
     return r;
 }
-__device__ __forceinline__ uint32_t hmul2_u(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
 __device__ __forceinline__ u64 h2_to_f2(uint32_t h) {
     const float2 f = __half22float2(u2h_(h));
     return pk2(f.x, f.y);
-}
-__device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0, float c0, float c1,
-                                        float c2, float c3) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(b0), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 __device__ __forceinline__ uint32_t hmin2_u(uint32_t a, uint32_t b) {
     uint32_t r;
@@ -840,7 +971,7 @@ static void launch_mma(Plane<__half, 4> img, Plane<__half, 2> grad, const float*
 // returns GLS_ERR_TIMEOUT.
 struct PSmem {
     union {
-        alignas(16) unsigned char bm[bm_pair_smem_bytes<8, 4>()];  // a 32 x 32 tile of the pair form
+        BmTileSmem<8, 2> bm;  // a 32 x 16 tile
         EigenSmem eig;
         CovSmem cov;
     };
@@ -872,8 +1003,8 @@ __device__ __noinline__ void persistent_eigen(const PLevel& L) {
                     reinterpret_cast<PSmem*>(smem_raw)->eig);
 }
 
-// a block-matching task: one 32 x 32 tile of the default (pair-form)
-// matcher in its 8 x 4 variant, the same bits as every stream variant
+// a block-matching task: one 32 x 16 tile of the default matcher by the
+// block's 8 warps, the same bits as every stream variant
 __device__ __noinline__ void persistent_bm(const PLevel& L, uint32_t item) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Plane<__half, 4> layer = L.layer, den = L.den;
@@ -881,8 +1012,7 @@ __device__ __noinline__ void persistent_bm(const PLevel& L, uint32_t item) {
     const float* basis = L.basis;
     const BlockMatchArgs ba = L.ba;
     const int tx = int(item) % L.tiles_x, ty = int(item) / L.tiles_x;
-    bm_pair_tile<8, 4>(tx * BM_T, ty * BM_T, threadIdx.x & 31, threadIdx.x >> 5, layer, grad, basis, den, ba,
-                       reinterpret_cast<PSmem*>(smem_raw)->bm);
+    bm_tile<8, 2>(tx * BX_TX, ty * kPBmRows, layer, grad, basis, den, ba, reinterpret_cast<PSmem*>(smem_raw)->bm);
 }
 
 __global__ void __launch_bounds__(BM_THREADS, 2)
@@ -981,18 +1111,17 @@ void launch_pyramid_persistent(const PTask* tasks, int n, const PLevel* lv, PCou
     k_pyramid_persistent<<<grid, BM_THREADS, sizeof(PSmem), s>>>(tasks, n, lv, cnt, next, err, limit_ns);
 }
 
-// Tile autotuner of the FP16 block matcher. Its variants (thread rows x
-// pixels per thread: 8 x 4 and 16 x 2 for 32 x 32 tiles, 4 x 4 and 8 x 2
-// for 32 x 16) compute identical results (the same per-pixel arithmetic,
-// pairs of pixels in packed FP32, and the same centring), so the choice only
-// changes speed: 32 x 32 tiles amortise the staged halo better, 32 x 16
-// tiles fill the GPU on small pyramid levels, and one pair per thread
-// trades the reuse of a staged neighbour for occupancy. The first call for
-// a level size times every variant on the caller's stream (leaving the
-// result in `out`) and keeps the fastest; later calls reuse the choice, and
-// so do calls made while the stream is being captured into a graph
-// (default 8 x 4 for a size not timed yet). GLS_BM_TILE=84, 44, 82 or 162 in
-// the environment (or 8 / 4 for 84 / 44) fixes the variant.
+// The tile variant of the FP16 block matcher. The variants (warps x pixels per
+// lane: 8 x 4 and 16 x 2 for 32 x 32 tiles, 4 x 4 and 8 x 2 for 32 x 16)
+// compute identical results (a pixel's group, its walk and its centring are
+// the same), so the choice only changes speed. 8 x 2 is taken for every size:
+// two of its blocks share an SM, so one stages while the other computes. A
+// 32 x 32 tile stages 28% fewer positions per pixel but fills an SM alone:
+// 16 x 2 takes 2.26 ms a 2016x1512 denoise against 2.09, 48.5 ms a batch of six
+// 12 MP frames against 46.2, 0.385 ms a 256x192 frame against 0.314; 8 x 4 and
+// 4 x 4 hold half the warps (2.61 and 2.55 ms). GLS_BM_TILE=84, 44, 82 or 162
+// in the environment (or 8 / 4 for 84 / 44) fixes the variant. The choices are
+// listed by level size for gls_block_match_tiles.
 static std::mutex g_tile_mu;
 static std::map<std::pair<int, int>, int> g_tile_choice;
 
@@ -1010,8 +1139,7 @@ int bm_tile_list(int* whty, int max) {
     return n;
 }
 
-template <class Run>
-static int bm_tile_variant(int w, int h, Run&& run_variant, cudaStream_t s) {
+static int bm_tile_variant(int w, int h) {
     static const int forced = [] {
         const char* e = std::getenv("GLS_BM_TILE");
         const int v = e ? std::atoi(e) : 0;
@@ -1022,37 +1150,8 @@ static int bm_tile_variant(int w, int h, Run&& run_variant, cudaStream_t s) {
         return 0;
     }();
     if (forced) return forced;
-    {
-        std::lock_guard<std::mutex> lk(g_tile_mu);
-        auto it = g_tile_choice.find({w, h});
-        if (it != g_tile_choice.end()) return it->second;
-    }
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 84;
-    constexpr int NV = sizeof(kBmVariants) / sizeof(kBmVariants[0]);
-    cudaEvent_t e[NV + 1];
-    for (auto& ev : e) cudaEventCreate(&ev);
-    cudaEventRecord(e[0], s);
-    for (int v = 0; v < NV; v++) {
-        run_variant(kBmVariants[v]);
-        cudaEventRecord(e[v + 1], s);
-    }
-    int choice = 84;
-    if (cudaEventSynchronize(e[NV]) == cudaSuccess) {
-        float best = 0.f;
-        for (int v = 0; v < NV; v++) {
-            float t = 0.f;
-            if (cudaEventElapsedTime(&t, e[v], e[v + 1]) != cudaSuccess) continue;
-            if (v == 0 || t < best) {
-                best = t;
-                choice = kBmVariants[v];
-            }
-        }
-    }
-    for (auto& ev : e) cudaEventDestroy(ev);
     std::lock_guard<std::mutex> lk(g_tile_mu);
-    g_tile_choice[{w, h}] = choice;
-    return 0;  // `out` already holds the result
+    return g_tile_choice.emplace(std::make_pair(w, h), 82).first->second;
 }
 
 template <class S>
@@ -1069,10 +1168,7 @@ void launch_block_match(Plane<S, 4> img, Plane<S, 2> grad, Plane<S, 8> pca, cons
             launch_mma(img, grad, basis, out, a, s);
             return;
         }
-        const int code = bm_tile_variant(img.w, img.h, [&](int c) {
-            launch_pair_variant(c, img, grad, basis, out, a, s);
-        }, s);
-        if (code) launch_pair_variant(code, img, grad, basis, out, a, s);
+        launch_pair_variant(bm_tile_variant(img.w, img.h), img, grad, basis, out, a, s);
     } else {
         ensure_dynamic_smem(reinterpret_cast<const void*>(k_block_match_plain<S>), int(sizeof(BmPlainSmem)));
         dim3 b(BP_TX, BP_TY);

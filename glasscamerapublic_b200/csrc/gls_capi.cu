@@ -1076,7 +1076,7 @@ static gls_status persistent_plan(gls_converter* conv, const gls_frame_desc* fra
             d.basis = static_cast<float*>(P.basis.p) + i * 200;
             d.status = static_cast<int*>(P.status.p) + i;
             d.tiles_x = (wi + 31) / 32;
-            d.n_bm = d.tiles_x * ((hi + 31) / 32);
+            d.n_bm = d.tiles_x * ((hi + kPBmRows - 1) / kPBmRows);
             d.sn_tiles_x = (wi + kPSnTile - 1) / kPSnTile;
             d.n_sn = i < L - 1 ? d.sn_tiles_x * ((hi + kPSnTile - 1) / kPSnTile) : 0;
             d.n_cov = pca_cov_rows(wi, hi);

@@ -139,6 +139,7 @@ constexpr uint32_t kPTaskItemMask = 0x3fffffffu;
 // side of a persistent reconstruct task's tile: 64 x 64 pixels (16 per
 // thread), so the per-task fetch and bookkeeping stay small beside the work
 constexpr int kPSnTile = 64;
+constexpr int kPBmRows = 16;  // block-matching tasks: 32 x 16 pixels
 struct PLevel {
     Plane<__half, 4> img, layer, den;  // the level's image, reconstructed layer, denoised output
     Plane<__half, 2> grad;
