@@ -7,8 +7,7 @@
 // accumulated in FP32; output (Y, Cb, Cr, sum of luma weights).
 //
 // The kernels stage the tile's window region (halo 10) in shared memory. The
-// one for the FP32 plain path evaluates the formula directly with correctly
-// rounded exponentials (parity with the oracle's FP32 run), two vertically
+// one for the FP32 plain path evaluates the formula directly, two vertically
 // adjacent pixels a thread; the FP16-storage path's forms the distances on the
 // tensor cores and the weights and sums in packed FP32.
 #include <cmath>
@@ -96,112 +95,161 @@ __device__ __forceinline__ float spatial_weight(int i, int j) {  // gaussian(0.1
     return expf(-2.f * d * d);
 }
 
-// ============================================================ FP32 plain path
-// Two vertically adjacent pixels per thread, tile 32 x 16, FP32 staging.
-constexpr int BP_TX = 32, BP_TY = 8, BP_W = BP_TX + 20, BP_H = 2 * BP_TY + 20;
+typedef unsigned long long u64;
 
-struct BmPlainSmem {
-    float4 pca[BP_H * BP_W][2];
-    float4 ycc[BP_H * BP_W];
-    float spatial[21 * 21];
+__device__ __forceinline__ u64 pk2(float a, float b) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void upk2(u64 r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// ============================================================ FP32 plain path
+// NP vertically adjacent pixels per thread, 32 x 4 threads, FP32 staging. The
+// arithmetic of a tap and the order of a window's sums (row by row) are the
+// same whatever the tile, so every tile gives the same bits. Differences and
+// chroma terms are packed FP32 (the same roundings in half the instructions),
+// the distance's sum stays a serial chain; ex2.approx.ftz where exp2f only
+// adds the scaling that keeps results below 2^-126.
+//
+// What bounds it: two pixels' tap takes 60 cycles of a sub-partition's FMA
+// pipe, 32 of its MUFU and 57 issue slots, and the SM's shared memory serves
+// four of them in 52 wavefronts. The coefficients lie in two arrays because a
+// warp's 16-byte loads at a 32-byte stride hit each bank twice (84 wavefronts,
+// the former bound). 1024x768: 550 -> 428 us, 128x96: 63 -> 23 us; three
+// blocks of 32 x 8 pixels an SM where two of 32 x 16 leave a longer last wave
+// (512x384: 125 us with those).
+template <int NP>
+struct BmPlainTile {
+    static constexpr int TX = 32, TY = 4, THREADS = TX * TY, ROWS = NP * TY;
+    static constexpr int W = TX + 20, H = ROWS + 20;
+    struct Smem {
+        ulonglong2 pca0[H * W], pca1[H * W];  // coefficients 0..3, 4..7
+        float4 ycc[H * W];                    // Cb, Cr, Y
+        float2 spatial[22][21];               // the weights of window rows j and j - 1
+    };
 };
 
 struct BmPlainPix {
-    float4 p0, p1;
-    float kl;              // -2 log2(e) s^2
-    float c1, c2, o1, o2;  // sqrt(2 log2 e) c, times the centre chroma
+    u64 n[4];   // minus the coefficients
+    float kl;   // -2 log2(e) s^2
+    u64 c, no;  // sqrt(2 log2 e) (c1, c2), minus that times the centre chroma
 };
 
-template <bool UP, bool LO>
-__device__ __forceinline__ void bmp_row(const BmPlainSmem& sm, int base, int r, const BmPlainPix& u,
-                                        const BmPlainPix& l, float (&acc)[10]) {
+// One row of the union of the pixels' windows: the upper pixel's taps when UP,
+// the lower's when LO.
+template <bool UP, bool LO, int NP, class Smem>
+__device__ __forceinline__ void bmp_row(const Smem& sm, int base, int r, const BmPlainPix (&pix)[NP],
+                                        float (&acc)[NP][5]) {
     const float kLk = 2.f * 1.4426950408889634f;
 #pragma unroll
     for (int i = 0; i < 21; i++) {
-        const float4 q0 = sm.pca[base + i][0], q1 = sm.pca[base + i][1];
+        const ulonglong2 q0 = sm.pca0[base + i], q1 = sm.pca1[base + i];
         const float4 y = sm.ycc[base + i];
-        auto tap = [&](const BmPlainPix& p, int j, int o) {
-            float d, d2;
-            d = q0.x - p.p0.x; d2 = d * d;
-            d = q0.y - p.p0.y; d2 = fmaf(d, d, d2);
-            d = q0.z - p.p0.z; d2 = fmaf(d, d, d2);
-            d = q0.w - p.p0.w; d2 = fmaf(d, d, d2);
-            d = q1.x - p.p1.x; d2 = fmaf(d, d, d2);
-            d = q1.y - p.p1.y; d2 = fmaf(d, d, d2);
-            d = q1.z - p.p1.z; d2 = fmaf(d, d, d2);
-            d = q1.w - p.p1.w; d2 = fmaf(d, d, d2);
-            const float lw = exp2f(p.kl * d2);
-            const float e1 = fmaf(p.c1, y.y, -p.o1), e2 = fmaf(p.c2, y.z, -p.o2);
-            const float cw = exp2f(-fmaf(kLk * lw, lw, fmaf(e1, e1, e2 * e2)));
-            const float sw = sm.spatial[j * 21 + i];
-            const float wy = sw * lw, wc = sw * cw;
-            acc[o + 0] = fmaf(wy, y.x, acc[o + 0]);
-            acc[o + 1] = fmaf(wc, y.y, acc[o + 1]);
-            acc[o + 2] = fmaf(wc, y.z, acc[o + 2]);
-            acc[o + 3] += wy;
-            acc[o + 4] += wc;
-        };
-        if (UP) tap(u, r, 0);
-        if (LO) tap(l, r - 1, 5);
+        const float2 sw = sm.spatial[r][i];
+        const u64 ch = pk2(y.x, y.y);
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            if (p == 0 ? !UP : !LO) continue;
+            const BmPlainPix& P = pix[p];
+            float(&s)[5] = acc[p];
+            float d[8], e1, e2;
+            upk2(add2(q0.x, P.n[0]), d[0], d[1]);
+            upk2(add2(q0.y, P.n[1]), d[2], d[3]);
+            upk2(add2(q1.x, P.n[2]), d[4], d[5]);
+            upk2(add2(q1.y, P.n[3]), d[6], d[7]);
+            float d2 = d[0] * d[0];
+#pragma unroll
+            for (int k = 1; k < 8; k++) d2 = fmaf(d[k], d[k], d2);
+            const float lw = ex2_approx(P.kl * d2);
+            upk2(fma2(P.c, ch, P.no), e1, e2);
+            const float cw = ex2_approx(-fmaf(kLk * lw, lw, fmaf(e1, e1, e2 * e2)));
+            const float w = p == 0 ? sw.x : sw.y;
+            const float wy = w * lw, wc = w * cw;
+            s[0] = fmaf(wy, y.z, s[0]);
+            s[1] = fmaf(wc, y.x, s[1]);
+            s[2] = fmaf(wc, y.y, s[2]);
+            s[3] += wy;
+            s[4] += wc;
+        }
     }
 }
 
-template <class S>
-__global__ void __launch_bounds__(256) k_block_match_plain(Plane<S, 4> img, Plane<S, 2> grad, Plane<S, 8> pca,
-                                                           Plane<S, 4> out, BlockMatchArgs a) {
+template <int NP>
+__global__ void __launch_bounds__(128, 3)
+    k_block_match_plain(Plane<float, 4> img, Plane<float, 2> grad, Plane<float, 8> pca, Plane<float, 4> out,
+                        BlockMatchArgs a) {
+    using T = BmPlainTile<NP>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    BmPlainSmem& sm = *reinterpret_cast<BmPlainSmem*>(smem_raw);
-    const int x0 = blockIdx.x * BP_TX, y0 = blockIdx.y * (2 * BP_TY);
-    const int tid = threadIdx.y * BP_TX + threadIdx.x;
-    for (int k = tid; k < 441; k += 256) sm.spatial[k] = spatial_weight(k % 21 - 10, k / 21 - 10);
-    for (int k = tid; k < BP_W * BP_H; k += 256) {
-        const int ty = k / BP_W, tx = k % BP_W;
+    typename T::Smem& sm = *reinterpret_cast<typename T::Smem*>(smem_raw);
+    const int x0 = blockIdx.x * T::TX, y0 = blockIdx.y * T::ROWS;
+    const int tid = threadIdx.y * T::TX + threadIdx.x;
+    for (int k = tid; k < 22 * 21; k += T::THREADS) {
+        const int j = k / 21, i = k % 21;
+        sm.spatial[j][i] = make_float2(spatial_weight(i - 10, j - 10), spatial_weight(i - 10, j - 11));
+    }
+    for (int k = tid; k < T::W * T::H; k += T::THREADS) {
+        const int ty = k / T::W, tx = k % T::W;
         const int sx = clampi(x0 - 10 + tx, 0, img.w - 1), sy = clampi(y0 - 10 + ty, 0, img.h - 1);
-        const S* q = pca.px(sx, sy);
-        if constexpr (is_half<S>::value) {
-            const uint4 u = *reinterpret_cast<const uint4*>(q);
-            const float2 a0 = __half22float2(u2h_(u.x)), a1 = __half22float2(u2h_(u.y));
-            const float2 a2 = __half22float2(u2h_(u.z)), a3 = __half22float2(u2h_(u.w));
-            sm.pca[k][0] = make_float4(a0.x, a0.y, a1.x, a1.y);
-            sm.pca[k][1] = make_float4(a2.x, a2.y, a3.x, a3.y);
-        } else {
-            const float4* q4 = reinterpret_cast<const float4*>(q);
-            sm.pca[k][0] = q4[0];
-            sm.pca[k][1] = q4[1];
-        }
-        const f4 p = ld4<S>(img.px(sx, sy));
-        sm.ycc[k] = make_float4(p.x, p.y, p.z, 0.f);
+        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(pca.px(sx, sy));
+        sm.pca0[k] = q[0];
+        sm.pca1[k] = q[1];
+        const f4 p = ld4<float>(img.px(sx, sy));
+        sm.ycc[k] = make_float4(p.y, p.z, p.x, 0.f);
     }
     __syncthreads();
-    const int x = x0 + threadIdx.x, yu = y0 + 2 * threadIdx.y;
+    const int x = x0 + threadIdx.x, y = y0 + NP * threadIdx.y;
     const float kLog2e = 1.4426950408889634f, sq = sqrtf(2.f * kLog2e);
-    BmPlainPix pix[2];
+    BmPlainPix pix[NP];
 #pragma unroll
-    for (int p = 0; p < 2; p++) {
-        const int c = (2 * threadIdx.y + p + 10) * BP_W + threadIdx.x + 10;
+    for (int p = 0; p < NP; p++) {
+        const int c = (NP * threadIdx.y + p + 10) * T::W + threadIdx.x + 10;
         const float4 in = sm.ycc[c];
-        const BmConst k = bm_const<S>(a, grad, img.w, img.h, min(x, img.w - 1), min(yu + p, img.h - 1), in.x, in.y, in.z);
+        const BmConst k = bm_const<float>(a, grad, img.w, img.h, min(x, img.w - 1), min(y + p, img.h - 1), in.z, in.x, in.y);
         BmPlainPix& P = pix[p];
-        P.p0 = sm.pca[c][0];
-        P.p1 = sm.pca[c][1];
+        const float4 p0 = *reinterpret_cast<const float4*>(&sm.pca0[c]), p1 = *reinterpret_cast<const float4*>(&sm.pca1[c]);
+        P.n[0] = pk2(-p0.x, -p0.y);
+        P.n[1] = pk2(-p0.z, -p0.w);
+        P.n[2] = pk2(-p1.x, -p1.y);
+        P.n[3] = pk2(-p1.z, -p1.w);
         P.kl = -2.f * kLog2e * k.s * k.s;
-        P.c1 = sq * k.c1;
-        P.c2 = sq * k.c2;
-        P.o1 = P.c1 * in.y;
-        P.o2 = P.c2 * in.z;
+        const float c1 = sq * k.c1, c2 = sq * k.c2;
+        P.c = pk2(c1, c2);
+        P.no = pk2(-(c1 * in.x), -(c2 * in.y));
     }
-    float acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const int col = threadIdx.x, row0 = 2 * threadIdx.y;
-    bmp_row<true, false>(sm, row0 * BP_W + col, 0, pix[0], pix[1], acc);
-    for (int r = 1; r <= 20; r++) bmp_row<true, true>(sm, (row0 + r) * BP_W + col, r, pix[0], pix[1], acc);
-    bmp_row<false, true>(sm, (row0 + 21) * BP_W + col, 21, pix[0], pix[1], acc);
-    if (x < out.w) {
-        if (yu < out.h) st4<S>(out.px(x, yu), f4{acc[0] / acc[3], acc[1] / acc[4], acc[2] / acc[4], acc[3]});
-        if (yu + 1 < out.h) st4<S>(out.px(x, yu + 1), f4{acc[5] / acc[8], acc[6] / acc[9], acc[7] / acc[9], acc[8]});
-        if (a.nc_out) {
-            if (yu < out.h) a.nc_out[size_t(yu) * out.w + x] = acc[4];
-            if (yu + 1 < out.h) a.nc_out[size_t(yu + 1) * out.w + x] = acc[9];
-        }
+    float acc[NP][5] = {};
+    const int base = NP * threadIdx.y * T::W + threadIdx.x;
+    if constexpr (NP == 2) {
+        bmp_row<true, false, NP>(sm, base, 0, pix, acc);
+#pragma unroll 1
+        for (int r = 1; r <= 20; r++) bmp_row<true, true, NP>(sm, base + r * T::W, r, pix, acc);
+        bmp_row<false, true, NP>(sm, base + 21 * T::W, 21, pix, acc);
+    } else {
+#pragma unroll 1
+        for (int r = 0; r <= 20; r++) bmp_row<true, false, NP>(sm, base + r * T::W, r, pix, acc);
+    }
+    if (x >= out.w) return;
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+        if (y + p >= out.h) continue;
+        const float(&s)[5] = acc[p];
+        st4<float>(out.px(x, y + p), f4{s[0] / s[3], s[1] / s[4], s[2] / s[4], s[3]});
+        if (a.nc_out) a.nc_out[size_t(y + p) * out.w + x] = s[4];
     }
 }
 
@@ -252,29 +300,6 @@ struct BxTile {
     static_assert(ROWS == 16 || ROWS == 32, "tile heights divide the 32-row centring tiles");
     static_assert((BX_W * H) % 16 == 0, "the projection takes 16 positions at a time");
 };
-typedef unsigned long long u64;
-
-__device__ __forceinline__ u64 pk2(float a, float b) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk2(u64 r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ uint32_t hmul2_u(uint32_t a, uint32_t b) {
     uint32_t r;
@@ -1154,6 +1179,15 @@ static int bm_tile_variant(int w, int h) {
     return g_tile_choice.emplace(std::make_pair(w, h), 82).first->second;
 }
 
+template <int NP>
+static void launch_plain(Plane<float, 4> img, Plane<float, 2> grad, Plane<float, 8> pca, Plane<float, 4> out,
+                         const BlockMatchArgs& a, cudaStream_t s) {
+    using T = BmPlainTile<NP>;
+    ensure_dynamic_smem(reinterpret_cast<const void*>(k_block_match_plain<NP>), int(sizeof(typename T::Smem)));
+    const dim3 g((img.w + T::TX - 1) / T::TX, (img.h + T::ROWS - 1) / T::ROWS);
+    k_block_match_plain<NP><<<g, dim3(T::TX, T::TY), sizeof(typename T::Smem), s>>>(img, grad, pca, out, a);
+}
+
 template <class S>
 void launch_block_match(Plane<S, 4> img, Plane<S, 2> grad, Plane<S, 8> pca, const float* basis, Plane<S, 4> out,
                         const BlockMatchArgs& a, cudaStream_t s) {
@@ -1170,10 +1204,13 @@ void launch_block_match(Plane<S, 4> img, Plane<S, 2> grad, Plane<S, 8> pca, cons
         }
         launch_pair_variant(bm_tile_variant(img.w, img.h), img, grad, basis, out, a, s);
     } else {
-        ensure_dynamic_smem(reinterpret_cast<const void*>(k_block_match_plain<S>), int(sizeof(BmPlainSmem)));
-        dim3 b(BP_TX, BP_TY);
-        dim3 g((img.w + BP_TX - 1) / BP_TX, (img.h + 2 * BP_TY - 1) / (2 * BP_TY));
-        k_block_match_plain<S><<<g, b, sizeof(BmPlainSmem), s>>>(img, grad, pca, out, a);
+        // One pixel a thread while its 32 x 4 tiles fit the chip's 148 SMs one
+        // each: 128x96 (96 of them) 23 us, 32 with two pixels a thread; at
+        // 256x192 (384) both take 47-49 us, at 1024x768 580 and 428.
+        if (((img.w + 31) / 32) * ((img.h + 3) / 4) <= 148)
+            launch_plain<1>(img, grad, pca, out, a, s);
+        else
+            launch_plain<2>(img, grad, pca, out, a, s);
     }
 }
 

@@ -85,3 +85,34 @@ def test_extreme_distance_scales_keep_the_pixel(var):
     got = _denoise(ycc, grad, _params(h, w, a=var, b=0.0), True)
     assert np.isfinite(got).all()
     assert np.abs(got[..., :3] - ycc[..., :3]).max() < 1e-3
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (3, 5), (4, 32), (5, 33), (17, 31), (70, 41),
+                                 (148, 128), (149, 128), (149, 129), (401, 803)])
+def test_fp32_matcher_against_float64(h, w):
+    """One and two pixels a thread (128 x 148 is the largest with one). The
+    coefficients' rounding (25 terms of 0.5 in FP32, 5e-7) moves an exponent by
+    4 d s^2 5e-7: 1e-3 of a weight at |d s| = 3 and s = 130, so a mean of
+    deviations up to 0.04 by at most 4e-5."""
+    import torch
+    import _torch_pyramid as TP
+    ycc, grad = _image(h, w, h * 1000 + w)
+    p = _params(h, w)
+    t = [torch.from_numpy(a).cuda() for a in (ycc, grad)]
+    out = torch.empty((h, w, 4), device="cuda")
+    v = [g.ImageView(C.c_void_p(a.data_ptr()), w, h, a.shape[2], g.F32, a.stride(0) * 4) for a in (*t, out)]
+    conv = g.RawConverter(0)
+    try:
+        g.check(g.lib().gls_pyramid_denoise(conv.handle, C.byref(v[0]), C.byref(v[1]), C.byref(p), g.SYNC,
+                                            C.byref(v[2]), None))
+        basis = torch.from_numpy(conv.pca_basis(0)).cuda().double()
+    finally:
+        conv.close()
+    layer, dp = t[0].double(), p.denoise[0]
+    nlf = [torch.tensor([float(q) for q in x], dtype=torch.float64, device="cuda")
+           for x in (p.pyramid_nlf[0].a, p.pyramid_nlf[0].b)]
+    ref = TP.block_match(layer, t[1].double(), TP.pca_project(layer, basis), *nlf,
+                         (dp.luma, dp.chroma, dp.chroma), dp).cpu().numpy()
+    got = out.cpu().numpy()
+    assert np.abs(got[..., :3] - ref[..., :3]).max() < 4e-5
+    assert (np.abs(got[..., 3] - ref[..., 3]) < 1e-3 * ref[..., 3]).all()
