@@ -17,13 +17,12 @@
 // img_{l+1} = down(img_l), img_0 = the despeckled front-end output, so the
 // sweep also accumulates dL/d img_l and pushes it down to img_0.
 //   * k_adj_head          dL/d den_0 = M^T 2 (out - target) / N, and the loss
-//   * k_bm_bwd_center     block matching, the pixel as the window centre:
-//                         from the forward's outputs and kernel norms,
-//                         recomputes its weights, then dL/d(its scales, its
-//                         own PCA coefficients and chroma), dL/dtheta, and a
-//                         per-pixel record for the neighbour pass
-//   * k_bm_bwd_neighbor   the pixel as a neighbour q of every centre p whose
-//                         window reads it (clamp-to-edge preimages included)
+//   * k_bm_bwd_record     per pixel, what block matching's transpose needs of
+//                         it: from the forward's outputs and kernel norms
+//   * k_bm_bwd            block matching transposed, each pixel as a window
+//                         centre and as a neighbour q of every centre p whose
+//                         window reads it (clamp-to-edge preimages included):
+//                         dL/d(layer), dL/d(PCA coefficients), dL/dtheta
 //   * k_pca_bwd           transpose of the 5x5 x 25x8 projection
 //   * k_sn_bwd            subtractNoiseImage: dL/d(up-sampled den_{l+1}) and
 //                         dL/dtheta through the sharpening gate
@@ -37,15 +36,15 @@
 // Every reduction is per block and summed in block order: the gradient does
 // not depend on scheduling.
 #include <cfloat>
+#include <type_traits>
 
 #include "gls_common.cuh"
 #include "gls_kernels.h"
 
 namespace gls {
 
-constexpr int AT_X = 32, AT_Y = 8;        // adjoint tile (pixels)
-constexpr int AH = 10;                     // block-matching window radius
-constexpr int AW_ = AT_X + 2 * AH, AH_ = AT_Y + 2 * AH;
+constexpr int AT_X = 32;  // adjoint tile width
+constexpr int AH = 10;    // block-matching window radius
 
 // offsets d in [-R, R] with clamp(p + d, 0, n - 1) == q
 __device__ __forceinline__ bool preimage(int q, int p, int R, int n, int& lo, int& hi) {
@@ -106,99 +105,320 @@ __device__ __forceinline__ float spatial_w(int i, int j) {
     return expf(-2.f * d * d);
 }
 
-struct CenterSmem {
-    float4 q[AH_ * AW_][3];  // (Y, Cb, Cr, -), pca 0..3, pca 4..7 of the clamped window positions
-    float sw[441];
+__device__ __forceinline__ float ex2a(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 pk2(float a, float b) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 up2(u64 r) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
+    return v;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// Per pixel, what its pairs need of it (12 floats):
+//   Y, kl, Cb, Cr | gY/ny, gY/ny (Y - Y_out), g . (chroma - chroma_out), - | g, K^2
+// with kl = -2 log2(e) L^2, S = sqrt(2 log2 e), g = 4 / S (gCb, gCr)/nc and
+// K = S (K1, K2). In these units, for a centre's tap of spatial weight s at
+// coefficient distance d2, luma difference dY and chroma difference c:
+// l = exp2(kl d2 + log2 S) is S times the luma weight, the chroma weight is
+// cw = exp2(-l^2 - |K c|^2), and with w = s cw (g . (chroma + c - chroma_out)):
+//   dL/dL      = -4 L / S   sum d2 E,   E = l (s gY (Y + dY - Y_out) - w l)
+//   dL/dK1     = -K         sum w c^2   (each channel)
+//   dL/dchroma =  1 / S     sum w c K^2    (of both ends; plus the mean's term)
+//   dL/dpca    = -4 / S^3   sum kl E (q - p)   (of both ends)
+// The differences from the outputs are taken relative to the centre, so that
+// nothing cancels.
+constexpr float kAdjS = 1.6986436005760381f, kAdjLog2S = 0.7643831864724489f;
+
+__global__ void __launch_bounds__(256) k_bm_bwd_record(AdjointLevelArgs a) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    if (x >= a.w || y >= a.h) return;
+    const size_t pi = size_t(y) * a.w + x;
+    const float4 in = *reinterpret_cast<const float4*>(a.layer + pi * 4);
+    const float2 gr = *reinterpret_cast<const float2*>(a.grad + pi * 2);
+    const BmScales S = bm_scales(a, in.x, sqrtf(gr.x * gr.x + gr.y * gr.y));
+    const float4 dv = *reinterpret_cast<const float4*>(a.den + pi * 4);
+    const float* g = a.g_den + pi * 3;
+    const float nc = a.nc[pi], k = 4.f / kAdjS;
+    float4* rec = reinterpret_cast<float4*>(a.rec + pi * 12);
+    rec[0] = make_float4(in.x, -kAdjS * kAdjS * S.L * S.L, in.y, in.z);
+    const float gY = g[0] / dv.w, g1 = k * (g[1] / nc), g2 = k * (g[2] / nc);
+    const float K1 = kAdjS * S.K1, K2 = kAdjS * S.K2;
+    rec[1] = make_float4(gY, gY * (in.x - dv.x), fmaf(g1, in.y - dv.y, g2 * (in.z - dv.z)), 0.f);
+    rec[2] = make_float4(g1, g2, K1 * K1, K2 * K2);
+}
+
+// Block matching transposed: every pixel x against every pixel y of the
+// 21 x 21 box around it, x as the centre that reads y and x as the neighbour
+// that the centre y reads. Both weights take the same coefficient distance,
+// and both gradients of x's coefficients run along y - x: one pass over the
+// pairs does both.
+//
+// A pixel at the image border is read through several taps that clamp onto it.
+// All terms are linear in the spatial weight, so such a pair takes the sum of
+// its taps' weights: a product of a column and a row table, used by the blocks
+// whose box touches the border (0 for positions outside the image).
+//
+// What bounds it: the FMA pipe and the MUFU together (69 FP32 operations and 4
+// ex2 a pair) and, with one pixel a thread, the 80 bytes of a pair's other
+// pixel (20 shared-memory wavefronts for a warp); a thread takes two vertically
+// adjacent pixels, whose windows share 20 of 22 rows. A block's 12 warps take
+// 32 x 24 pixels (183 KB of staging, one block an SM), or, KS = 4, 8 warps take
+// 32 x 4 pixels with each window's rows dealt to four warps, for levels too
+// small to fill the chip. 2048x1536: 3.87 ms (8 warps 4.05, 16 warps 3.92),
+// where a pass for the centres and one for the neighbours took 3.49 + 4.39;
+// 128x96: 45 us for 75 + 308.
+template <int KS>
+struct BwdTile {
+    static constexpr int WARPS = KS == 1 ? 12 : 8, THREADS = 32 * WARPS;
+    static constexpr int ROWS = 2 * WARPS / KS, W = AT_X + 2 * AH, H = ROWS + 2 * AH;
+    struct Smem {
+        float4 v[5][H * W];  // the record, pca 0..3, pca 4..7
+        union {
+            float2 sw[22][21];  // the weights of box rows j and j - 1
+            struct {            // weights of a pair by offset, x as the centre / as the neighbour
+                float cx[AT_X][21], nx[AT_X][21];
+                float2 y[ROWS][21];
+            } b;
+        };
+    };
 };
 
-// Block matching, the pixel p as the window centre. Writes the record
-// (gY/ny, Y_out, gCb/nc, Cb_out, gCr/nc, Cr_out, L, K1, K2) the neighbour
-// pass needs, the centre's own gradients (luma via its scales, chroma and
-// PCA coefficients via the distances) and per-block dL/dtheta partials
-// (luma, chroma, A_Y, B_Y, A_C, B_C).
-__global__ void __launch_bounds__(256) k_bm_bwd_center(AdjointLevelArgs a) {
+struct BwdPix {
+    u64 n[4], nc;  // minus the coefficients, minus the chroma
+    float Y, kl, gY, gYd, gcd, g1, g2, K1, K2;  // the record
+    // sums
+    u64 p[4];
+    float E, luma, c1, c2, cc1, cc2, mean1, mean2, n1, n2;
+};
+
+__device__ __forceinline__ void bwd_pair(BwdPix& x, const ulonglong2 q0, const ulonglong2 q1, const float4 v0,
+                                         const float4 v1, const float4 v2, float sc, float sn) {
+    const u64 d[4] = {add2(q0.x, x.n[0]), add2(q0.y, x.n[1]), add2(q1.x, x.n[2]), add2(q1.y, x.n[3])};
+    const float2 s = up2(fma2(d[3], d[3], fma2(d[2], d[2], fma2(d[1], d[1], mul2(d[0], d[0])))));
+    const float d2 = s.x + s.y, dY = v0.x - x.Y;
+    const float2 c = up2(add2(pk2(v0.z, v0.w), x.nc));
+    const float c1 = c.x, c2 = c.y, cc1 = c1 * c1, cc2 = c2 * c2;
+    float Ec, En;
+    {  // x the centre
+        const float l = ex2a(fmaf(x.kl, d2, kAdjLog2S));
+        const float cw = ex2a(-fmaf(l, l, fmaf(x.K1, cc1, x.K2 * cc2)));
+        const float w = sc * cw * fmaf(x.g1, c1, fmaf(x.g2, c2, x.gcd));
+        Ec = l * fmaf(-w, l, sc * fmaf(x.gY, dY, x.gYd));
+        x.E = fmaf(Ec, d2, x.E);
+        x.c1 = fmaf(w, c1, x.c1);
+        x.c2 = fmaf(w, c2, x.c2);
+        x.cc1 = fmaf(w, cc1, x.cc1);
+        x.cc2 = fmaf(w, cc2, x.cc2);
+    }
+    {  // the other pixel the centre: its differences are minus these
+        const float l = ex2a(fmaf(v0.y, d2, kAdjLog2S));
+        const float cw = ex2a(-fmaf(l, l, fmaf(v2.z, cc1, v2.w * cc2)));
+        const float wc = sn * cw, w = wc * fmaf(-v2.x, c1, fmaf(-v2.y, c2, v1.z));
+        En = l * fmaf(-w, l, sn * fmaf(-v1.x, dY, v1.y));
+        x.luma = fmaf(v1.x, sn * l, x.luma);
+        x.mean1 = fmaf(v2.x, wc, x.mean1);
+        x.mean2 = fmaf(v2.y, wc, x.mean2);
+        x.n1 = fmaf(w * v2.z, c1, x.n1);
+        x.n2 = fmaf(w * v2.w, c2, x.n2);
+    }
+    const float G = fmaf(Ec, x.kl, En * v0.y);
+    const u64 GG = pk2(G, G);
+#pragma unroll
+    for (int k = 0; k < 4; k++) x.p[k] = fma2(GG, d[k], x.p[k]);
+}
+
+template <int KS>
+__global__ void __launch_bounds__(BwdTile<KS>::THREADS, KS == 1 ? 1 : 2) k_bm_bwd(AdjointLevelArgs a) {
+    using T = BwdTile<KS>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    CenterSmem& sm = *reinterpret_cast<CenterSmem*>(smem_raw);
-    __shared__ float red[8][6];
+    typename T::Smem& sm = *reinterpret_cast<typename T::Smem*>(smem_raw);
+    __shared__ float red[T::WARPS][6];
     const int W = a.w, H = a.h;
-    const int x0 = blockIdx.x * AT_X, y0 = blockIdx.y * AT_Y;
+    const int x0 = blockIdx.x * AT_X, y0 = blockIdx.y * T::ROWS;
     const int tid = threadIdx.y * AT_X + threadIdx.x;
-    for (int k = tid; k < 441; k += 256) sm.sw[k] = spatial_w(k % 21 - 10, k / 21 - 10);
-    for (int k = tid; k < AH_ * AW_; k += 256) {
-        const int ty = k / AW_, tx = k % AW_;
-        const int sx = clampi(x0 - AH + tx, 0, W - 1), sy = clampi(y0 - AH + ty, 0, H - 1);
-        const float4 l = *reinterpret_cast<const float4*>(a.layer + (size_t(sy) * W + sx) * 4);
-        const float4* pc = reinterpret_cast<const float4*>(a.pca + (size_t(sy) * W + sx) * 8);
-        sm.q[k][0] = make_float4(l.x, l.y, l.z, 0.f);
-        sm.q[k][1] = pc[0];
-        sm.q[k][2] = pc[1];
+    const bool border = x0 < AH + 1 || y0 < AH + 1 || x0 + AT_X + AH > W - 1 || y0 + T::ROWS + AH > H - 1;
+    for (int k = tid; k < T::W * T::H; k += T::THREADS) {
+        const int px = x0 - AH + k % T::W, py = y0 - AH + k / T::W;
+        const bool in = px >= 0 && px < W && py >= 0 && py < H;
+        const size_t pi = in ? size_t(py) * W + px : 0;
+        const float4* rec = reinterpret_cast<const float4*>(a.rec + pi * 12);
+        const float4* pca = reinterpret_cast<const float4*>(a.pca + pi * 8);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < 3; c++) sm.v[c][k] = in ? rec[c] : zero;
+        sm.v[3][k] = in ? pca[0] : zero;
+        sm.v[4][k] = in ? pca[1] : zero;
+    }
+    if (!border) {
+        for (int k = tid; k < 22 * 21; k += T::THREADS) {
+            const int j = k / 21, i = k % 21;
+            sm.sw[j][i] = make_float2(spatial_w(i - AH, j - AH), spatial_w(i - AH, j - 1 - AH));
+        }
+    } else {
+        // sum of the 1-D weights of the offsets d with clamp(p + d) == q
+        auto weights = [&](int q, int p, int n) {
+            int lo, hi;
+            float v = 0.f;
+            if (q >= 0 && q < n && p >= 0 && p < n && preimage(q, p, AH, n, lo, hi))
+                for (int d = lo; d <= hi; d++) v += spatial_w(d, 0);
+            return v;
+        };
+        for (int k = tid; k < (AT_X + T::ROWS) * 21; k += T::THREADS) {
+            const int t = k / 21, i = k % 21;
+            if (t < AT_X) {
+                const int x = x0 + t, y = x + i - AH;
+                sm.b.cx[t][i] = weights(y, x, W);
+                sm.b.nx[t][i] = weights(x, y, W);
+            } else {
+                const int x = y0 + t - AT_X, y = x + i - AH;
+                sm.b.y[t - AT_X][i] = make_float2(weights(y, x, H), weights(x, y, H));
+            }
+        }
     }
     __syncthreads();
-    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
-    float th[6] = {0, 0, 0, 0, 0, 0};
-    if (x < W && y < H) {
-        const size_t pi = size_t(y) * W + x;
-        const int c = (threadIdx.y + AH) * AW_ + threadIdx.x + AH;
-        const float4 in = sm.q[c][0];
-        const float4 ip0 = sm.q[c][1], ip1 = sm.q[c][2];
-        const float ip[8] = {ip0.x, ip0.y, ip0.z, ip0.w, ip1.x, ip1.y, ip1.z, ip1.w};
-        const float2 gr = *reinterpret_cast<const float2*>(a.grad + pi * 2);
-        const float mag = sqrtf(gr.x * gr.x + gr.y * gr.y);
-        const BmScales S = bm_scales(a, in.x, mag);
-        const float L2 = S.L * S.L;
-        // the forward's sums: outputs and the two kernel norms
-        const float4 dv = *reinterpret_cast<const float4*>(a.den + pi * 4);
-        const float Yo = dv.x, Cbo = dv.y, Cro = dv.z, ny = dv.w, nc = a.nc[pi];
-        const float3 g = *reinterpret_cast<const float3*>(a.g_den + pi * 3);
-        const float gYn = g.x / ny, gCbn = g.y / nc, gCrn = g.z / nc;
-        // gradients of the centre's own quantities, tap by tap
-        float gL = 0, gK1 = 0, gK2 = 0, gcb = 0, gcr = 0;
-        float gip[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int j = 0; j < 21; j++)
-            for (int i = 0; i < 21; i++) {
-                const int q = (threadIdx.y + j) * AW_ + threadIdx.x + i;
-                const float4 s = sm.q[q][0], p0 = sm.q[q][1], p1 = sm.q[q][2];
-                const float sp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-                float d2 = 0.f;
+    const int pair = threadIdx.y / KS, part = threadIdx.y % KS;
+    BwdPix pix[2];
 #pragma unroll
-                for (int k = 0; k < 8; k++) d2 += (sp[k] - ip[k]) * (sp[k] - ip[k]);
-                const float lw = __expf(-2.f * d2 * L2);
-                const float dcb = s.y - in.y, dcr = s.z - in.z;
-                const float c1 = dcb * S.K1, c2 = dcr * S.K2;
-                const float cw = __expf(-2.f * (lw * lw + c1 * c1 + c2 * c2));
-                const float sw = sm.sw[j * 21 + i];
-                const float gw = gYn * (s.x - Yo);
-                const float gc = gCbn * (s.y - Cbo) + gCrn * (s.z - Cro);
-                const float garg = -2.f * gc * sw * cw;
-                const float glw = gw * sw + 2.f * garg * lw;
-                const float gc1 = 2.f * garg * c1, gc2 = 2.f * garg * c2;
-                const float gE = -2.f * glw * lw;  // E = d2 L^2
-                gL += gE * 2.f * d2 * S.L;
-                const float gd2 = gE * L2;
-#pragma unroll
-                for (int k = 0; k < 8; k++) gip[k] -= 2.f * gd2 * (sp[k] - ip[k]);
-                gK1 += gc1 * dcb;
-                gK2 += gc2 * dcr;
-                gcb -= gc1 * S.K1;
-                gcr -= gc2 * S.K2;
+    for (int p = 0; p < 2; p++) {
+        const int c = (2 * pair + p + AH) * T::W + threadIdx.x + AH;
+        const float4 v0 = sm.v[0][c], v1 = sm.v[1][c], v2 = sm.v[2][c], p0 = sm.v[3][c], p1 = sm.v[4][c];
+        BwdPix& x = pix[p];
+        x.n[0] = pk2(-p0.x, -p0.y);
+        x.n[1] = pk2(-p0.z, -p0.w);
+        x.n[2] = pk2(-p1.x, -p1.y);
+        x.n[3] = pk2(-p1.z, -p1.w);
+        x.Y = v0.x;
+        x.kl = v0.y;
+        x.nc = pk2(-v0.z, -v0.w);
+        x.gY = v1.x;
+        x.gYd = v1.y;
+        x.gcd = v1.z;
+        x.g1 = v2.x;
+        x.g2 = v2.y;
+        x.K1 = v2.z;
+        x.K2 = v2.w;
+        x.p[0] = x.p[1] = x.p[2] = x.p[3] = 0;
+        x.E = x.luma = x.c1 = x.c2 = x.cc1 = x.cc2 = x.mean1 = x.mean2 = x.n1 = x.n2 = 0.f;
+    }
+    const int base = 2 * pair * T::W + threadIdx.x;
+    // row r of the box of the pair of pixels: row r of the upper's, r - 1 of the lower's
+    auto row = [&](int r, auto up, auto lo, auto at_border) {
+        float2 wu = make_float2(0.f, 0.f), wl = wu;
+        if constexpr (at_border) {
+            if (up) wu = sm.b.y[2 * pair][r];
+            if (lo) wl = sm.b.y[2 * pair + 1][r - 1];
+        }
+#pragma unroll 3
+        for (int i = 0; i < 21; i++) {
+            const int k = base + r * T::W + i;
+            const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(&sm.v[3][k]);
+            const ulonglong2 q1 = *reinterpret_cast<const ulonglong2*>(&sm.v[4][k]);
+            const float4 v0 = sm.v[0][k], v1 = sm.v[1][k], v2 = sm.v[2][k];
+            if constexpr (at_border) {
+                const float c = sm.b.cx[threadIdx.x][i], n = sm.b.nx[threadIdx.x][i];
+                if (up) bwd_pair(pix[0], q0, q1, v0, v1, v2, c * wu.x, n * wu.y);
+                if (lo) bwd_pair(pix[1], q0, q1, v0, v1, v2, c * wl.x, n * wl.y);
+            } else {
+                const float2 w = sm.sw[r][i];
+                if (up) bwd_pair(pix[0], q0, q1, v0, v1, v2, w.x, w.x);
+                if (lo) bwd_pair(pix[1], q0, q1, v0, v1, v2, w.y, w.y);
             }
+        }
+    };
+    auto rows = [&](auto at_border) {
+        constexpr std::true_type yes{};
+        constexpr std::false_type no{};
+        if (part == 0) row(0, yes, no, at_border);
+#pragma unroll 1
+        for (int r = part == 0 ? KS : part; r <= 20; r += KS) row(r, yes, yes, at_border);
+        if (part == 21 % KS) row(21, no, yes, at_border);
+    };
+    if (border)
+        rows(std::true_type{});
+    else
+        rows(std::false_type{});
+    if constexpr (KS > 1) {  // the parts' sums, in order
+        static_assert(256 * 36 * sizeof(float) <= sizeof(typename T::Smem), "the sums take the staging's place");
+        __syncthreads();
+        float* t = reinterpret_cast<float*>(smem_raw) + tid;
+        auto each = [&](auto f) {
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                BwdPix& x = pix[p];
+                float* const one[10] = {&x.E, &x.luma, &x.c1, &x.c2, &x.cc1, &x.cc2, &x.mean1, &x.mean2, &x.n1, &x.n2};
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    float2 v = up2(x.p[c]);
+                    f(v.x, 18 * p + 2 * c);
+                    f(v.y, 18 * p + 2 * c + 1);
+                    x.p[c] = pk2(v.x, v.y);
+                }
+#pragma unroll
+                for (int c = 0; c < 10; c++) f(*one[c], 18 * p + 8 + c);
+            }
+        };
+        each([&](float& v, int c) { t[c * 256] = v; });
+        __syncthreads();
+        if (part == 0) each([&](float& v, int c) {
+#pragma unroll
+            for (int k = 1; k < KS; k++) v += t[c * 256 + k * AT_X];
+        });
+    }
+    float th[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+        const BwdPix& v = pix[p];
+        const int x = x0 + threadIdx.x, y = y0 + 2 * pair + p;
+        if (part != 0 || x >= W || y >= H) continue;
+        const size_t pi = size_t(y) * W + x;
+        const float2 gr = *reinterpret_cast<const float2*>(a.grad + pi * 2);
+        const BmScales S = bm_scales(a, v.Y, sqrtf(gr.x * gr.x + gr.y * gr.y));
+        const float gL = -4.f / kAdjS * S.L * v.E;
+        const float gK1 = -kAdjS * S.K1 * v.cc1, gK2 = -kAdjS * S.K2 * v.cc2;
         // scales -> centre luma and theta (ls = 1: no lens shading on this path)
         const float gsig0 = gL * S.dL_dsig0, gsig1 = gK1 * S.dK1_dsig1, gsig2 = gK2 * S.dK2_dsig2;
         const float gY = gsig0 * a.var_b[0] / (2.f * S.sig0) + gsig1 * a.var_b[1] / (2.f * S.sig1) +
                          gsig2 * a.var_b[2] / (2.f * S.sig2);
-        th[0] = gL * (-S.L / a.tm[0]);                                     // luma
-        th[1] = gK1 * (-S.K1 / a.tm[1]) + gK2 * (-S.K2 / a.tm[2]);        // chroma
-        th[2] = gsig0 / (2.f * S.sig0);                                    // A_Y
-        th[3] = gsig0 * in.x / (2.f * S.sig0);                             // B_Y
-        th[4] = gsig1 / (2.f * S.sig1) + gsig2 / (2.f * S.sig2);           // A_C (a[1] = a[2])
-        th[5] = (gsig1 / (2.f * S.sig1) + gsig2 / (2.f * S.sig2)) * in.x;  // B_C
-        float* rec = a.rec + pi * 12;
-        *reinterpret_cast<float4*>(rec) = make_float4(gYn, Yo, gCbn, Cbo);
-        *reinterpret_cast<float4*>(rec + 4) = make_float4(gCrn, Cro, S.L, S.K1);
-        *reinterpret_cast<float4*>(rec + 8) = make_float4(S.K2, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(a.g_layer + pi * 4) = make_float4(gY, gcb, gcr, 0.f);
-        *reinterpret_cast<float4*>(a.g_pca + pi * 8) = make_float4(gip[0], gip[1], gip[2], gip[3]);
-        *reinterpret_cast<float4*>(a.g_pca + pi * 8 + 4) = make_float4(gip[4], gip[5], gip[6], gip[7]);
+        const float aY = gsig0 / (2.f * S.sig0), aC = gsig1 / (2.f * S.sig1) + gsig2 / (2.f * S.sig2);
+        th[0] += gL * (-S.L / a.tm[0]);                               // luma
+        th[1] += gK1 * (-S.K1 / a.tm[1]) + gK2 * (-S.K2 / a.tm[2]);  // chroma
+        th[2] += aY;                                                  // A_Y
+        th[3] += aY * v.Y;                                            // B_Y
+        th[4] += aC;                                                  // A_C (a[1] = a[2])
+        th[5] += aC * v.Y;                                            // B_C
+        *reinterpret_cast<float4*>(a.g_layer + pi * 4) =
+            make_float4(gY + v.luma / kAdjS, 0.25f * kAdjS * v.mean1 + fmaf(v.K1, v.c1, v.n1) / kAdjS,
+                        0.25f * kAdjS * v.mean2 + fmaf(v.K2, v.c2, v.n2) / kAdjS, 0.f);
+        const float k = -4.f / (kAdjS * kAdjS * kAdjS);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const float2 u = up2(v.p[2 * c]), w = up2(v.p[2 * c + 1]);
+            *reinterpret_cast<float4*>(a.g_pca + pi * 8 + 4 * c) = make_float4(k * u.x, k * u.y, k * w.x, k * w.y);
+        }
     }
     // per-block theta partials, warp then block, fixed order
 #pragma unroll
@@ -210,115 +430,17 @@ __global__ void __launch_bounds__(256) k_bm_bwd_center(AdjointLevelArgs a) {
     __syncthreads();
     if (tid < 6) {
         float v = 0.f;
-        for (int w = 0; w < 8; w++) v += red[w][tid];
+        for (int w = 0; w < T::WARPS; w++) v += red[w][tid];
         a.part[(size_t(blockIdx.y) * gridDim.x + blockIdx.x) * 6 + tid] = v;
     }
 }
 
-// The neighbour pass stages 80 bytes per window position, so its tile is
-// taller than the centre pass's: 32 x 16 pixels and 512 threads per block
-// stage 52 x 36 positions (3.7 per pixel instead of 5.7) in 150 KB, and a
-// block holds 16 warps on its SM.
-constexpr int NT_Y = 16, NH_ = NT_Y + 2 * AH, NT_THREADS = AT_X * NT_Y;
-
-struct NeighborSmem {
-    float4 p[NH_ * AW_][5];  // (gYn, Yo, gCbn, Cbo), (gCrn, Cro, L, K1), (K2, cb, cr, -), pca 0..3, pca 4..7
-    float sw[441];
-};
-
-// Block matching, the pixel q as a neighbour of every centre p whose
-// window reads it (p in the 21 x 21 box around q; at the image border,
-// every tap offset that clamps onto q).
-__global__ void __launch_bounds__(NT_THREADS, 1) k_bm_bwd_neighbor(AdjointLevelArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    NeighborSmem& sm = *reinterpret_cast<NeighborSmem*>(smem_raw);
-    const int W = a.w, H = a.h;
-    const int x0 = blockIdx.x * AT_X, y0 = blockIdx.y * NT_Y;
-    const int tid = threadIdx.y * AT_X + threadIdx.x;
-    for (int k = tid; k < 441; k += NT_THREADS) sm.sw[k] = spatial_w(k % 21 - 10, k / 21 - 10);
-    for (int k = tid; k < NH_ * AW_; k += NT_THREADS) {
-        const int ty = k / AW_, tx = k % AW_;
-        const int px = x0 - AH + tx, py = y0 - AH + ty;
-        if (px < 0 || px >= W || py < 0 || py >= H) continue;  // not a pixel: never read
-        const size_t pi = size_t(py) * W + px;
-        const float* rec = a.rec + pi * 12;
-        const float4 l = *reinterpret_cast<const float4*>(a.layer + pi * 4);
-        sm.p[k][0] = *reinterpret_cast<const float4*>(rec);
-        sm.p[k][1] = *reinterpret_cast<const float4*>(rec + 4);
-        sm.p[k][2] = make_float4(rec[8], l.y, l.z, 0.f);
-        sm.p[k][3] = *reinterpret_cast<const float4*>(a.pca + pi * 8);
-        sm.p[k][4] = *reinterpret_cast<const float4*>(a.pca + pi * 8 + 4);
-    }
-    __syncthreads();
-    const int qx = x0 + threadIdx.x, qy = y0 + threadIdx.y;
-    if (qx >= W || qy >= H) return;
-    const size_t qi = size_t(qy) * W + qx;
-    const float4 s = *reinterpret_cast<const float4*>(a.layer + qi * 4);
-    const float4 q0 = *reinterpret_cast<const float4*>(a.pca + qi * 8);
-    const float4 q1 = *reinterpret_cast<const float4*>(a.pca + qi * 8 + 4);
-    const float sp[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-    float gs0 = 0, gs1 = 0, gs2 = 0;
-    float gsp[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    // the contribution of centre p reading q through tap offset (i, j)
-    auto pair = [&](int k, int ilo, int ihi, int jlo, int jhi) {
-        const float4 r0 = sm.p[k][0], r1 = sm.p[k][1], r2 = sm.p[k][2], c0 = sm.p[k][3], c1v = sm.p[k][4];
-        const float gYn = r0.x, Yo = r0.y, gCbn = r0.z, Cbo = r0.w;
-        const float gCrn = r1.x, Cro = r1.y, L = r1.z, K1 = r1.w, K2 = r2.x, cbp = r2.y, crp = r2.z;
-        const float ip[8] = {c0.x, c0.y, c0.z, c0.w, c1v.x, c1v.y, c1v.z, c1v.w};
-        float d2 = 0.f;
-#pragma unroll
-        for (int m = 0; m < 8; m++) d2 += (sp[m] - ip[m]) * (sp[m] - ip[m]);
-        const float L2 = L * L;
-        const float lw = __expf(-2.f * d2 * L2);
-        const float dcb = s.y - cbp, dcr = s.z - crp;
-        const float c1 = dcb * K1, c2 = dcr * K2;
-        const float cw = __expf(-2.f * (lw * lw + c1 * c1 + c2 * c2));
-        const float gw = gYn * (s.x - Yo);
-        const float gc = gCbn * (s.y - Cbo) + gCrn * (s.z - Cro);
-        float gd2 = 0.f;
-        for (int j = jlo; j <= jhi; j++)
-            for (int i = ilo; i <= ihi; i++) {
-                const float sw = sm.sw[(j + AH) * 21 + i + AH];
-                const float wy = sw * lw, wc = sw * cw;
-                const float garg = -2.f * gc * sw * cw;
-                const float glw = gw * sw + 2.f * garg * lw;
-                gs0 += gYn * wy;
-                gs1 += gCbn * wc + 2.f * garg * c1 * K1;
-                gs2 += gCrn * wc + 2.f * garg * c2 * K2;
-                gd2 += -2.f * glw * lw * L2;
-            }
-#pragma unroll
-        for (int m = 0; m < 8; m++) gsp[m] += 2.f * gd2 * (sp[m] - ip[m]);
-    };
-    const int py0 = max(qy - AH, 0), py1 = min(qy + AH, H - 1);
-    const int px0 = max(qx - AH, 0), px1 = min(qx + AH, W - 1);
-    if (qx > 0 && qx < W - 1 && qy > 0 && qy < H - 1) {
-        // not on the image border: every centre reads q through exactly one tap
-        for (int py = py0; py <= py1; py++) {
-            const int j = qy - py;
-            for (int px = px0; px <= px1; px++) {
-                const int i = qx - px;
-                pair((py - y0 + AH) * AW_ + (px - x0 + AH), i, i, j, j);
-            }
-        }
-    } else {
-        for (int py = py0; py <= py1; py++) {
-            int jlo, jhi;
-            if (!preimage(qy, py, AH, H, jlo, jhi)) continue;
-            for (int px = px0; px <= px1; px++) {
-                int ilo, ihi;
-                if (!preimage(qx, px, AH, W, ilo, ihi)) continue;
-                pair((py - y0 + AH) * AW_ + (px - x0 + AH), ilo, ihi, jlo, jhi);
-            }
-        }
-    }
-    float4* gl = reinterpret_cast<float4*>(a.g_layer + qi * 4);
-    const float4 cur = *gl;
-    *gl = make_float4(cur.x + gs0, cur.y + gs1, cur.z + gs2, 0.f);
-    float4* gp = reinterpret_cast<float4*>(a.g_pca + qi * 8);
-    const float4 p0 = gp[0], p1 = gp[1];
-    gp[0] = make_float4(p0.x + gsp[0], p0.y + gsp[1], p0.z + gsp[2], p0.w + gsp[3]);
-    gp[1] = make_float4(p1.x + gsp[4], p1.y + gsp[5], p1.z + gsp[6], p1.w + gsp[7]);
+// Window rows dealt to four warps while there are fewer than four 32 x 16 tiles
+// for each of the chip's 148 SMs: 512x384 (384 tiles) 305 us, 339 without.
+static int bwd_split(int w, int h) { return ((w + AT_X - 1) / AT_X) * ((h + 15) / 16) < 4 * 148 ? 4 : 1; }
+static dim3 bwd_grid(int w, int h) {
+    const int rows = bwd_split(w, h) == 4 ? BwdTile<4>::ROWS : BwdTile<1>::ROWS;
+    return dim3((w + AT_X - 1) / AT_X, (h + rows - 1) / rows);
 }
 
 // pcaProjection transposed (demosaic.metal:774-796): dL/d luma(x) +=
@@ -596,9 +718,6 @@ void launch_unpack3(const float* src, float* dst, size_t pitch_floats, int chann
     k_unpack3<<<g, b, 0, s>>>(src, dst, pitch_floats, channels, w, h);
 }
 
-size_t adjoint_center_smem() { return sizeof(CenterSmem); }
-size_t adjoint_neighbor_smem() { return sizeof(NeighborSmem); }
-
 void launch_adj_head(const float* den0, const float* target, int tstride, int w, int h, const AdjointHeadArgs& a,
                      float* g_den, double* loss_part, cudaStream_t s) {
     const dim3 b(32, 8), g((w + 31) / 32, (h + 7) / 8);
@@ -606,13 +725,16 @@ void launch_adj_head(const float* den0, const float* target, int tstride, int w,
 }
 
 void launch_bm_bwd(const AdjointLevelArgs& a, cudaStream_t s) {
-    ensure_dynamic_smem(reinterpret_cast<const void*>(k_bm_bwd_center), int(sizeof(CenterSmem)));
-    ensure_dynamic_smem(reinterpret_cast<const void*>(k_bm_bwd_neighbor), int(sizeof(NeighborSmem)));
-    const dim3 b(AT_X, AT_Y), g((a.w + AT_X - 1) / AT_X, (a.h + AT_Y - 1) / AT_Y);
-    k_bm_bwd_center<<<g, b, sizeof(CenterSmem), s>>>(a);
-    const dim3 nb(AT_X, NT_Y), ng((a.w + AT_X - 1) / AT_X, (a.h + NT_Y - 1) / NT_Y);
-    k_bm_bwd_neighbor<<<ng, nb, sizeof(NeighborSmem), s>>>(a);
-    const dim3 b2(32, 8), g2((a.w + 31) / 32, (a.h + 7) / 8);
+    const dim3 b2(32, 8), g2((a.w + 31) / 32, (a.h + 7) / 8), g = bwd_grid(a.w, a.h);
+    k_bm_bwd_record<<<g2, b2, 0, s>>>(a);
+    auto run = [&](auto kernel, int warps, size_t bytes) {
+        ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), int(bytes));
+        kernel<<<g, dim3(AT_X, warps), bytes, s>>>(a);
+    };
+    if (bwd_split(a.w, a.h) == 4)
+        run(k_bm_bwd<4>, BwdTile<4>::WARPS, sizeof(BwdTile<4>::Smem));
+    else
+        run(k_bm_bwd<1>, BwdTile<1>::WARPS, sizeof(BwdTile<1>::Smem));
     k_pca_bwd<<<g2, b2, 0, s>>>(a);
 }
 
@@ -633,7 +755,10 @@ void launch_down_bwd(const float* g_coarse, int cw, int ch, float* g_fine, int w
     k_down_bwd<<<g, b, 0, s>>>(g_coarse, cw, ch, g_fine, w, h, float(w) / float(cw), float(h) / float(ch));
 }
 
-int adjoint_blocks(int w, int h) { return ((w + AT_X - 1) / AT_X) * ((h + AT_Y - 1) / AT_Y); }
+int adjoint_blocks(int w, int h) {
+    const dim3 g = bwd_grid(w, h);
+    return int(g.x * g.y);
+}
 int adjoint_sn_blocks(int w, int h) { return ((w + 31) / 32) * ((h + 7) / 8); }
 
 }  // namespace gls

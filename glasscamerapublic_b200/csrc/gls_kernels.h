@@ -215,7 +215,7 @@ struct AdjointLevelArgs {
     const float* pca;    // 8 ch, projected with `basis`
     const float* basis;  // 25 x 8 (device)
     const float* g_den;  // 3 ch: dL/d(block-matching output Y, Cb, Cr)
-    float* rec;          // 12 per pixel: centre record for the neighbour pass
+    float* rec;          // 12 per pixel: what its pairs need of a pixel
     float* g_layer;      // 4 ch out: dL/d layer (Y, Cb, Cr)
     float* g_pca;        // 8 ch scratch
     float* part;         // per-block dL/dtheta: luma, chroma, A_Y, B_Y, A_C, B_C

@@ -93,6 +93,26 @@ def test_adjoint_input_gradient_matches_autograd(converter):
     assert np.abs(g_ds - g_ref).max() <= 1e-3 * np.abs(g_ref).max()
 
 
+@pytest.mark.parametrize("size", [(16, 12), (38, 26), (34, 70), (774, 394)])
+def test_adjoint_at_the_edges_of_its_tiles(converter, size):
+    """One level: images smaller than a window, tiles cut on the right and at
+    the bottom, and (the largest) the tiles that are not split over warps."""
+    w, h = size
+    wl = scene.Workload("adj", w, h, levels=1, gain=0.8, read=3.0, iso=800, seed=90 + w)
+    raw, clean = scene.make_raw(wl)
+    p = scene.make_params(wl)
+    target = scene.target_rgb(clean).astype(np.float32)
+    loss, grad = A.loss_and_grad(converter, raw, p, target)
+    g_ds = converter.plane(g.PLANE_ADJ_DESPECKLED)
+    ds, gplane = converter.plane(g.PLANE_DESPECKLED), converter.plane(g.PLANE_GRADIENT)
+    _, inv = O.cam_ycbcr(np.eye(3), scene.XYZ_SRGB)
+    loss_t, g_t, _, g_ref = TP.loss_and_grad(ds, gplane, p, converter.pca_basis(0)[None].astype(np.float64), inv, target,
+                                             with_ds=True, device="cuda", checkpoint=True)
+    torch.cuda.empty_cache()
+    _check(loss, grad, loss_t, g_t, 1)
+    assert np.abs(g_ds - g_ref).max() <= 1e-3 * np.abs(g_ref).max()
+
+
 def _front_loss(raw, p, grad, bases, inv, target):
     """The loss with the front end from the FP64 oracle's stages and the
     pyramid from the FP64 oracle (bases and gradient plane fixed)."""
