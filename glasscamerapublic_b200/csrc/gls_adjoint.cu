@@ -445,33 +445,67 @@ static dim3 bwd_grid(int w, int h) {
 
 // pcaProjection transposed (demosaic.metal:774-796): dL/d luma(x) +=
 // sum over the patches that read x of basis . dL/d pca.
+// Bound by shared memory: two vertically adjacent pixels a thread read 30
+// positions' 8 values (240 wavefronts a warp) and the basis (50, broadcasts)
+// from a staged 36 x 20 region, 0 outside the image; 2048x1536: 131 us, 609
+// with every value from global memory. Pixels on the image border, which
+// several taps of a patch can read, take the general sum.
+constexpr int PB_H = 16;
 __global__ void __launch_bounds__(256) k_pca_bwd(AdjointLevelArgs a) {
-    __shared__ float B[25][8];
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    if (tid < 200) B[tid / 8][tid % 8] = a.basis[tid];
-    __syncthreads();
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= a.w || y >= a.h) return;
-    float acc = 0.f;
-    for (int py = max(y - 2, 0); py <= min(y + 2, a.h - 1); py++) {
-        int jlo, jhi;
-        if (!preimage(y, py, 2, a.h, jlo, jhi)) continue;
-        for (int px = max(x - 2, 0); px <= min(x + 2, a.w - 1); px++) {
-            int ilo, ihi;
-            if (!preimage(x, px, 2, a.w, ilo, ihi)) continue;
-            const float* gp = a.g_pca + (size_t(py) * a.w + px) * 8;
-            float g[8];
-#pragma unroll
-            for (int m = 0; m < 8; m++) g[m] = gp[m];
-            for (int j = jlo; j <= jhi; j++)
-                for (int i = ilo; i <= ihi; i++) {
-                    const int row = (j + 2) * 5 + (i + 2);
-#pragma unroll
-                    for (int m = 0; m < 8; m++) acc += B[row][m] * g[m];
-                }
-        }
+    __shared__ float4 B[25][2], g[2][(PB_H + 4) * (AT_X + 4)];
+    const int tid = threadIdx.y * AT_X + threadIdx.x;
+    const int x0 = blockIdx.x * AT_X, y0 = blockIdx.y * PB_H;
+    if (tid < 50) B[tid / 2][tid % 2] = reinterpret_cast<const float4*>(a.basis)[tid];
+    for (int k = tid; k < 2 * (PB_H + 4) * (AT_X + 4); k += 256) {
+        const int q = k >> 1, px = x0 - 2 + q % (AT_X + 4), py = y0 - 2 + q / (AT_X + 4);
+        const bool in = px >= 0 && px < a.w && py >= 0 && py < a.h;
+        g[k & 1][q] = in ? reinterpret_cast<const float4*>(a.g_pca)[(size_t(py) * a.w + px) * 2 + (k & 1)]
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    a.g_layer[(size_t(y) * a.w + x) * 4] += acc;
+    __syncthreads();
+    const int x = x0 + threadIdx.x, yt = 2 * threadIdx.y;
+    float acc[2] = {0.f, 0.f};
+#pragma unroll
+    for (int r = 0; r < 6; r++)  // position (x + i - 2, y0 + yt + r - 2) reads x through tap 2 - i, row offset 2 - r (+ 1)
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            const int q = (yt + r) * (AT_X + 4) + threadIdx.x + i;
+            const float4 u = g[0][q], v = g[1][q];
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                const int j = 4 - r + p;
+                if (j < 0 || j > 4) continue;
+                const float4 b = B[j * 5 + 4 - i][0], c = B[j * 5 + 4 - i][1];
+                acc[p] = fmaf(b.x, u.x, fmaf(b.y, u.y, fmaf(b.z, u.z, fmaf(b.w, u.w, acc[p]))));
+                acc[p] = fmaf(c.x, v.x, fmaf(c.y, v.y, fmaf(c.z, v.z, fmaf(c.w, v.w, acc[p]))));
+            }
+        }
+    if (x >= a.w) return;
+    for (int p = 0; p < 2; p++) {
+        const int y = y0 + yt + p;
+        if (y >= a.h) break;
+        if (x == 0 || x == a.w - 1 || y == 0 || y == a.h - 1) {
+            float s = 0.f;
+            for (int py = max(y - 2, 0); py <= min(y + 2, a.h - 1); py++) {
+                int jlo, jhi;
+                if (!preimage(y, py, 2, a.h, jlo, jhi)) continue;
+                for (int px = max(x - 2, 0); px <= min(x + 2, a.w - 1); px++) {
+                    int ilo, ihi;
+                    if (!preimage(x, px, 2, a.w, ilo, ihi)) continue;
+                    const int q = (py - y0 + 2) * (AT_X + 4) + px - x0 + 2;
+                    const float4 u = g[0][q], v = g[1][q];
+                    for (int j = jlo; j <= jhi; j++)
+                        for (int i = ilo; i <= ihi; i++) {
+                            const float4 b = B[(j + 2) * 5 + i + 2][0], c = B[(j + 2) * 5 + i + 2][1];
+                            s += b.x * u.x + b.y * u.y + b.z * u.z + b.w * u.w + c.x * v.x + c.y * v.y + c.z * v.z +
+                                 c.w * v.w;
+                        }
+                }
+            }
+            acc[p] = s;
+        }
+        a.g_layer[(size_t(y) * a.w + x) * 4] += acc[p];
+    }
 }
 
 // 2 (out - target) / N through the output transform; the loss per block.
@@ -735,7 +769,7 @@ void launch_bm_bwd(const AdjointLevelArgs& a, cudaStream_t s) {
         run(k_bm_bwd<4>, BwdTile<4>::WARPS, sizeof(BwdTile<4>::Smem));
     else
         run(k_bm_bwd<1>, BwdTile<1>::WARPS, sizeof(BwdTile<1>::Smem));
-    k_pca_bwd<<<g2, b2, 0, s>>>(a);
+    k_pca_bwd<<<dim3((a.w + AT_X - 1) / AT_X, (a.h + PB_H - 1) / PB_H), dim3(AT_X, PB_H / 2), 0, s>>>(a);
 }
 
 void launch_sn_bwd(const AdjointSnArgs& a, cudaStream_t s) {
