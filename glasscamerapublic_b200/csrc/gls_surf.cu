@@ -31,6 +31,7 @@
 #include "gls_common.cuh"
 #include "gls_devbuf.h"
 #include "gls_fmath.h"
+#include "gls_kernels.h"
 #include "gls_warp.cuh"
 
 namespace gls {
@@ -96,6 +97,7 @@ struct DetectArgs {
     int n_oct;
     const float* sum;
     int sum_pitch;  // floats
+    int sum_w, sum_h;
     float threshold;
     int per_axis;  // corrected interpolation (else the reference's scale-offset broadcast)
     gls_keypoint* cand;
@@ -181,7 +183,51 @@ __device__ __forceinline__ float det3(const float a[3], const float b[3], const 
     return fadd(fadd(fmul(a[0], cx), fmul(a[1], cy)), fmul(a[2], cz));
 }
 
-constexpr int DT_X = 32, DT_Y = 8;  // NMS positions per detector tile
+// A detector tile: 64 x 32 samples, NMS positions the 62 x 30 inside. A thread
+// evaluates 8 rows of a column, so that a box corner's address is formed once
+// for 8 samples; the first octave's tiles (three quarters of all samples) read
+// the corners from the integral image's region in shared memory, one wavefront
+// a read where the unaligned global read takes two, the later octaves' regions
+// do not fit.
+constexpr int DS_X = 64, DS_Y = 32, DS_R = 8;
+constexpr int DT_X = DS_X - 2, DT_Y = DS_Y - 2;
+constexpr int DR_W = DS_X + 27, DR_H = DS_Y + 27;  // region of the first octave: its largest wavelet spans 27
+
+struct DetectSmem {
+    int4 corner[kLayers][8];  // corner offsets of the 8 boxes, in rect_gpu's order
+    float det[kLayers][DS_Y][DS_X];
+    float sum[DR_H][DR_W];
+};
+
+// calcHaarPatternDx / Dy / Dxy + the determinant (SURF.metal:77-145) of DS_R
+// samples, `dy` floats apart.
+__device__ __forceinline__ void det_column(const float* __restrict__ p, const int4 (&corner)[8], int dy, float w,
+                                           float wxy, float (&det)[DS_R]) {
+    auto box = [&](int k, float (&v)[DS_R]) {
+        const int4 c = corner[k];
+        const float *q0 = p + c.x, *q1 = p + c.y, *q2 = p + c.z, *q3 = p + c.w;
+#pragma unroll
+        for (int r = 0; r < DS_R; r++) v[r] = rect_gpu(q0[r * dy], q1[r * dy], q2[r * dy], q3[r * dy]);
+    };
+    float u[DS_R], v[DS_R], dx[DS_R];
+    box(0, u);
+    box(1, v);
+#pragma unroll
+    for (int r = 0; r < DS_R; r++) dx[r] = fmul(w, fsub(u[r], fmul(3.0f, v[r])));
+    box(2, u);
+    box(3, v);
+#pragma unroll
+    for (int r = 0; r < DS_R; r++) det[r] = fmul(dx[r], fmul(w, fsub(u[r], fmul(3.0f, v[r]))));
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        box(4 + k, u);
+#pragma unroll
+        for (int r = 0; r < DS_R; r++)
+            v[r] = fadd(k == 0 ? 0.0f : v[r], fmul(k == 0 || k == 3 ? wxy : -wxy, u[r]));
+    }
+#pragma unroll
+    for (int r = 0; r < DS_R; r++) det[r] = fsub(det[r], fmul(fmul(0.81f, v[r]), v[r]));
+}
 
 // A feature slot's count, set from a host value (gls_surf_load_features).
 __global__ void k_store_count(int* count, int n) { *count = n; }
@@ -191,51 +237,89 @@ __global__ void k_store_count(int* count, int n) { *count = n; }
 // (SURF.metal:249-313) with interpolateKeypoint (:207-247) for the two
 // middle layers. Determinants outside a layer's margin crop are 0, as an
 // unwritten determinant plane.
+//
+// What bounds it: 32 corner reads and some 90 instructions a sample and layer.
+// 2016x1512: 171 us; 423 when every sample formed its corners' addresses (480
+// instructions a sample, tiles of 32 x 8 positions).
 __global__ void __launch_bounds__(256) k_hessian_nms(DetectArgs a) {
-    __shared__ float det[kLayers][DT_Y + 2][DT_X + 2];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    DetectSmem& sm = *reinterpret_cast<DetectSmem*>(smem_raw);
+    auto& det = sm.det;
+    // the later octaves first: their blocks take the longest
+    const int block = gridDim.x - 1 - blockIdx.x;
     int o = 0;
-    while (o + 1 < a.n_oct && int(blockIdx.x) >= a.oct[o + 1].block0) o++;
+    while (o + 1 < a.n_oct && block >= a.oct[o + 1].block0) o++;
     const OctaveDev& O = a.oct[o];
-    const int b = blockIdx.x - O.block0;
+    const int b = block - O.block0;
     const int bx = b % O.tiles_x, by = b / O.tiles_x;
-    const int x0 = bx * DT_X, y0 = by * DT_Y;
+    const int x0 = bx * DT_X - 1, y0 = by * DT_Y - 1;  // first sample
     const int step = O.step;
-    for (int i = threadIdx.x; i < kLayers * (DT_Y + 2) * (DT_X + 2); i += blockDim.x) {
-        const int l = i / ((DT_Y + 2) * (DT_X + 2));
-        const int r = i % ((DT_Y + 2) * (DT_X + 2));
-        const int ly = r / (DT_X + 2), lx = r % (DT_X + 2);
-        const int gx = x0 + lx - 1, gy = y0 + ly - 1;
-        const LayerDev& L = O.layer[l];
-        const int ix = gx - L.mx, iy = gy - L.my;
-        float d = 0.0f;
-        if (ix >= 0 && ix < L.mw && iy >= 0 && iy < L.mh) {
-            float t;
-            det_trace_at(a.sum, a.sum_pitch, ix * step, iy * step, L, &d, &t);
+    const int tx = threadIdx.x % DS_X, ty = threadIdx.x / DS_X * DS_R;
+    // first octave: layer l reads [x - (4 + 3 l), x + 5 + 3 l], at most 13 before and 14 after
+    const int rx = x0 - 13, ry = y0 - 13;
+    if (o == 0) {
+        for (int i = threadIdx.x; i < DR_W * DR_H; i += 256) {
+            const int x = rx + i % DR_W, y = ry + i / DR_W;
+            (&sm.sum[0][0])[i] = x >= 0 && x < a.sum_w && y >= 0 && y < a.sum_h ? __ldg(a.sum + size_t(y) * a.sum_pitch + x) : 0.0f;
         }
-        det[l][ly][lx] = d;
+    }
+    if (threadIdx.x < kLayers * 32) {
+        const int l = threadIdx.x / 32, e = threadIdx.x % 32;
+        const LayerDev& L = O.layer[l];
+        // r97 r92 r07 r02, r67 r62 r37 r32; r79 r70 r29 r20, r76 r73 r26 r23
+        const int order = int((0x1435062723450167ull >> (4 * (e % 16))) & 15);
+        const short* c = e < 8 ? L.dx[order] : e < 16 ? L.dy[order] : L.dxy[(e - 16) / 4][e % 4];
+        reinterpret_cast<int*>(sm.corner[l])[e] = c[1] * (o == 0 ? DR_W : a.sum_pitch) + c[0];
     }
     __syncthreads();
-    const int tx = threadIdx.x % DT_X, ty = threadIdx.x / DT_X;
-    const int x = x0 + tx, y = y0 + ty;
+#pragma unroll 1
+    for (int l = 0; l < kLayers; l++) {
+        const LayerDev& L = O.layer[l];
+        const int ix = x0 + tx - L.mx, iy = y0 + ty - L.my;
+        float d[DS_R];
+        const bool col = ix >= 0 && ix < L.mw;
+        if (o == 0) {
+            det_column(&sm.sum[y0 + ty - L.my - ry][x0 + tx - L.mx - rx], sm.corner[l], DR_W, L.w, L.wxy, d);
+        } else if (col && iy >= 0 && iy + DS_R <= L.mh) {
+            det_column(a.sum + size_t(iy * step) * a.sum_pitch + ix * step, sm.corner[l], step * a.sum_pitch, L.w, L.wxy,
+                       d);
+        } else {
+#pragma unroll 1
+            for (int r = 0; r < DS_R; r++) {
+                float v = 0.0f, t;
+                if (col && iy + r >= 0 && iy + r < L.mh)
+                    det_trace_at(a.sum, a.sum_pitch, ix * step, (iy + r) * step, L, &v, &t);
+                det[l][ty + r][tx] = v;
+            }
+            continue;
+        }
 #pragma unroll
-    for (int l = 1; l <= 2; l++) {
+        for (int r = 0; r < DS_R; r++) det[l][ty + r][tx] = col && iy + r >= 0 && iy + r < L.mh ? d[r] : 0.0f;
+    }
+    __syncthreads();
+    const int x = x0 + tx;
+    if (tx < 1 || tx > DT_X) return;
+#pragma unroll 1
+    for (int k = 0; k < 2 * DS_R; k++) {
+        const int l = 1 + k % 2, sy = ty + k / 2, y = y0 + sy;
+        if (sy < 1 || sy > DT_Y) continue;
+        const float v = det[l][sy][tx];
+        if (!(v > a.threshold)) continue;
         const LayerDev& L = O.layer[l];
         const int margin = (O.layer[l + 1].size / 2) / step + 1;
         if (x < margin || x >= O.lw - margin || y < margin || y >= O.lh - margin) continue;
-        const float v = det[l][ty + 1][tx + 1];
-        if (!(v > a.threshold)) continue;
         bool mx = true;
         for (int i = 0; i < 3 && mx; i++)
             for (int dy = -1; dy <= 1 && mx; dy++)
                 for (int dx = -1; dx <= 1; dx++) {
                     if (i == 1 && dx == 0 && dy == 0) continue;
-                    if (!(v > det[l - 1 + i][ty + 1 + dy][tx + 1 + dx])) {
+                    if (!(v > det[l - 1 + i][sy + dy][tx + dx])) {
                         mx = false;
                         break;
                     }
                 }
         if (!mx) continue;
-        auto n9 = [&](int i, int dy, int dx) { return det[l - 1 + i][ty + 1 + dy][tx + 1 + dx]; };
+        auto n9 = [&](int i, int dy, int dx) { return det[l - 1 + i][sy + dy][tx + dx]; };
         const int size = L.size, s0 = O.layer[l - 1].size;
         const int sum_y = step * (y - (size / 2) / step);
         const int sum_x = step * (x - (size / 2) / step);
@@ -1732,6 +1816,8 @@ gls_status gls_surf_detect_and_compute(gls_surf* s, const gls_image_view* img, i
     da.n_oct = s->n_oct;
     da.sum = S;
     da.sum_pitch = W + 1;
+    da.sum_w = W + 1;
+    da.sum_h = H + 1;
     da.threshold = s->threshold;
     da.per_axis = (flags & GLS_SURF_CORRECTED) ? 1 : 0;
     da.cand = reinterpret_cast<gls_keypoint*>(s->cand.p);
@@ -1749,7 +1835,8 @@ gls_status gls_surf_detect_and_compute(gls_surf* s, const gls_image_view* img, i
         blocks += O.tiles_x * O.tiles_y;
     }
     GLS_CUDA(cudaMemsetAsync(s->cand_count.p, 0, sizeof(int), st));
-    k_hessian_nms<<<blocks, 256, 0, st>>>(da);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(k_hessian_nms), int(sizeof(DetectSmem)));
+    k_hessian_nms<<<blocks, 256, sizeof(DetectSmem), st>>>(da);
     GLS_TRY(launch_check(s, "k_hessian_nms"));
     SurfSlotState& sl = s->slot[slot];
     const int keep = s->capacity;

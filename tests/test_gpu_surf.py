@@ -100,6 +100,41 @@ def test_detect_and_compute_bit_exact(max_features, seed):
         s.close()
 
 
+@pytest.mark.parametrize("w,h", [(40, 36), (62, 30), (63, 31), (124, 60), (125, 61), (190, 131)])
+def test_detect_at_tile_edges_bit_exact(w, h):
+    rng = np.random.default_rng(w)
+    img = rng.random((h, w), dtype=np.float32)
+    s = SURF(w, h, max_features=-1, hessianThreshold=0.001)
+    try:
+        kps, desc = s.detectAndCompute(img, slot=0)
+        rk, rd, _ = R.detect(img, max_features=-1, threshold=0.001)
+        assert len(kps) == len(rk) and (len(rk) > 0 or (w, h) == (62, 30))  # none fits one tile
+        for f in kps.dtype.names:
+            assert np.array_equal(kps[f], rk[f]), f
+        assert np.array_equal(desc, rd)
+    finally:
+        s.close()
+
+
+def test_detect_orders_equal_responses_bit_exact():
+    """A pattern that repeats in both directions: many candidates with the same
+    response, ordered by the further keys. Values are multiples of 1/4 minus
+    1/2, so that the integral image is exact and the repeats are equal."""
+    rng = np.random.default_rng(9)
+    cell = rng.integers(0, 4, size=(24, 32)).astype(np.float32) * 0.25
+    img = np.tile(cell, (8, 8))
+    s = SURF(img.shape[1], img.shape[0], max_features=300, hessianThreshold=0.01)
+    try:
+        kps, desc = s.detectAndCompute(img, slot=0)
+        rk, rd, found = R.detect(img, max_features=300, threshold=0.01)
+        assert found > 300 and len(np.unique(rk["response"])) < len(rk)
+        for f in kps.dtype.names:
+            assert np.array_equal(kps[f], rk[f]), f
+        assert np.array_equal(desc, rd)
+    finally:
+        s.close()
+
+
 def test_reference_detector_leaves_the_undescribed_tail():
     # 45 keypoints: the reference's SURFInvoker::run describes the first 36
     raw, img = _gray(seed=3)
