@@ -376,27 +376,50 @@ __device__ __forceinline__ bool kp_before(const gls_keypoint& a, int ia, const g
 }
 
 // Rank sort of the candidates and the max_features cut (SURF.cpp:1285,
-// 1413-1418): candidate i goes to its rank if the rank is below keep.
-__global__ void __launch_bounds__(256) k_keypoint_rank(const gls_keypoint* __restrict__ cand,
-                                                       const int* __restrict__ cand_count, int keep,
-                                                       gls_keypoint* __restrict__ out, int* __restrict__ out_count) {
-    __shared__ gls_keypoint tile[256];
+// 1413-1418): candidate i goes to its rank if the rank is below keep. Bound by
+// its n^2 comparisons: a block ranks 16 candidates, 16 threads each over every
+// 16th four others, on the responses alone; a candidate whose response is not
+// its own alone compares the further keys in a second sweep. 7000 candidates:
+// 21 us, 278 with a thread a candidate (28 blocks) and the full comparison.
+constexpr int kRankPer = 16, kRankLanes = 16;
+__global__ void __launch_bounds__(kRankPer * kRankLanes)
+    k_keypoint_rank(const gls_keypoint* __restrict__ cand, const int* __restrict__ cand_count, int keep,
+                    gls_keypoint* __restrict__ out, int* __restrict__ out_count) {
+    constexpr int N = 4 * kRankPer * kRankLanes;
+    __shared__ float4 tile[N / 4];
     const int n = min(*cand_count, kMaxKeypoints);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.x * blockDim.x >= n) return;  // whole block past the end (block-uniform)
+    if (blockIdx.x == 0 && threadIdx.x == 0) *out_count = min(n, keep);
+    if (blockIdx.x * kRankPer >= n) return;  // whole block past the end (block-uniform)
+    const int i = blockIdx.x * kRankPer + threadIdx.x / kRankLanes, lane = threadIdx.x % kRankLanes;
     gls_keypoint me{};
     if (i < n) me = cand[i];
-    int rank = 0;
-    for (int j0 = 0; j0 < n; j0 += 256) {
+    const float key = me.response;
+    int rank = 0, equal = 0;
+    for (int j0 = 0; j0 < n; j0 += N) {
         __syncthreads();
-        if (j0 + threadIdx.x < n) tile[threadIdx.x] = cand[j0 + threadIdx.x];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {  // past the end: behind every candidate
+            const int j = threadIdx.x + k * (N / 4);
+            reinterpret_cast<float*>(tile)[j] = j0 + j < n ? cand[j0 + j].response : -INFINITY;
+        }
         __syncthreads();
-        const int m = min(256, n - j0);
-        if (i < n)
-            for (int j = 0; j < m; j++) rank += kp_before(tile[j], j0 + j, me, i) ? 1 : 0;
+#pragma unroll 8
+        for (int j = lane; j < N / 4; j += kRankLanes) {
+            const float4 r = tile[j];
+            rank += (r.x > key) + (r.y > key) + (r.z > key) + (r.w > key);
+            equal += (r.x == key) + (r.y == key) + (r.z == key) + (r.w == key);
+        }
     }
-    if (i < n && rank < keep) out[rank] = me;
-    if (i == 0) *out_count = min(n, keep);
+#pragma unroll
+    for (int o = kRankLanes / 2; o > 0; o >>= 1) equal += __shfl_xor_sync(0xffffffffu, equal, o);
+    if (i < n && equal > 1)  // not only itself: the further keys decide
+        for (int j = lane; j < n; j += kRankLanes) {
+            const gls_keypoint c = cand[j];
+            if (c.response == key && kp_before(c, j, me, i)) rank++;
+        }
+#pragma unroll
+    for (int o = kRankLanes / 2; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+    if (lane == 0 && i < n && rank < keep) out[rank] = me;
 }
 
 // ------------------------------------------------------------ descriptors
@@ -1840,7 +1863,7 @@ gls_status gls_surf_detect_and_compute(gls_surf* s, const gls_image_view* img, i
     GLS_TRY(launch_check(s, "k_hessian_nms"));
     SurfSlotState& sl = s->slot[slot];
     const int keep = s->capacity;
-    k_keypoint_rank<<<(kMaxKeypoints + 255) / 256, 256, 0, st>>>(
+    k_keypoint_rank<<<(kMaxKeypoints + kRankPer - 1) / kRankPer, kRankPer * kRankLanes, 0, st>>>(
         reinterpret_cast<const gls_keypoint*>(s->cand.p), reinterpret_cast<const int*>(s->cand_count.p), keep,
         reinterpret_cast<gls_keypoint*>(sl.kps.p), reinterpret_cast<int*>(sl.count.p));
     GLS_TRY(launch_check(s, "k_keypoint_rank"));
