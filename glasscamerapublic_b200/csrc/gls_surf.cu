@@ -1397,94 +1397,101 @@ __global__ void k_raw_channels(ChanArgs a) {
 
 // ------------------------------------------------------------ integral
 constexpr int IT = 32;  // integral tile edge
+constexpr int IM = 8;   // warps that move a tile's values
+constexpr int ID = 8;   // tiles loaded ahead
+
+// A strip of 32 running sums, tile by tile: one warp adds down the tile's 32
+// rows (a lane a sum, sequential in float) while the others write the tile
+// before it, put the next one into shared memory and load the one after the
+// next two: one barrier a tile, three tile buffers. Bound by the serial
+// additions and the scan warp's way through shared memory; only W / 32 or H / 32
+// blocks have work. 2016x1512: columns 33 us, rows 40 (38 and 48 with three
+// barriers a tile, the scan between them).
+// load(tile, k): value of row k of the tile for this lane; out(tile, k, buffer).
+template <class Load, class Out>
+__device__ __forceinline__ void running_sums(int tiles, float sub, Load load, Out out) {
+    __shared__ float buf[3][IT][IT + 1];
+    const int lane = threadIdx.x, w = threadIdx.y;
+    float acc = 0.0f, next[ID][IT / IM];
+    auto fetch = [&](int t, float (&v)[IT / IM]) {
+#pragma unroll
+        for (int k = 0; k < IT / IM; k++) v[k] = load(t, w + IM * k);
+    };
+    auto put = [&](int t, const float (&v)[IT / IM]) {
+#pragma unroll
+        for (int k = 0; k < IT / IM; k++) buf[t % 3][w + IM * k][lane] = v[k];
+    };
+    auto flush = [&](int t) {
+#pragma unroll
+        for (int k = 0; k < IT / IM; k++) out(t, w + IM * k, buf[t % 3]);
+    };
+    if (w < IM) {
+#pragma unroll
+        for (int t = 0; t < ID; t++) fetch(t, next[t]);
+        put(0, next[0]);
+        fetch(ID, next[0]);
+    }
+    __syncthreads();
+    auto step = [&](int t, float (&v)[IT / IM]) {  // v: tile t + 1
+        if (w == IM) {
+            float(&b)[IT][IT + 1] = buf[t % 3];
+            float c[IT];
+#pragma unroll
+            for (int k = 0; k < IT; k++) c[k] = b[k][lane];
+#pragma unroll
+            for (int k = 0; k < IT; k++) c[k] = acc = fadd(acc, fsub(c[k], sub));
+#pragma unroll
+            for (int k = 0; k < IT; k++) b[k][lane] = c[k];
+        } else {
+            if (t > 0) flush(t - 1);
+            put(t + 1, v);
+            fetch(t + 1 + ID, v);
+        }
+        __syncthreads();
+    };
+    for (int t = 0; t < tiles; t += ID)
+#pragma unroll
+        for (int k = 0; k < ID; k++)
+            if (t + k < tiles) step(t + k, next[(k + 1) % ID]);
+    if (w < IM) flush(tiles - 1);
+}
 
 // Column pass (integral_sum_cols_image, SURF.metal:315-338): a running sum
-// of (v - 0.5) down each column, sequential in float; written transposed
-// (T[x][y]) through a shared-memory tile. The next tile is loaded into
-// registers while one warp scans the current one.
-__global__ void __launch_bounds__(256) k_integral_cols(const float* __restrict__ img, int pitch, int W, int H,
-                                                       float* __restrict__ T, int tpitch) {
-    __shared__ float tile[IT][IT + 1];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * IT;
-    float nxt[IT / 8];
-    auto load = [&](int y0) {
-#pragma unroll
-        for (int k = 0; k < IT / 8; k++) {
-            const int r = ty + 8 * k, x = x0 + tx, y = y0 + r;
-            nxt[k] = (x < W && y < H) ? __ldg(img + size_t(y) * pitch + x) : 0.0f;
-        }
-    };
-    load(0);
-    float acc = 0.0f;
-    for (int y0 = 0; y0 < H; y0 += IT) {
-#pragma unroll
-        for (int k = 0; k < IT / 8; k++) tile[ty + 8 * k][tx] = nxt[k];
-        __syncthreads();
-        if (y0 + IT < H) load(y0 + IT);
-        if (ty == 0) {
-            const int rows = min(IT, H - y0);
-#pragma unroll 8
-            for (int r = 0; r < rows; r++) {
-                acc = fadd(acc, fsub(tile[r][tx], 0.5f));
-                tile[r][tx] = acc;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < IT / 8; k++) {
-            const int c = ty + 8 * k, x = x0 + c, y = y0 + tx;
-            if (x < W && y < H) T[size_t(x) * tpitch + y] = tile[tx][c];
-        }
-        __syncthreads();
-    }
+// of (v - 0.5) down each column, written transposed (T[x][y]).
+__global__ void __launch_bounds__(32 * (IM + 1)) k_integral_cols(const float* __restrict__ img, int pitch, int W, int H,
+                                                                 float* __restrict__ T, int tpitch) {
+    const int x0 = blockIdx.x * IT, lane = threadIdx.x;
+    running_sums(
+        (H + IT - 1) / IT, 0.5f,
+        [&](int t, int r) {
+            const int x = x0 + lane, y = t * IT + r;
+            return x < W && y < H ? __ldg(img + size_t(y) * pitch + x) : 0.0f;
+        },
+        [&](int t, int c, const float (&b)[IT][IT + 1]) {
+            const int x = x0 + c, y = t * IT + lane;
+            if (x < W && y < H) T[size_t(x) * tpitch + y] = b[lane][c];
+        });
 }
 
 // Row pass (integral_sum_rows_image, SURF.metal:340-421): a running sum of
-// the column sums along each row, sequential in float, into the
-// (W+1) x (H+1) sum image with a zero first row and column.
-__global__ void __launch_bounds__(256) k_integral_rows(const float* __restrict__ T, int tpitch, int W, int H,
-                                                       float* __restrict__ S, int spitch) {
-    __shared__ float tile[IT][IT + 1];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int y0 = blockIdx.x * IT;
-    float nxt[IT / 8];
-    auto load = [&](int x0) {
-#pragma unroll
-        for (int k = 0; k < IT / 8; k++) {
-            const int c = ty + 8 * k, x = x0 + c, y = y0 + tx;
-            nxt[k] = (x < W && y < H) ? __ldg(T + size_t(x) * tpitch + y) : 0.0f;
-        }
-    };
+// the column sums along each row into the (W+1) x (H+1) sum image with a zero
+// first row and column.
+__global__ void __launch_bounds__(32 * (IM + 1)) k_integral_rows(const float* __restrict__ T, int tpitch, int W, int H,
+                                                                 float* __restrict__ S, int spitch) {
+    const int y0 = blockIdx.x * IT, lane = threadIdx.x;
     if (blockIdx.x == 0)
-        for (int x = ty * IT + tx; x <= W; x += 8 * IT) S[x] = 0.0f;
-    for (int k = 0; k < IT / 8; k++) {
-        const int y = y0 + ty + 8 * k;
-        if (tx == 0 && y < H) S[size_t(y + 1) * spitch] = 0.0f;
-    }
-    load(0);
-    float acc = 0.0f;
-    for (int x0 = 0; x0 < W; x0 += IT) {
-#pragma unroll
-        for (int k = 0; k < IT / 8; k++) tile[ty + 8 * k][tx] = nxt[k];
-        __syncthreads();
-        if (x0 + IT < W) load(x0 + IT);
-        if (ty == 0) {
-            const int cols = min(IT, W - x0);
-#pragma unroll 8
-            for (int c = 0; c < cols; c++) {
-                acc = fadd(acc, tile[c][tx]);
-                tile[c][tx] = acc;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < IT / 8; k++) {
-            const int r = ty + 8 * k, y = y0 + r, x = x0 + tx;
-            if (x < W && y < H) S[size_t(y + 1) * spitch + x + 1] = tile[tx][r];
-        }
-        __syncthreads();
-    }
+        for (int x = threadIdx.y * IT + lane; x <= W; x += (IM + 1) * IT) S[x] = 0.0f;
+    if (threadIdx.y == 0 && y0 + lane < H) S[size_t(y0 + lane + 1) * spitch] = 0.0f;
+    running_sums(
+        (W + IT - 1) / IT, 0.0f,
+        [&](int t, int c) {
+            const int x = t * IT + c, y = y0 + lane;
+            return x < W && y < H ? __ldg(T + size_t(x) * tpitch + y) : 0.0f;
+        },
+        [&](int t, int r, const float (&b)[IT][IT + 1]) {
+            const int x = t * IT + lane, y = y0 + r;
+            if (x < W && y < H) S[size_t(y + 1) * spitch + x + 1] = b[lane][r];
+        });
 }
 
 // ------------------------------------------------------------ warps
@@ -1830,9 +1837,9 @@ gls_status gls_surf_detect_and_compute(gls_surf* s, const gls_image_view* img, i
     const int tpitch = H;
     float* T = reinterpret_cast<float*>(s->colT.p);
     float* S = reinterpret_cast<float*>(s->sum.p);
-    k_integral_cols<<<(W + IT - 1) / IT, dim3(32, 8), 0, st>>>(src, pitch, W, H, T, tpitch);
+    k_integral_cols<<<(W + IT - 1) / IT, dim3(32, IM + 1), 0, st>>>(src, pitch, W, H, T, tpitch);
     GLS_TRY(launch_check(s, "k_integral_cols"));
-    k_integral_rows<<<(H + IT - 1) / IT, dim3(32, 8), 0, st>>>(T, tpitch, W, H, S, W + 1);
+    k_integral_rows<<<(H + IT - 1) / IT, dim3(32, IM + 1), 0, st>>>(T, tpitch, W, H, S, W + 1);
     GLS_TRY(launch_check(s, "k_integral_rows"));
     // fastHessianDetector (SURF.cpp:1229-1286)
     DetectArgs da{};
