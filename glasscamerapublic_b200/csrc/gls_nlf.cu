@@ -35,8 +35,8 @@ namespace {
 // its largest variance v (raw_converter.cpp:357-362), taken from the first
 // channel on so that a NaN in a later channel never wins. The truncation
 // makes the classes (0, 1e-6], (1e-6, 1e-5], (1e-5, 1e-4], (1e-4, 1e-3],
-// (1e-3, 1e-2] and above; compared in FP64 on an FP32 variance, which lies
-// more than 1e-11 (relative) from every power of ten, the thresholds give
+// (1e-3, 1e-2] and above: an FP32 variance lies more than 1e-11 (relative)
+// from every power of ten, so the thresholds, rounded down to floats, give
 // the logarithm's classes exactly. -1: no class (a NaN; for the YCbCr fit
 // also a non-positive variance; a NaN largest value, which the reference
 // turns into an undefined histogram index).
@@ -50,127 +50,175 @@ __device__ __forceinline__ int variance_class(const float (&v)[N], bool raw) {
 #pragma unroll
     for (int c = 1; c < N; c++)
         if (v[c] > m) m = v[c];
-    const double d = double(m);
-    return d <= 1e-6 ? 0 : d <= 1e-5 ? 1 : d <= 1e-4 ? 2 : d <= 1e-3 ? 3 : d <= 1e-2 ? 4 : 5;
+    // the largest floats below the powers of ten
+    constexpr float t6 = 0x1.0c6f7a0000000p-20f, t5 = 0x1.4f8b580000000p-17f, t4 = 0x1.a36e2e0000000p-14f;
+    constexpr float t3 = 0x1.0624dc0000000p-10f, t2 = 0x1.47ae140000000p-7f;
+    return m <= t6 ? 0 : m <= t5 ? 1 : m <= t4 ? 2 : m <= t3 ? 3 : m <= t2 ? 4 : 5;
 }
 
-constexpr int RS_TX = 32, RS_TY = 8;                     // half-resolution positions per block
-constexpr int RS_W = 2 * RS_TX + 10, RS_H = 2 * RS_TY + 10;  // full-resolution tile: 2x + [-4, 5]
+// a value and its square, added to a sum and a sum of squares at once (packed
+// FP32: each lane rounds as the scalar operation)
+typedef unsigned long long u64;
+__device__ __forceinline__ float2 with_square(float t) { return make_float2(t, __fmul_rn(t, t)); }
+__device__ __forceinline__ void add_to(u64& s, u64 t) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s) : "l"(t)); }
+__device__ __forceinline__ float2 sums_of(u64 s) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(s));
+    return v;
+}
 
-// the block's class counts: a ballot per class in each warp, one shared
-// atomic per warp and class
-__device__ __forceinline__ void count_class(unsigned* cls, int k) {
-    const unsigned lane = threadIdx.x & 31;
-#pragma unroll
-    for (int j = 0; j < 6; j++) {
-        const unsigned b = __ballot_sync(0xffffffffu, k == j);
-        if (lane == 0 && b) atomicAdd(&cls[j], unsigned(__popc(b)));
+constexpr int RS_TX = 32, RS_TY = 8, RS_P = 2, RS_ROWS = RS_TY * RS_P;  // half-resolution positions per block
+constexpr int RS_W = 2 * RS_TX + 10, RS_H = 2 * RS_ROWS + 10;             // full-resolution tile: 2x + [-4, 5]
+
+// the block's class counts: 8 bits a class in two words, summed over the warp
+// (at most 4 positions a lane), one shared atomic per warp and class
+struct ClassCount {
+    unsigned lo = 0, hi = 0;
+    __device__ __forceinline__ void add(int k) {
+        if (k >= 0) (k < 4 ? lo : hi) += 1u << (8 * (k & 3));
     }
+    __device__ __forceinline__ void flush(unsigned* cls) const {
+        const unsigned lane = threadIdx.x & 31;
+        // 32 lanes' counts of 4: up to 128
+        const unsigned a = __reduce_add_sync(0xffffffffu, lo), b = __reduce_add_sync(0xffffffffu, hi);
+        const unsigned n = (lane < 4 ? a : b) >> (8 * (lane & 3)) & 255u;
+        if (lane < 6 && n) atomicAdd(&cls[lane], n);
+    }
+};
+
+// x / D, correctly rounded, in two operations with the reciprocal as a sum of
+// two floats (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", 2004; all 2^23
+// significands checked for 25 and 81); outside the exponents where the products
+// neither overflow nor lose bits, the division itself.
+template <int D>
+__device__ __forceinline__ float div_const(float x) {
+    constexpr float zh = 1.f / float(D), zl = float(1.0 / double(D) - double(zh));
+    const float a = fabsf(x);
+    if ((a >= 0x1p-90f && a <= 0x1p100f) || a == 0.f) return __fmaf_rn(x, zh, __fmul_rn(x, zl));
+    return __fdiv_rn(x, float(D));
 }
 
 // PATTERN: the Bayer pattern, so every channel's tap set is known at
-// compile time
+// compile time. Bound by the FMA pipe: 648 additions a position whose order is
+// fixed, in 324 packed instructions; values are staged with their squares, and
+// two vertically adjacent positions share 8 of their 10 rows. 2016x1512
+// positions: 119 us (132 with scalar additions, a position a thread).
 template <class S, int PATTERN>
 __global__ void __launch_bounds__(RS_TX* RS_TY) k_raw_stats(Plane<S, 1> raw, Plane<float, 4> mean,
                                                             Plane<float, 4> var, unsigned* __restrict__ hist) {
     constexpr int OX[4][4] = {{1, 0, 0, 1}, {0, 0, 1, 1}, {0, 0, 1, 1}, {1, 0, 0, 1}};
     constexpr int OY[4][4] = {{0, 0, 1, 1}, {1, 0, 0, 1}, {0, 1, 1, 0}, {1, 1, 0, 0}};
-    __shared__ float tile[RS_H][RS_W];
+    __shared__ __align__(16) float2 tile[RS_H][RS_W];
     __shared__ unsigned cls[6];
-    const int X0 = blockIdx.x * RS_TX, Y0 = blockIdx.y * RS_TY;  // half-resolution origin
+    const int X0 = blockIdx.x * RS_TX, Y0 = blockIdx.y * RS_ROWS;  // half-resolution origin
     const int tid = threadIdx.y * RS_TX + threadIdx.x;
     if (tid < 6) cls[tid] = 0;
-    for (int k = tid; k < RS_W * RS_H; k += RS_TX * RS_TY) {
-        const int ty = k / RS_W, tx = k % RS_W;
-        tile[ty][tx] = to_f(*raw.pxc(2 * X0 - 4 + tx, 2 * Y0 - 4 + ty));
-    }
+    for (int ty = threadIdx.y; ty < RS_H; ty += RS_TY)
+        for (int tx = threadIdx.x; tx < RS_W; tx += RS_TX)
+            tile[ty][tx] = with_square(to_f(*raw.pxc(2 * X0 - 4 + tx, 2 * Y0 - 4 + ty)));
     __syncthreads();
-    const int x = X0 + threadIdx.x, y = Y0 + threadIdx.y;
-    int k = -1;
-    if (x < mean.w && y < mean.h) {
-        float sum[4] = {0.f, 0.f, 0.f, 0.f}, sumSq[4] = {0.f, 0.f, 0.f, 0.f};
-        // the window steps one full-resolution pixel from 2 (x, y) - 4 and
-        // reads each channel at its Bayer offset (readRAWQuad): channel c
-        // reads the 10 x 10 block's 9 x 9 sub-block at its offset. Each
-        // value is loaded once and added to the channels that read it, each
-        // channel still in row-major order of its own taps.
-        const int bx0 = 2 * threadIdx.x, by0 = 2 * threadIdx.y;
+    const int x = X0 + threadIdx.x, y0 = Y0 + RS_P * threadIdx.y;
+    // the window steps one full-resolution pixel from 2 (x, y) - 4 and
+    // reads each channel at its Bayer offset (readRAWQuad): channel c
+    // reads the 10 x 10 block's 9 x 9 sub-block at its offset. Each
+    // value is loaded once and added to the channels that read it, each
+    // channel still in row-major order of its own taps.
+    u64 acc[RS_P][4] = {};
+    const int bx0 = 2 * threadIdx.x, by0 = 2 * RS_P * threadIdx.y;
 #pragma unroll
-        for (int u = 0; u < 10; u++)
+    for (int r = 0; r < 2 * RS_P + 8; r++)
 #pragma unroll
-            for (int v = 0; v < 10; v++) {
-                const float t = tile[by0 + u][bx0 + v];
-                const float t2 = __fmul_rn(t, t);
+        for (int v = 0; v < 10; v += 2) {
+            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&tile[by0 + r][bx0 + v]);
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (u - OY[PATTERN][c] >= 0 && u - OY[PATTERN][c] < 9 && v - OX[PATTERN][c] >= 0 &&
-                        v - OX[PATTERN][c] < 9) {
-                        sum[c] = __fadd_rn(sum[c], t);
-                        sumSq[c] = __fadd_rn(sumSq[c], t2);
+            for (int e = 0; e < 2; e++)
+#pragma unroll
+                for (int p = 0; p < RS_P; p++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        const int j = r - 2 * p - OY[PATTERN][c], i = v + e - OX[PATTERN][c];
+                        if (j >= 0 && j < 9 && i >= 0 && i < 9) add_to(acc[p][c], e ? q.y : q.x);
                     }
-            }
+        }
+    ClassCount count;
+#pragma unroll
+    for (int p = 0; p < RS_P; p++) {
+        const int y = y0 + p;
+        if (x >= mean.w || y >= mean.h) continue;
         f4 m, vv;
         float* mp = &m.x;
         float* vp = &vv.x;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            mp[c] = __fdiv_rn(sum[c], 81.f);
-            vp[c] = __fdiv_rn(__fsub_rn(sumSq[c], __fdiv_rn(__fmul_rn(sum[c], sum[c]), 81.f)), 81.f);
+            const float2 t = sums_of(acc[p][c]);
+            mp[c] = div_const<81>(t.x);
+            vp[c] = div_const<81>(__fsub_rn(t.y, div_const<81>(__fmul_rn(t.x, t.x))));
         }
         st4<float>(mean.px(x, y), m);
         st4<float>(var.px(x, y), vv);
         const float vc[4] = {vv.x, vv.y, vv.z, vv.w};
-        k = variance_class<4>(vc, true);
+        count.add(variance_class<4>(vc, true));
     }
-    count_class(cls, k);
+    count.flush(cls);
     __syncthreads();
     if (tid < 6 && cls[tid]) atomicAdd(&hist[tid], cls[tid]);
 }
 
-constexpr int YS_TX = 32, YS_TY = 8;
-constexpr int YS_W = YS_TX + 4, YS_H = YS_TY + 4;
+// Four vertically adjacent positions a thread: a row's values, staged with their
+// squares, are read once for the up to four windows that take them. Bound by the FMA pipe
+// (150 additions a position whose order is fixed) and 390 MB of traffic.
+// 4032x3024: 143 us (224 with one position a thread).
+constexpr int YS_TX = 32, YS_TY = 8, YS_P = 4, YS_ROWS = YS_TY * YS_P;
+constexpr int YS_W = YS_TX + 4, YS_H = YS_ROWS + 4;
 
 template <class S>
 __global__ void __launch_bounds__(YS_TX* YS_TY) k_ycc_stats(Plane<S, 4> img, Plane<float, 4> stats,
                                                             unsigned* __restrict__ hist) {
-    __shared__ float tile[3][YS_H][YS_W];
+    __shared__ float2 tile[3][YS_H][YS_W];
     __shared__ unsigned cls[6];
-    const int x0 = blockIdx.x * YS_TX, y0 = blockIdx.y * YS_TY;
+    const int x0 = blockIdx.x * YS_TX, y0 = blockIdx.y * YS_ROWS;
     const int tid = threadIdx.y * YS_TX + threadIdx.x;
     if (tid < 6) cls[tid] = 0;
     for (int k = tid; k < YS_W * YS_H; k += YS_TX * YS_TY) {
         const int ty = k / YS_W, tx = k % YS_W;
         const f4 p = ld4<S>(img.pxc(x0 - 2 + tx, y0 - 2 + ty));
-        tile[0][ty][tx] = p.x;
-        tile[1][ty][tx] = p.y;
-        tile[2][ty][tx] = p.z;
+        tile[0][ty][tx] = with_square(p.x);
+        tile[1][ty][tx] = with_square(p.y);
+        tile[2][ty][tx] = with_square(p.z);
     }
     __syncthreads();
-    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
-    int k = -1;
-    if (x < img.w && y < img.h) {
-        float sum[3] = {0.f, 0.f, 0.f}, sumSq[3] = {0.f, 0.f, 0.f};
+    const int x = x0 + threadIdx.x, ty = threadIdx.y * YS_P;
+    u64 acc[YS_P][3] = {};
 #pragma unroll
-        for (int dy = 0; dy < 5; dy++)
+    for (int r = 0; r < YS_P + 4; r++)
 #pragma unroll
-            for (int dx = 0; dx < 5; dx++)
+        for (int dx = 0; dx < 5; dx++)
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    const float t = tile[c][threadIdx.y + dy][threadIdx.x + dx];
-                    sum[c] = __fadd_rn(sum[c], t);
-                    sumSq[c] = __fadd_rn(sumSq[c], __fmul_rn(t, t));
-                }
+            for (int c = 0; c < 3; c++) {
+                const u64 t = *reinterpret_cast<const u64*>(&tile[c][ty + r][threadIdx.x + dx]);
+#pragma unroll
+                for (int p = 0; p < YS_P; p++)
+                    if (r - p >= 0 && r - p < 5) add_to(acc[p][c], t);
+            }
+    ClassCount count;
+#pragma unroll
+    for (int p = 0; p < YS_P; p++) {
+        const int y = y0 + ty + p;
+        if (x >= img.w || y >= img.h) continue;
         f4 o;
-        o.x = __fdiv_rn(sum[0], 25.f);
         float* op = &o.y;
 #pragma unroll
-        for (int c = 0; c < 3; c++)
-            op[c] = __fdiv_rn(__fsub_rn(sumSq[c], __fdiv_rn(__fmul_rn(sum[c], sum[c]), 25.f)), 25.f);
+        for (int c = 0; c < 3; c++) {
+            const float2 t = sums_of(acc[p][c]);
+            if (c == 0) o.x = div_const<25>(t.x);
+            op[c] = div_const<25>(__fsub_rn(t.y, div_const<25>(__fmul_rn(t.x, t.x))));
+        }
         st4<float>(stats.px(x, y), o);
         const float vc[3] = {o.y, o.z, o.w};
-        k = variance_class<3>(vc, false);
+        count.add(variance_class<3>(vc, false));
     }
-    count_class(cls, k);
+    count.flush(cls);
     __syncthreads();
     if (tid < 6 && cls[tid]) atomicAdd(&hist[tid], cls[tid]);
 }
@@ -191,38 +239,37 @@ struct FitInput {
 
 constexpr int FIT_BLOCKS = 296, FIT_THREADS = 256, FIT_K = 24;
 
+// one position's regressors and variances (ycc: one regressor, three variances)
+template <bool RAW>
 struct Sample {
-    double m[4], v[4];
+    static constexpr int NM = RAW ? 4 : 1, NV = RAW ? 4 : 3;
+    float m[NM], v[NV];
 };
 
-__device__ __forceinline__ Sample load_sample(const FitInput& in, long i) {
-    const int x = int(i % in.w), y = int(i / in.w);
-    Sample s;
-    if (in.raw) {
-        const float4 m = in.mean[size_t(y) * in.pitch + x], v = in.var[size_t(y) * in.pitch + x];
-        s.m[0] = m.x, s.m[1] = m.y, s.m[2] = m.z, s.m[3] = m.w;
-        s.v[0] = v.x, s.v[1] = v.y, s.v[2] = v.z, s.v[3] = v.w;
+template <bool RAW>
+__device__ __forceinline__ Sample<RAW> load_sample(const FitInput& in, int x, int y) {
+    const size_t i = size_t(y) * in.pitch + x;
+    if constexpr (RAW) {
+        const float4 m = __ldg(in.mean + i), v = __ldg(in.var + i);
+        return {{m.x, m.y, m.z, m.w}, {v.x, v.y, v.z, v.w}};
     } else {
-        const float4 t = in.mean[size_t(y) * in.pitch + x];
-        s.m[0] = s.m[1] = s.m[2] = s.m[3] = t.x;
-        s.v[0] = t.y, s.v[1] = t.z, s.v[2] = t.w, s.v[3] = 0.0;
+        const float4 t = __ldg(in.mean + i);
+        return {{t.x}, {t.y, t.z, t.w}};
     }
-    return s;
 }
 
 __device__ __forceinline__ int nch(const FitInput& in) { return in.raw ? 4 : 3; }
 
 // a position counts in the fits: no NaN, every mean in [0.001, 0.9] and
-// every variance within the bound
-__device__ __forceinline__ bool usable(const FitInput& in, const Sample& s, const double* bound) {
-    const int n = nch(in);
+// every variance within the bound (rounded down: the same on FP32 variances;
+// likewise 0.001f is the least float above 0.001 and 0.9f the largest below 0.9)
+template <bool RAW>
+__device__ __forceinline__ bool usable(const Sample<RAW>& s, const float (&bound)[4]) {
     bool ok = true;
 #pragma unroll
-    for (int c = 0; c < 4; c++)
-        if (c < n) ok = ok && !isnan(s.m[c]) && !isnan(s.v[c]);
+    for (int c = 0; c < s.NM; c++) ok = ok && s.m[c] >= 0.001f && s.m[c] <= 0.9f;
 #pragma unroll
-    for (int c = 0; c < 4; c++)
-        if (c < n) ok = ok && s.m[c] >= 0.001 && s.m[c] <= 0.9 && s.v[c] <= bound[c];
+    for (int c = 0; c < s.NV; c++) ok = ok && s.v[c] <= bound[c];
     return ok;
 }
 
@@ -237,63 +284,84 @@ __device__ __forceinline__ double max_s(double v, double s) { return v > s ? v :
 
 // pass: 1 the first fit's sums; 2 its squared residuals; 3 the second fit's
 // sums and squared residuals (the class histogram, pass 0, comes with the
-// statistics)
-template <int PASS>
-__global__ void __launch_bounds__(FIT_THREADS) k_fit_pass(FitInput in, const FitState* __restrict__ st_,
+// statistics). Bound by reading the statistics, 97 MB (raw) or 195 MB (YCbCr)
+// at 4032x3024 with few warps in flight: four or eight positions a thread are
+// loaded before they are summed. Passes 1, 2, 3 of both fits at that size: 64,
+// 63, 73 us (180, 164, 149 with one position at a time, a 64-bit division for each and
+// the tests in FP64).
+template <int PASS, bool RAW>
+__global__ void __launch_bounds__(FIT_THREADS, 2) k_fit_pass(FitInput in, const FitState* __restrict__ st_,
                                                           double* __restrict__ partial) {
-    constexpr int NK = PASS == 1 ? 17 : PASS == 2 ? 4 : 21;
+    constexpr int NK = PASS == 1 ? 17 : PASS == 2 ? 4 : 21, AHEAD = RAW ? 4 : 8;
+    using Smp = Sample<RAW>;
     __shared__ double red[FIT_THREADS / 32][NK];
     double acc[NK];
 #pragma unroll
     for (int k = 0; k < NK; k++) acc[k] = 0.0;
     const FitState st = *st_;
-    const int n = nch(in);
-    const long total = long(in.w) * in.h;
-    for (long i = long(blockIdx.x) * FIT_THREADS + threadIdx.x; i < total; i += long(FIT_BLOCKS) * FIT_THREADS) {
-        const Sample s = load_sample(in, i);
-        if (!usable(in, s, st.bound)) continue;
-        if (PASS == 1) {
+    float bound[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (c < n) {
-                    acc[c] += s.m[c];
-                    acc[4 + c] += s.v[c];
-                    acc[8 + c] += s.m[c] * s.m[c];
-                    acc[12 + c] += s.m[c] * s.v[c];
-                }
-            acc[16] += 1.0;
-        } else if (PASS == 2) {
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (c < n) {
-                    const double d = (st.A[c] + st.B[c] * s.m[c]) - s.v[c];
-                    acc[c] += d * d;
-                }
-        } else {
-            double d2[4];
+    for (int c = 0; c < 4; c++) bound[c] = __double2float_rd(st.bound[c]);
+    unsigned count = 0;
+    auto add = [&](const Smp& s) {
+        if (!usable<RAW>(s, bound)) return;
+        if (PASS > 1) {
+            double d2[4] = {0.0, 0.0, 0.0, 0.0};
             bool fits = true;
-            const double f = in.raw ? 0.5 : 1.0;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                d2[c] = 0.0;
-                if (c < n) {
-                    const double d = fabs((st.A[c] + st.B[c] * s.m[c]) - s.v[c]);
-                    d2[c] = d * d;
-                    fits = fits && d2[c] <= f * st.err2[c];
-                }
+            for (int c = 0; c < Smp::NV; c++) {
+                const double d = (st.A[c] + st.B[c] * double(s.m[RAW ? c : 0])) - double(s.v[c]);
+                d2[c] = d * d;
+                fits = fits && (PASS == 2 || d2[c] <= (RAW ? 0.5 : 1.0) * st.err2[c]);
             }
-            if (fits) {
+            if (!fits) return;
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (c < n) {
-                        acc[c] += s.m[c];
-                        acc[4 + c] += s.v[c];
-                        acc[8 + c] += s.m[c] * s.m[c];
-                        acc[12 + c] += s.m[c] * s.v[c];
-                        acc[17 + (c & 3)] += d2[c];
-                    }
-                acc[16] += 1.0;
+            for (int c = 0; c < Smp::NV; c++) acc[(PASS == 2 ? 0 : 17) + c] += d2[c];
+        }
+        if (PASS != 2) {
+#pragma unroll
+            for (int c = 0; c < Smp::NM; c++) {
+                const double m = s.m[c];
+                acc[c] += m;
+                acc[8 + c] += m * m;
             }
+#pragma unroll
+            for (int c = 0; c < Smp::NV; c++) {
+                const double v = s.v[c];
+                acc[4 + c] += v;
+                acc[12 + c] += double(s.m[RAW ? c : 0]) * v;
+            }
+            count++;
+        }
+    };
+    constexpr unsigned stride = FIT_BLOCKS * FIT_THREADS;
+    const unsigned first = blockIdx.x * FIT_THREADS + threadIdx.x;
+    const int step_x = int(stride % unsigned(in.w)), step_y = int(stride / unsigned(in.w));
+    int x = int(first % unsigned(in.w)), y = int(first / unsigned(in.w));
+    while (y < in.h) {
+        Smp s[AHEAD];
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) {
+            if (y >= in.h) break;
+            s[k] = load_sample<RAW>(in, x, y);
+            n = k + 1;
+            x += step_x;
+            y += step_y;
+            if (x >= in.w) {
+                x -= in.w;
+                y++;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++)
+            if (k < n) add(s[k]);
+    }
+    if constexpr (PASS != 2) {
+        acc[16] = double(count);
+        if constexpr (!RAW) {  // the three channels' regressor is one
+            acc[1] = acc[2] = acc[0];
+            acc[9] = acc[10] = acc[8];
         }
     }
     // block sums in a fixed order: a shuffle tree per warp, then the warps
@@ -407,13 +475,14 @@ FitScratch fit_scratch(void* scratch) {
     return f;
 }
 
+template <bool RAW>
 void launch_fit(const FitInput& in, const FitScratch& f, gls_raw_nlf* out, cudaStream_t s) {
     k_fit_finish<0><<<1, FIT_K * 32, 0, s>>>(in, f.partial, f.hist, f.st, out);
-    k_fit_pass<1><<<FIT_BLOCKS, FIT_THREADS, 0, s>>>(in, f.st, f.partial);
+    k_fit_pass<1, RAW><<<FIT_BLOCKS, FIT_THREADS, 0, s>>>(in, f.st, f.partial);
     k_fit_finish<1><<<1, FIT_K * 32, 0, s>>>(in, f.partial, f.hist, f.st, out);
-    k_fit_pass<2><<<FIT_BLOCKS, FIT_THREADS, 0, s>>>(in, f.st, f.partial);
+    k_fit_pass<2, RAW><<<FIT_BLOCKS, FIT_THREADS, 0, s>>>(in, f.st, f.partial);
     k_fit_finish<2><<<1, FIT_K * 32, 0, s>>>(in, f.partial, f.hist, f.st, out);
-    k_fit_pass<3><<<FIT_BLOCKS, FIT_THREADS, 0, s>>>(in, f.st, f.partial);
+    k_fit_pass<3, RAW><<<FIT_BLOCKS, FIT_THREADS, 0, s>>>(in, f.st, f.partial);
     k_fit_finish<3><<<1, FIT_K * 32, 0, s>>>(in, f.partial, f.hist, f.st, out);
 }
 
@@ -429,7 +498,7 @@ template <class S>
 int launch_measure_raw_nlf(Plane<S, 1> scaled, int pattern, Plane<float, 4> mean, Plane<float, 4> var,
                            float exposure, void* scratch, gls_raw_nlf* out, cudaStream_t s) {
     const FitScratch f = fit_scratch(scratch);
-    const dim3 g((mean.w + RS_TX - 1) / RS_TX, (mean.h + RS_TY - 1) / RS_TY);
+    const dim3 g((mean.w + RS_TX - 1) / RS_TX, (mean.h + RS_ROWS - 1) / RS_ROWS);
     const dim3 b(RS_TX, RS_TY);
     switch (pattern) {
         case 0: k_raw_stats<S, 0><<<g, b, 0, s>>>(scaled, mean, var, f.hist); break;
@@ -439,7 +508,7 @@ int launch_measure_raw_nlf(Plane<S, 1> scaled, int pattern, Plane<float, 4> mean
     }
     FitInput in{reinterpret_cast<const float4*>(mean.p), reinterpret_cast<const float4*>(var.p), mean.w, mean.h,
                 mean.pitch / 4, 1, double(scaled.w) * double(scaled.h), exposure};
-    launch_fit(in, f, out, s);
+    launch_fit<true>(in, f, out, s);
     return 8;
 }
 
@@ -447,11 +516,11 @@ template <class S>
 int launch_measure_ycc_nlf(Plane<S, 4> img, Plane<float, 4> stats, float exposure, void* scratch,
                            gls_raw_nlf* out, cudaStream_t s) {
     const FitScratch f = fit_scratch(scratch);
-    const dim3 g((img.w + YS_TX - 1) / YS_TX, (img.h + YS_TY - 1) / YS_TY);
+    const dim3 g((img.w + YS_TX - 1) / YS_TX, (img.h + YS_ROWS - 1) / YS_ROWS);
     k_ycc_stats<S><<<g, dim3(YS_TX, YS_TY), 0, s>>>(img, stats, f.hist);
     FitInput in{reinterpret_cast<const float4*>(stats.p), nullptr, stats.w, stats.h, stats.pitch / 4, 0,
                 double(img.w) * double(img.h), exposure};
-    launch_fit(in, f, out, s);
+    launch_fit<false>(in, f, out, s);
     return 8;
 }
 

@@ -79,6 +79,26 @@ def test_ycbcr_statistics_and_fit(converter, chart, half):
         lvl = O.downsample(lvl, lvl.shape[1] // 2, lvl.shape[0] // 2, f64=False)
 
 
+@pytest.mark.parametrize("w,h", [(16, 12), (64, 32), (66, 34), (126, 70)])
+@pytest.mark.parametrize("scale", [0.0, 1.0, 1e-12, 3e-29, 1e18, 3e19])
+def test_statistics_at_tile_edges_and_extreme_scales(converter, w, h, scale):
+    """Bit-exact whatever the exponent: the quotients by 81 and 25 take their
+    short form between 2^-90 and 2^100 and at 0, the squares of the last scale
+    overflow."""
+    import torch
+    rng = np.random.default_rng(w)
+    with np.errstate(over="ignore", invalid="ignore"):
+        raw = (rng.random((h, w), dtype=np.float32) + np.float32(0.5)) * np.float32(scale)
+        raw[:, : w // 3] = np.float32(scale)  # variances of 0 and of rounding errors
+        converter.MeasureRawNLF(torch.from_numpy(raw).cuda(), 1, 1.0)
+        om, ov = O.raw_noise_stats(raw, 1)
+        assert np.array_equal(_plane(converter, g.PLANE_NLF_MEAN), om, equal_nan=True)
+        assert np.array_equal(_plane(converter, g.PLANE_NLF_VAR), ov, equal_nan=True)
+        ycc = (rng.standard_normal((h, w, 4)).astype(np.float32)) * np.float32(scale)
+        converter.MeasureYCbCrNLF(torch.from_numpy(ycc).cuda(), 1.0)
+        assert np.array_equal(_plane(converter, g.PLANE_NLF_STATS), O.ycc_noise_stats(ycc), equal_nan=True)
+
+
 def test_calibrating_converter_matches_the_oracle():
     conv = g.RawConverter(0, calibrateFromImage=True)
     try:
