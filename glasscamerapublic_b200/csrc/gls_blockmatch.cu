@@ -422,9 +422,10 @@ __device__ __forceinline__ void bm_group(const Sm& sm, int gx, int gy, u64 (&acc
     }
 }
 
-// A warp's share of the tile's groups, the results into shared memory.
+// A warp's share of the tile's groups (of the part `part` of `parts`), the
+// results into shared memory.
 template <bool SAFE, bool CLAMP, int TY, class Sm>
-__device__ __forceinline__ void bm_groups(Sm& sm) {
+__device__ __forceinline__ void bm_groups(Sm& sm, int part, int parts) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     constexpr int GROUPS = (BX_TX / 4) * (Sm::T::ROWS / 2);
     // the column part of the spatial weight: neighbour g of each segment,
@@ -437,7 +438,7 @@ __device__ __forceinline__ void bm_groups(Sm& sm) {
     }
     const bool second = lane & 16;
 #pragma unroll 1
-    for (int grp = warp; grp < GROUPS; grp += TY) {
+    for (int grp = warp + TY * part; grp < GROUPS; grp += TY * parts) {
         const int gx = (grp % (BX_TX / 4)) * 4, gy = (grp / (BX_TX / 4)) * 2;
         u64 part[3][5];
         bm_group<SAFE, CLAMP>(sm, gx, gy, part);
@@ -468,7 +469,7 @@ __device__ __forceinline__ void bm_groups(Sm& sm) {
 template <int TY, int NP>
 __device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& img, const Plane<__half, 2>& grad,
                                         const float* __restrict__ basis, const Plane<__half, 4>& out,
-                                        const BlockMatchArgs& a, BmTileSmem<TY, NP>& sm) {
+                                        const BlockMatchArgs& a, BmTileSmem<TY, NP>& sm, int part = 0, int parts = 1) {
     using T = BxTile<TY, NP>;
     constexpr int NT = T::THREADS, NPOS = BX_W * T::H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -635,13 +636,15 @@ __device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& 
     // largest |q'|^2: the exponents stay below log2 sqrt(lk) + 1 < 2 unasked
     // unless the tile's kl are extreme
     const bool clamp = !(__uint_as_float(sm.nn_max) * __uint_as_float(sm.kl_max) < 0x1p18f);
-    if (safe) bm_groups<true, true, TY>(sm);
-    else if (clamp) bm_groups<false, true, TY>(sm);
-    else bm_groups<false, false, TY>(sm);
+    if (safe) bm_groups<true, true, TY>(sm, part, parts);
+    else if (clamp) bm_groups<false, true, TY>(sm, part, parts);
+    else bm_groups<false, false, TY>(sm, part, parts);
     __syncthreads();
     for (int i = tid; i < T::ROWS * BX_TX; i += NT) {
         const int x = x0 + i % BX_TX, y = y0 + i / BX_TX;
         if (x >= out.w || y >= out.h) continue;
+        // the group's round: another part's pixels still hold their constants
+        if ((i / (2 * BX_TX) * (BX_TX / 4) + i % BX_TX / 4) / TY % parts != part) continue;
         const float ny = sm.k[3][i], nc = sm.k[4][i];
         // sums that vanish: at scales where the distance's rounding alone
         // exceeds the exponent's range even the pixel's own weight is lost
@@ -658,15 +661,21 @@ __global__ void __launch_bounds__(BxTile<TY, NP>::THREADS, BxTile<TY, NP>::MIN_B
                        Plane<__half, 4> out, BlockMatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bm_tile<TY, NP>(blockIdx.x * BX_TX, blockIdx.y * (NP * TY), img, grad, basis, out, a,
-                    *reinterpret_cast<BmTileSmem<TY, NP>*>(smem_raw));
+                    *reinterpret_cast<BmTileSmem<TY, NP>*>(smem_raw), blockIdx.z, gridDim.z);
 }
 
 template <int TY, int NP>
 static void launch_pair(Plane<__half, 4> img, Plane<__half, 2> grad, const float* basis, Plane<__half, 4> out,
-                        const BlockMatchArgs& a, cudaStream_t s) {
+                        const BlockMatchArgs& a, cudaStream_t s, bool split = false) {
     const size_t smem = sizeof(BmTileSmem<TY, NP>);
     ensure_dynamic_smem(reinterpret_cast<const void*>(k_block_match_pair<TY, NP>), int(smem));
     dim3 g((img.w + BX_TX - 1) / BX_TX, (img.h + NP * TY - 1) / (NP * TY));
+    // A level too small for the 296 blocks that fit the chip: each tile's groups
+    // are dealt to up to 8 blocks, which stage it alike. 126x94 (24 tiles) 20 us,
+    // 43 with a block a tile; 252x189 (96) 42 and 44; taken further, to twice
+    // the blocks that fit, 252x189 takes 52.
+    if (split)
+        while (g.z < 8 && g.x * g.y * g.z * 2 <= 296) g.z *= 2;
     k_block_match_pair<TY, NP><<<g, BxTile<TY, NP>::THREADS, smem, s>>>(img, grad, basis, out, a);
 }
 
@@ -677,7 +686,7 @@ static void launch_pair_variant(int code, Plane<__half, 4> img, Plane<__half, 2>
                                 Plane<__half, 4> out, const BlockMatchArgs& a, cudaStream_t s) {
     switch (code) {
         case 44: launch_pair<4, 4>(img, grad, basis, out, a, s); break;
-        case 82: launch_pair<8, 2>(img, grad, basis, out, a, s); break;
+        case 82: launch_pair<8, 2>(img, grad, basis, out, a, s, true); break;
         case 162: launch_pair<16, 2>(img, grad, basis, out, a, s); break;
         default: launch_pair<8, 4>(img, grad, basis, out, a, s); break;
     }
