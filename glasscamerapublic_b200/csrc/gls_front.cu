@@ -166,152 +166,228 @@ __global__ void __launch_bounds__(256) k_sobel_blur(Plane<S, 1> raw, Plane<S, 2>
     }
 }
 
-// The FP16-storage path's form of the same stencil. The wide blur's 25
-// bilinear taps sit on a 5 x 5 grid whose x offsets depend on the column
+// The FP16-storage path's form of the same stencil. Each blur's bilinear taps
+// sit on a grid (2 x 2 narrow, 5 x 5 wide) whose x offsets depend on the column
 // only and y offsets on the row only, and whose weights are the Gaussian's
-// 2 x 2 block sums, a product of a row and a column factor: the blur is
-// separable. It runs as a horizontal pass (5 taps, two texels each) into
-// shared memory and a vertical pass over it, a third of the operations of
-// the 25 bilinear taps. The one tap off the grid is the corner, which the
-// folding puts at (width/2, width/2) = (4.5, 4.5) (demosaic_utils.cpp:984)
-// instead of (4, 4): it is moved there by one correction term. The factors
-// come from the tap table (row and column sums of the weights), so the
-// result is the 25-tap blur up to FP32 rounding of the factorisation.
-struct SepSmem {
-    float sraw[SB_RH][SB_RW];
-    float2 ssob[SB_SH][SB_SW];
-    float4 hsum[SB_SH][SB_TW];  // horizontal pass: (gx, gy, |gx|, |gy|) per sobel-tile row, output column
-    float u[5], v[5];
-    int ix[5], iy[5];
-    float fx[5], fy[5];
-    float total, wc, cdx, cdy;  // corner tap: weight, offset
+// 2 x 2 block sums, a product of a row and a column factor: as sums over texels
+// the blurs are separable filters of 3 and 9 texels. The one tap off the grid
+// is the corner, which the folding puts at (width/2, width/2) (1.5 and 4.5,
+// demosaic_utils.cpp:984) instead of (1, 1) and (4, 4): it is moved there by
+// one correction term. The factors come from the tap table (row and column
+// sums of the weights), so the result is the bilinear taps' up to FP32
+// rounding of the factorisation.
+//
+// Bound by instruction issue: a thread runs down 7 rows of Sobel values, takes
+// 4 adjacent columns in the horizontal pass and 4 adjacent rows in the vertical
+// one, so that a texel is read once for all of them, and (gx, gy) and their
+// magnitudes are packed FP32 pairs. 4032x3024: 130 us (322 with a position a
+// thread and bilinear reads).
+struct SepBlur {
+    float2 wide_x[9], wide_y[9];      // factors of the texels -4 .. 4, each twice (over the sum of weights in y)
+    float2 narrow_x[3], narrow_y[3];  // of -1 .. 1
+    float2 wide_c, narrow_c;          // the corner taps' weights
+    float var0, var1, inv_sqrt45;
 };
 
-__device__ __forceinline__ float4 bil4(const float2 (*ssob)[SB_SW], int ix, int iy, float ax, float ay) {
-    const float2 p00 = ssob[iy][ix], p01 = ssob[iy][ix + 1];
-    const float2 p10 = ssob[iy + 1][ix], p11 = ssob[iy + 1][ix + 1];
-    auto bil = [&](float v00, float v01, float v10, float v11) {
-        const float top = v00 + (v01 - v00) * ax;
-        const float bot = v10 + (v11 - v10) * ax;
-        return top + (bot - top) * ay;
-    };
-    return make_float4(bil(p00.x, p01.x, p10.x, p11.x), bil(p00.y, p01.y, p10.y, p11.y),
-                       bil(fabsf(p00.x), fabsf(p01.x), fabsf(p10.x), fabsf(p11.x)),
-                       bil(fabsf(p00.y), fabsf(p01.y), fabsf(p10.y), fabsf(p11.y)));
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 sb_fma(u64 a, float2 w, u64 c) {
+    u64 d;
+    asm("{\n\t.reg .b64 w;\n\tmov.b64 w, {%2, %3};\n\tfma.rn.f32x2 %0, %1, w, %4;\n\t}"
+        : "=l"(d) : "l"(a), "f"(w.x), "f"(w.y), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 sb_add(u64 a, u64 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 sb_abs(u64 a) { return a & 0x7fffffff7fffffffull; }
+__device__ __forceinline__ float2 sb_pair(u64 a) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(a));
+    return v;
 }
 
+constexpr int SB_HR = SB_TH + 8, SB_HP = SB_TW + 1;  // rows and pitch of the horizontal sums
+constexpr int SB_COL = 7;                            // Sobel rows a thread runs down
+struct SepSmem {
+    float sraw[SB_RH][SB_RW];
+    u64 ssob[SB_SH][SB_SW];          // (gx, gy)
+    ulonglong2 hsum[SB_HR * SB_HP];  // horizontal sums of (gx, gy) and (|gx|, |gy|)
+};
+
 template <class S>
-__global__ void __launch_bounds__(256) k_sobel_blur_sep(Plane<S, 1> raw, Plane<S, 2> out, BlurArgs a) {
-    __shared__ SepSmem sm;
+__global__ void __launch_bounds__(256, 4) k_sobel_blur_sep(Plane<S, 1> raw, Plane<S, 2> out, const SepBlur a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SepSmem& sm = *reinterpret_cast<SepSmem*>(smem_raw);
     const int x0 = blockIdx.x * SB_TW, y0 = blockIdx.y * SB_TH;
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const int nth = blockDim.x * blockDim.y;
-    if (tid == 0) {  // the wide taps' grid: row / column offsets and weight factors
-        const int b = a.n1;
-        float total = 0.f, rs[5] = {0, 0, 0, 0, 0}, cs[5] = {0, 0, 0, 0, 0};
-        for (int r = 0; r < 5; r++)
-            for (int c = 0; c < 5; c++) {
-                const float w = a.w[b + r * 5 + c];
-                rs[r] += w;
-                cs[c] += w;
-                total += w;
-            }
-        for (int k = 0; k < 5; k++) {
-            sm.u[k] = rs[k] / total;  // u_r v_c = W_rc for a separable table
-            sm.v[k] = cs[k];
-            sm.ix[k] = a.ix[b + k];
-            sm.fx[k] = a.fx[b + k];
-            sm.iy[k] = a.iy[b + k * 5];
-            sm.fy[k] = a.fy[b + k * 5];
-        }
-        sm.total = total;
-        sm.wc = a.w[b + 24];
-        sm.cdx = float(a.ix[b + 24]) + a.fx[b + 24];
-        sm.cdy = float(a.iy[b + 24]) + a.fy[b + 24];
-    }
-    for (int i = tid; i < SB_RW * SB_RH; i += nth) {
-        const int ty = i / SB_RW, tx = i % SB_RW;
-        sm.sraw[ty][tx] = to_f(*raw.pxc(x0 - 5 + tx, y0 - 5 + ty));
+    const int tid = threadIdx.y * SB_TW + threadIdx.x;
+    if (const int tx = tid & 63; tx < SB_RW) {
+        S v[(SB_RH + 3) / 4];  // every load issued before the first store
+        const S* col = raw.px(clampi(x0 - 5 + tx, 0, raw.w - 1), 0);
+#pragma unroll
+        for (int k = 0; k < (SB_RH + 3) / 4; k++)
+            v[k] = col[size_t(clampi(y0 - 5 + (tid >> 6) + 4 * k, 0, raw.h - 1)) * raw.pitch];
+#pragma unroll
+        for (int k = 0; k < (SB_RH + 3) / 4; k++)
+            if ((tid >> 6) + 4 * k < SB_RH) sm.sraw[(tid >> 6) + 4 * k][tx] = to_f(v[k]);
     }
     __syncthreads();
     const float inv = a.inv_sqrt45;
-    for (int i = tid; i < SB_SW * SB_SH; i += nth) {
-        const int ty = i / SB_SW, tx = i % SB_SW;
-        const int qx = clampi(x0 - 4 + tx, 0, raw.w - 1) - (x0 - 5);
-        const int qy = clampi(y0 - 4 + ty, 0, raw.h - 1) - (y0 - 5);
-        const float tl = sm.sraw[qy - 1][qx - 1], tc = sm.sraw[qy - 1][qx], tr = sm.sraw[qy - 1][qx + 1];
-        const float ml = sm.sraw[qy][qx - 1], mr = sm.sraw[qy][qx + 1];
-        const float bl = sm.sraw[qy + 1][qx - 1], bc = sm.sraw[qy + 1][qx], br = sm.sraw[qy + 1][qx + 1];
-        const float gx = ((tl - tr) + 2.f * (ml - mr) + (bl - br)) * inv;
-        const float gy = ((tl - bl) + 2.f * (tc - bc) + (tr - br)) * inv;
-        sm.ssob[ty][tx] = make_float2(gx, gy);
+    if (x0 >= 4 && y0 >= 4 && x0 + SB_SW - 4 <= raw.w && y0 + SB_SH - 4 <= raw.h) {
+        static_assert(SB_SW * ((SB_SH + SB_COL - 1) / SB_COL) <= 256, "a column of Sobel rows for each thread");
+        const int tx = tid % SB_SW, t0 = tid / SB_SW * SB_COL;
+        float l = 0.f, c = 0.f, r = 0.f, d0 = 0.f, d1 = 0.f, s0 = 0.f, s1 = 0.f;
+        if (t0 < SB_SH)
+#pragma unroll
+            for (int k = 0; k < SB_COL + 2; k++) {
+                if (t0 + k >= SB_RH) break;
+                l = sm.sraw[t0 + k][tx], c = sm.sraw[t0 + k][tx + 1], r = sm.sraw[t0 + k][tx + 2];
+                const float d2 = l - r, s2 = fmaf(2.f, c, l + r);
+                if (k >= 2 && t0 + k - 2 < SB_SH) {
+                    const float2 g = make_float2((fmaf(2.f, d1, d0) + d2) * inv, (s0 - s2) * inv);
+                    sm.ssob[t0 + k - 2][tx] = *reinterpret_cast<const u64*>(&g);
+                }
+                d0 = d1, d1 = d2, s0 = s1, s1 = s2;
+            }
+    } else {
+        for (int i = tid; i < SB_SW * SB_SH; i += 256) {
+            const int ty = i / SB_SW, tx = i % SB_SW;
+            // Sobel at the clamped position of this tile entry
+            const int qx = clampi(x0 - 4 + tx, 0, raw.w - 1) - (x0 - 5);
+            const int qy = clampi(y0 - 4 + ty, 0, raw.h - 1) - (y0 - 5);
+            const float tl = sm.sraw[qy - 1][qx - 1], tc = sm.sraw[qy - 1][qx], tr = sm.sraw[qy - 1][qx + 1];
+            const float ml = sm.sraw[qy][qx - 1], mr = sm.sraw[qy][qx + 1];
+            const float bl = sm.sraw[qy + 1][qx - 1], bc = sm.sraw[qy + 1][qx], br = sm.sraw[qy + 1][qx + 1];
+            const float2 g = make_float2(((tl - tr) + 2.f * (ml - mr) + (bl - br)) * inv,
+                                         ((tl - bl) + 2.f * (tc - bc) + (tr - br)) * inv);
+            sm.ssob[ty][tx] = *reinterpret_cast<const u64*>(&g);
+        }
     }
     __syncthreads();
-    // horizontal pass: every sobel-tile row, every output column
-    for (int i = tid; i < SB_SH * SB_TW; i += nth) {
-        const int ry = i / SB_TW, cx = i % SB_TW;
-        float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+    // horizontal pass: rows -4 .. 35, four columns a thread; a warp's lanes run
+    // down the rows, whose pitches (41 pairs, 33 quads) spread over the banks
+    for (int i = tid; i < SB_HR * (SB_TW / 4); i += 256) {
+        const int ry = i % SB_HR, cx = i / SB_HR * 4;
+        u64 g[4] = {0, 0, 0, 0}, m[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int c = 0; c < 5; c++) {
-            const int xx = cx + 4 + sm.ix[c];
-            const float ax = sm.fx[c], vc = sm.v[c];
-            const float2 p0 = sm.ssob[ry][xx], p1 = sm.ssob[ry][xx + 1];
-            h.x += vc * (p0.x + (p1.x - p0.x) * ax);
-            h.y += vc * (p0.y + (p1.y - p0.y) * ax);
-            h.z += vc * (fabsf(p0.x) + (fabsf(p1.x) - fabsf(p0.x)) * ax);
-            h.w += vc * (fabsf(p0.y) + (fabsf(p1.y) - fabsf(p0.y)) * ax);
+        for (int j = 0; j < 12; j++) {
+            const u64 p = sm.ssob[ry][cx + j], q = sb_abs(p);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (j - k >= 0 && j - k < 9) {
+                    g[k] = sb_fma(p, a.wide_x[j - k], g[k]);
+                    m[k] = sb_fma(q, a.wide_x[j - k], m[k]);
+                }
         }
-        sm.hsum[ry][cx] = h;
+#pragma unroll
+        for (int k = 0; k < 4; k++) sm.hsum[ry * SB_HP + cx + k] = make_ulonglong2(g[k], m[k]);
     }
     __syncthreads();
-    for (int r = threadIdx.y; r < SB_TH; r += blockDim.y) {
-        const int x = x0 + threadIdx.x, y = y0 + r;
-        if (x >= out.w || y >= out.h) continue;
-        const int lx = threadIdx.x + 4, ly = r + 4;  // sobel tile index of (x, y)
-        float res[4];
-        {  // narrow blur: its few taps directly
-            float s0 = 0, s1 = 0, s2 = 0, s3 = 0, norm = 0;
-            for (int t = 0; t < a.n1; t++) {
-                const float w = a.w[t];
-                const float4 b = bil4(sm.ssob, lx + a.ix[t], ly + a.iy[t], a.fx[t], a.fy[t]);
-                s0 += w * b.x;
-                s1 += w * b.y;
-                s2 += w * b.z;
-                s3 += w * b.w;
-                norm += w;
-            }
-            res[0] = s0 / norm;
-            res[1] = s1 / norm;
-            res[2] = s2 / norm;
-            res[3] = s3 / norm;
-        }
-        const float sigma = sqrtf(a.var0 + a.var1 * sm.sraw[r + 5][threadIdx.x + 5]);
-        if (sqrtf(res[0] * res[0] + res[1] * res[1]) < 4.f * sigma) {
-            // vertical pass over the horizontal sums, then the corner tap moved
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    // four rows a thread: the narrow blur from the Sobel values
+    const int lx = threadIdx.x + 4, r0 = threadIdx.y * 4;  // Sobel tile: columns from -4, rows from -4
+    u64 g[4] = {0, 0, 0, 0}, m[4] = {0, 0, 0, 0};
+    u64 pg = 0, pm = 0, cg = 0, cm = 0;  // the row above's corner sums and texels (1, .)
 #pragma unroll
-            for (int k = 0; k < 5; k++) {
-                const int yy = ly + sm.iy[k];
-                const float ay = sm.fy[k], ur = sm.u[k];
-                const float4 h0 = sm.hsum[yy][threadIdx.x], h1 = sm.hsum[yy + 1][threadIdx.x];
-                acc.x += ur * (h0.x + (h1.x - h0.x) * ay);
-                acc.y += ur * (h0.y + (h1.y - h0.y) * ay);
-                acc.z += ur * (h0.z + (h1.z - h0.z) * ay);
-                acc.w += ur * (h0.w + (h1.w - h0.w) * ay);
+    for (int j = 0; j < 7; j++) {  // rows r0 - 1 .. r0 + 5
+        u64 p[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) p[k] = sm.ssob[r0 + 3 + j][lx - 1 + k];
+        if (j < 6) {
+            u64 hg = 0, hm = 0;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                hg = sb_fma(p[k], a.narrow_x[k], hg);
+                hm = sb_fma(sb_abs(p[k]), a.narrow_x[k], hm);
             }
-            const float gxo = float(sm.ix[4]) + sm.fx[4], gyo = float(sm.iy[4]) + sm.fy[4];  // the grid corner
-            const float4 on = bil4(sm.ssob, lx + int(floorf(gxo)), ly + int(floorf(gyo)), gxo - floorf(gxo),
-                                   gyo - floorf(gyo));
-            const float4 at = bil4(sm.ssob, lx + int(floorf(sm.cdx)), ly + int(floorf(sm.cdy)),
-                                   sm.cdx - floorf(sm.cdx), sm.cdy - floorf(sm.cdy));
-            const float it = 1.f / sm.total;
-            res[0] = (acc.x + sm.wc * (at.x - on.x)) * it;
-            res[1] = (acc.y + sm.wc * (at.y - on.y)) * it;
-            res[2] = (acc.z + sm.wc * (at.z - on.z)) * it;
-            res[3] = (acc.w + sm.wc * (at.w - on.w)) * it;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (j - k >= 0 && j - k < 3) {
+                    g[k] = sb_fma(hg, a.narrow_y[j - k], g[k]);
+                    m[k] = sb_fma(hm, a.narrow_y[j - k], m[k]);
+                }
         }
-        st2<S>(out.px(x, y), f2{copysignf(res[2], res[0]), copysignf(res[3], res[1])});
+        if (j >= 2) {  // corner of output j - 3: the mean of (1..2, 1..2) less (1, 1)
+            const u64 sg = sb_add(p[2], p[3]), q = sb_abs(p[2]), sq = sb_add(q, sb_abs(p[3]));
+            if (j >= 3) {
+                const float2 quarter = make_float2(0.25f * a.narrow_c.x, 0.25f * a.narrow_c.x);
+                const float2 minus = make_float2(-a.narrow_c.x, -a.narrow_c.x);
+                g[j - 3] = sb_fma(cg, minus, sb_fma(sb_add(pg, sg), quarter, g[j - 3]));
+                m[j - 3] = sb_fma(cm, minus, sb_fma(sb_add(pm, sq), quarter, m[j - 3]));
+            }
+            pg = sg, pm = sq, cg = p[2], cm = q;
+        }
     }
+    bool flat[4], any = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float sigma2 = a.var0 + a.var1 * sm.sraw[r0 + k + 5][threadIdx.x + 5];
+        const float2 v = sb_pair(g[k]);
+        flat[k] = sqrtf(v.x * v.x + v.y * v.y) < 4.f * sqrtf(sigma2);
+        any = any || flat[k];
+    }
+    if (__any_sync(0xffffffffu, any)) {  // the vertical pass over the horizontal sums
+        u64 wg[4] = {0, 0, 0, 0}, wm[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < 12; j++) {
+            const ulonglong2 h = sm.hsum[(r0 + j) * SB_HP + threadIdx.x];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (j - k >= 0 && j - k < 9) {
+                    wg[k] = sb_fma(h.x, a.wide_y[j - k], wg[k]);
+                    wm[k] = sb_fma(h.y, a.wide_y[j - k], wm[k]);
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < 5; j++) {  // the corner: (4..5, 4..5) less (4, 4)
+            const u64 p = sm.ssob[r0 + 8 + j][lx + 4], p1 = sm.ssob[r0 + 8 + j][lx + 5], q = sb_abs(p);
+            const u64 sg = sb_add(p, p1), sq = sb_add(q, sb_abs(p1));
+            if (j > 0) {
+                const float2 quarter = make_float2(0.25f * a.wide_c.x, 0.25f * a.wide_c.x);
+                const float2 minus = make_float2(-a.wide_c.x, -a.wide_c.x);
+                wg[j - 1] = sb_fma(cg, minus, sb_fma(sb_add(pg, sg), quarter, wg[j - 1]));
+                wm[j - 1] = sb_fma(cm, minus, sb_fma(sb_add(pm, sq), quarter, wm[j - 1]));
+            }
+            pg = sg, pm = sq, cg = p, cm = q;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (flat[k]) {
+                g[k] = wg[k];
+                m[k] = wm[k];
+            }
+    }
+    const int x = x0 + threadIdx.x;
+    if (x >= out.w) return;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int y = y0 + r0 + k;
+        if (y >= out.h) break;
+        const float2 s = sb_pair(g[k]), v = sb_pair(m[k]);
+        st2<S>(out.px(x, y), f2{copysignf(v.x, s.x), copysignf(v.y, s.y)});
+    }
+}
+
+// A blur's taps as texel factors: column sums in x, row sums over the total in y.
+template <int N, int R>
+static float sep_factors(const BlurArgs& a, int first, float2 (&fx)[2 * R + 1], float2 (&fy)[2 * R + 1]) {
+    float cs[2 * R + 1] = {}, rs[2 * R + 1] = {}, total = 0.f;
+    auto put = [](float (&f)[2 * R + 1], int i, float frac, float w) {
+        f[i + R] += w * (1.f - frac);
+        if (i < R) f[i + R + 1] += w * frac;  // at R the fraction is 0
+    };
+    for (int t = first; t < first + N * N; t++) total += a.w[t];
+    for (int r = 0; r < N; r++)
+        for (int c = 0; c < N; c++) {
+            const float w = a.w[first + r * N + c];
+            put(cs, a.ix[first + c], a.fx[first + c], w);
+            put(rs, a.iy[first + r * N], a.fy[first + r * N], w / total);
+        }
+    for (int k = 0; k < 2 * R + 1; k++) {
+        fx[k] = make_float2(cs[k] / total, cs[k] / total);  // (sum_c cs) (sum_r rs) = total / total
+        fy[k] = make_float2(rs[k], rs[k]);
+    }
+    return a.w[first + N * N - 1] / total;
 }
 
 // --------------------------------------------------------------------------
@@ -842,10 +918,22 @@ template <class S>
 void launch_sobel_blur(Plane<S, 1> raw, Plane<S, 2> out, const BlurArgs& a, cudaStream_t s) {
     dim3 b(32, 8);
     dim3 g((raw.w + SB_TW - 1) / SB_TW, (raw.h + SB_TH - 1) / SB_TH);
-    // the FP16-storage path takes the separable form of the 5 x 5 wide blur;
+    // the FP16-storage path takes the separable form of the two blurs;
     // the FP32 plain path evaluates the reference's 25 bilinear taps
-    if (is_half<S>::value && a.n2 == 25) k_sobel_blur_sep<S><<<g, b, 0, s>>>(raw, out, a);
-    else k_sobel_blur<S><<<g, b, 0, s>>>(raw, out, a);
+    if (is_half<S>::value && a.n1 == 4 && a.n2 == 25) {
+        SepBlur f;
+        const float nc = sep_factors<2, 1>(a, 0, f.narrow_x, f.narrow_y);
+        const float wc = sep_factors<5, 4>(a, a.n1, f.wide_x, f.wide_y);
+        f.narrow_c = make_float2(nc, nc);
+        f.wide_c = make_float2(wc, wc);
+        f.var0 = a.var0;
+        f.var1 = a.var1;
+        f.inv_sqrt45 = a.inv_sqrt45;
+        ensure_dynamic_smem(reinterpret_cast<const void*>(k_sobel_blur_sep<S>), int(sizeof(SepSmem)));
+        k_sobel_blur_sep<S><<<g, b, sizeof(SepSmem), s>>>(raw, out, f);
+    } else {
+        k_sobel_blur<S><<<g, b, 0, s>>>(raw, out, a);
+    }
 }
 
 template <class S>
