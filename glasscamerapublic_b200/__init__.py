@@ -275,7 +275,7 @@ def device_memory(reset_peak: bool = False) -> tuple[int, int]:
 
 
 def block_match_tiles() -> list:
-    """The FP16 block matcher's autotuned tile variants: [(w, h, variant)],
+    """The FP16 block matcher's tile variant of each level size met: [(w, h, variant)],
     variant = 10 x thread rows + pixels per thread (84, 162: 32x32-pixel
     tiles; 44, 82: 32x16)."""
     buf = (C.c_int32 * 192)()

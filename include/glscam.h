@@ -144,7 +144,7 @@ enum {
                                     launch (see there) */
     GLS_BM_TENSOR = 1u << 9      /* FP16 storage, stream-launched: block matching with the patch distances
                                     and the weighted sums on the tensor cores and the weights in half
-                                    precision; without it the FP16 matcher computes every weight in packed
+                                    precision; without it the FP16 matcher computes every weight and sum in
                                     FP32 (the persistent batch always does) */
 };
 
@@ -243,7 +243,7 @@ typedef struct gls_frame_desc {
  * eigen-solve and block matching, PyramidProcessor::denoise,
  * pyramid_processor.cpp:96-172) from a device work list whose tasks wait
  * on per-level counters, then the output transforms run; it runs the
- * stream kernels' device code (the default packed-FP32 block matcher), so
+ * stream kernels' device code (the default block matcher), so
  * the results are bit-identical to the stream-launched batch. The call
  * returns after the
  * kernel, with GLS_ERR_TIMEOUT if a task's wait for its inputs ran past
@@ -340,14 +340,13 @@ gls_status gls_converter_reset_stats(gls_converter* conv);
  * device during gls_demosaic with GLS_POSTPROCESS. */
 gls_status gls_grain_tables(uint32_t seed, int32_t* perm, float* grad);
 
-/* Decisions of the FP16 block matcher's tile autotuner (no reference
- * counterpart): for each pyramid level size met so far in this process,
- * (width, height, variant), variant = 10 x thread rows + pixels per thread:
- * 84 and 162 for 32x32-pixel tiles, 44 and 82 for 32x16. The first frame of
- * a size times every variant and keeps the fastest; all compute identical
- * results. Writes at most max_entries triples to entries; *n receives the
- * count. GLS_BM_TILE=84, 44, 82 or 162 in the environment (8 or 4 for 84 or
- * 44) fixes the variant. */
+/* The FP16 block matcher's tile variant (no reference counterpart): for each
+ * pyramid level size met so far in this process, (width, height, variant),
+ * variant = 10 x thread rows + pixels per thread: 84 and 162 for
+ * 32x32-pixel tiles, 44 and 82 for 32x16. Every size takes 82; all compute
+ * identical results. Writes at most max_entries triples to entries; *n
+ * receives the count. GLS_BM_TILE=84, 44, 82 or 162 in the environment (8 or
+ * 4 for 84 or 44) fixes the variant. */
 gls_status gls_block_match_tiles(int32_t* entries, int32_t max_entries, int32_t* n);
 
 /* ---- CameraCalibration<levels> (CameraCalibration.hpp:24-39) ----
