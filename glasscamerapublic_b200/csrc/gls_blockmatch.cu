@@ -672,10 +672,11 @@ static void launch_pair(Plane<__half, 4> img, Plane<__half, 2> grad, const float
     dim3 g((img.w + BX_TX - 1) / BX_TX, (img.h + NP * TY - 1) / (NP * TY));
     // A level too small for the 296 blocks that fit the chip: each tile's groups
     // are dealt to up to 8 blocks, which stage it alike. 126x94 (24 tiles) 20 us,
-    // 43 with a block a tile; 252x189 (96) 42 and 44; taken further, to twice
-    // the blocks that fit, 252x189 takes 52.
+    // 43 with a block a tile; 256x192 (96) 34 and 44 (41 over two blocks); taken
+    // further, past the blocks that fit, 52.
     if (split)
-        while (g.z < 8 && g.x * g.y * g.z * 2 <= 296) g.z *= 2;
+        for (const unsigned z : {2u, 3u, 4u, 8u})  // 4, 3, 2, 1 of a tile's 8 rounds of groups
+            if (g.x * g.y * z <= 296) g.z = z;
     k_block_match_pair<TY, NP><<<g, BxTile<TY, NP>::THREADS, smem, s>>>(img, grad, basis, out, a);
 }
 

@@ -62,9 +62,9 @@ def test_fp16_matcher_follows_the_fp32_one(h, w, lsc):
     assert (np.abs(a[..., 3] - b[..., 3]) < 0.05 * b[..., 3])[ok].all()
 
 
-@pytest.mark.parametrize("h,w", [(64, 90), (128, 150), (250, 250), (303, 610)])
+@pytest.mark.parametrize("h,w", [(64, 90), (128, 150), (192, 256), (250, 250), (303, 610)])
 def test_fp16_tiles_split_over_blocks(h, w):
-    """12, 40, 128 and 380 tiles: their groups over 8, 4, 2 and 1 blocks. Bounds as above."""
+    """12, 40, 96, 128 and 380 tiles: their groups over 8, 4, 3, 2 and 1 blocks. Bounds as above."""
     ycc, grad = _image(h, w, h)
     p = _params(h, w)
     a, b = _denoise(ycc, grad, p, True), _denoise(ycc, grad, p, False)
