@@ -525,51 +525,16 @@ struct DmSites {
     __device__ __forceinline__ bool blue(int px, int py) const { return (bx & 1) == (px & 1) && (by & 1) == (py & 1); }
 };
 
-// The interpolation's divisions, square roots and gradient direction: as
-// written on the FP32 path; on the FP16-storage path, still in FP32, by the
-// approximate instructions (2^-21) and an odd polynomial for the arc tangent
-// of a first-quadrant direction (degree 17, fitted on Chebyshev nodes, 8e-8).
-template <class S>
-struct DmMath {
-    static constexpr float kPi = 3.14159265358979323846f;
-    __device__ __forceinline__ static float div(float a, float b) { return a / b; }
-    __device__ __forceinline__ static float root(float a) { return sqrtf(a); }
-    __device__ __forceinline__ static float dir(float y, float x) { return 2.f * atan2f(y, x) / kPi; }
-    __device__ __forceinline__ static float step(float e0, float e1, float x) { return smoothstepf(e0, e1, x); }
-};
-template <>
-struct DmMath<__half> {
-    __device__ __forceinline__ static float div(float a, float b) { return __fdividef(a, b); }
-    __device__ __forceinline__ static float root(float a) {
-        float r;
-        asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
-        return r;
-    }
-    __device__ __forceinline__ static float dir(float y, float x) {  // 2 / pi atan2(y, x), y and x not negative
-        const float hi = fminf(fmaxf(y, x), 1e18f), t = __fdividef(fminf(y, x), fmaxf(hi, 1e-30f)), u = t * t;
-        float p = 0.0018042214421480179f;
-        p = fmaf(p, u, -0.010189118795096874f);
-        p = fmaf(p, u, 0.027112113311886787f);
-        p = fmaf(p, u, -0.047717489302158356f);
-        p = fmaf(p, u, 0.06771568208932877f);
-        p = fmaf(p, u, -0.09041637182235718f);
-        p = fmaf(p, u, 0.12727610766887665f);
-        p = fmaf(p, u, -0.21220488846302032f);
-        p = fmaf(p, u, 0.6366197466850281f) * t;
-        return y > x ? 1.f - p : p;
-    }
-    __device__ __forceinline__ static float step(float e0, float e1, float x) {
-        const float t = clampf(__fdividef(x - e0, e1 - e0), 0.f, 1.f);
-        return t * t * (3.f - 2.f * t);
-    }
-};
+// the direction of a gradient of magnitudes (x, y), 0 (along x) .. 1, and its length
+__device__ __forceinline__ float2 dm_direction(float x, float y) {
+    const float kPi = 3.14159265358979323846f;
+    return make_float2(2.f * atan2f(y, x) / kPi, sqrtf(x * x + y * y));
+}
 
 // interpolateGreen (demosaic.metal:215-316) at raw-tile index (lx, ly) of a
 // red or blue site; gg = the gradient's direction and length there.
-template <class S>
 __device__ __forceinline__ float dm_green(const DemosaicSmem& sm, int lx, int ly, float2 gg, const DemosaicArgs& a,
                                           float lowNoise) {
-    using M = DmMath<S>;
     auto R = [&](int di, int dj) { return sm.raw[ly + dj][lx + di]; };
     const float gl = R(-1, 0), gr = R(1, 0), gu = R(0, -1), gd = R(0, 1);
     const float cxy = R(0, 0);
@@ -578,19 +543,19 @@ __device__ __forceinline__ float dm_green(const DemosaicSmem& sm, int lx, int ly
     const float gave = (gl + gr + gu + gd) / 4.f;
     const float glfx = (gl + gr) / 2.f, glfy = (gu + gd) / 2.f;
     const float ghfx = ((cl + cr) - 2.f * cxy) / 4.f, ghfy = ((cu + cd) - 2.f * cxy) / 4.f;
-    const float sd = M::root(a.gv0 + a.gv1 * gave);
+    const float sd = sqrtf(a.gv0 + a.gv1 * gave);
     const float glen = gg.y;
-    const float gthr = M::step(sd, 4.f * sd, glen);
-    const float lowthr = 1.f - M::step(2.f * sd, 8.f * sd, glen);
+    const float gthr = smoothstepf(sd, 4.f * sd, glen);
+    const float lowthr = 1.f - smoothstepf(2.f * sd, 8.f * sd, glen);
     const float sharp = (0.5f + 0.5f * lowNoise) * gthr * (1.f + lowNoise * lowthr);
-    const float hl = 1.f - M::step(0.25f, 1.f, fmaxf(cxy, fmaxf(fmaxf(cl, cr), fmaxf(cu, cd))));
+    const float hl = 1.f - smoothstepf(0.25f, 1.f, fmaxf(cxy, fmaxf(fmaxf(cl, cr), fmaxf(cu, cd))));
     float dir = gg.x;
     if (a.gv1 < 1e-3f) {
-        dir = dir < 0.5f ? mixf(dir, 0.f, 1.f - M::step(0.3f, 0.45f, dir))
-                         : mixf(dir, 1.f, M::step(1.f - 0.45f, 1.f - 0.3f, dir));
+        dir = dir < 0.5f ? mixf(dir, 0.f, 1.f - smoothstepf(0.3f, 0.45f, dir))
+                         : mixf(dir, 1.f, smoothstepf(1.f - 0.45f, 1.f - 0.3f, dir));
     }
     const float cmin = fminf(cxy, fminf(gave, c2ave)), cmax = fmaxf(cxy, fmaxf(gave, c2ave));
-    const float white = M::div(cmin, cmax);
+    const float white = cmin / cmax;
     const float k = hl * white * sharp;
     const float gex = glfx - k * ghfx, gey = glfy - k * ghfy;
     float g = mixf(gey, gex, dir);
@@ -602,10 +567,8 @@ __device__ __forceinline__ float dm_green(const DemosaicSmem& sm, int lx, int ly
 
 // interpolateRedBlue (demosaic.metal:318-416) at a red or blue site: the
 // other colour; green-tile index (gx, gy), raw-tile index (lx, ly).
-template <class S>
 __device__ __forceinline__ float dm_redblue(const DemosaicSmem& sm, int gx, int gy, int lx, int ly, bool red,
                                             const DemosaicArgs& a) {
-    using M = DmMath<S>;
     auto R = [&](int di, int dj) { return sm.raw[ly + dj][lx + di]; };
     auto G = [&](int di, int dj) { return sm.green[gy + dj][gx + di]; };
     const float g0 = G(0, 0), c1 = R(0, 0);
@@ -615,12 +578,12 @@ __device__ __forceinline__ float dm_redblue(const DemosaicSmem& sm, int gx, int 
     const float gtl2 = G(-2, -2), gtr2 = G(2, -2), gbl2 = G(-2, 2), gbr2 = G(2, 2);
     const float gctl2 = gtl2 - R(-2, -2), gctr2 = gtr2 - R(2, -2), gcbl2 = gbl2 - R(-2, 2), gcbr2 = gbr2 - R(2, 2);
     const float v0 = red ? a.rv0 : a.bv0, v1 = red ? a.rv1 : a.bv1;
-    const float sd = M::root(v0 + v1 * c2ave);
+    const float sd = sqrtf(v0 + v1 * c2ave);
     const float2 gg = sm.grad[gy][gx];
     const float dir = 1.f - gg.x;
-    const float gthr = M::step(sd, 4.f * sd, gg.y);
+    const float gthr = smoothstepf(sd, 4.f * sd, gg.y);
     const float alpha = mixf(0.5f, dir, gthr);
-    const float hl = 1.f - M::step(0.25f, 1.f, fmaxf(g0, fmaxf(fmaxf(gtr2, gbl2), fmaxf(gtl2, gbr2))));
+    const float hl = 1.f - smoothstepf(0.25f, 1.f, fmaxf(g0, fmaxf(fmaxf(gtr2, gbl2), fmaxf(gtl2, gbr2))));
     const float gc = g0 - c1;
     const float aa = (gctr + gcbl) / 2.f + hl * (gctr2 + gcbl2 - 2.f * gc) / 8.f;
     const float bb = (gctl + gcbr) / 2.f + hl * (gctl2 + gcbr2 - 2.f * gc) / 8.f;
@@ -632,10 +595,8 @@ __device__ __forceinline__ float dm_redblue(const DemosaicSmem& sm, int gx, int 
 
 // interpolateRedBlueAtGreen (demosaic.metal:418-521) at a green site:
 // tmp-tile index (cx, cy); gg = the gradient's direction and length.
-template <class S>
 __device__ __forceinline__ void dm_rb_at_green(const DemosaicSmem& sm, int cx, int cy, float2 gg, const DemosaicArgs& a,
                                                float rgb[3]) {
-    using M = DmMath<S>;
     auto P = [&](int di, int dj, int c) { return sm.tmp[c][cy + dj][cx + di]; };
     const float g0 = P(0, 0, 1);
     const float lr = P(-1, 0, 0), lg = P(-1, 0, 1), lb = P(-1, 0, 2);
@@ -651,10 +612,10 @@ __device__ __forceinline__ void dm_rb_at_green(const DemosaicSmem& sm, int cx, i
     const float gbu3 = P(0, -3, 1) - P(0, -3, 2), gbd3 = P(0, 3, 1) - P(0, 3, 2);
     const float dir = gg.x;
     const float glen = gg.y;
-    const float rsd = M::root(a.rv0 + a.rv1 * red_ave), bsd = M::root(a.bv0 + a.bv1 * blue_ave);
-    const float ralpha = mixf(0.5f, dir, M::step(rsd, 4.f * rsd, glen));
-    const float balpha = mixf(0.5f, dir, M::step(bsd, 4.f * bsd, glen));
-    const float hl = 1.f - M::step(0.25f, 1.f, fmaxf(g0, fmaxf(fmaxf(rg, lg), fmaxf(dg, ug))));
+    const float rsd = sqrtf(a.rv0 + a.rv1 * red_ave), bsd = sqrtf(a.bv0 + a.bv1 * blue_ave);
+    const float ralpha = mixf(0.5f, dir, smoothstepf(rsd, 4.f * rsd, glen));
+    const float balpha = mixf(0.5f, dir, smoothstepf(bsd, 4.f * bsd, glen));
+    const float hl = 1.f - smoothstepf(0.25f, 1.f, fmaxf(g0, fmaxf(fmaxf(rg, lg), fmaxf(dg, ug))));
     const float red_v = g0 - mixf((gru + grd) / 2.f - hl * ((grd3 - gru) - (grd - gru3)) / 8.f,
                                   (grl + grr) / 2.f - hl * ((grr3 - grl) - (grr - grl3)) / 8.f, ralpha);
     const float blue_v = g0 - mixf((gbu + gbd) / 2.f - hl * ((gbd3 - gbu) - (gbd - gbu3)) / 8.f,
@@ -692,10 +653,11 @@ __device__ __forceinline__ f4 dm_finish(float rgb[3], const DemosaicArgs& a) {
     return o;
 }
 
-// Bound by instruction issue (84% of the slots; 4032x3024 FP16: 230 us, 342 with
-// the IEEE sequences, atan2f for each of a site's interpolations and a loop with
-// divisions for the staging; FP32 1024x768: 32 us, 38): the gradient's direction
-// and length are formed once per staged position.
+// Bound by instruction issue: FP32 as written for both storages, IEEE divisions
+// and square roots. The gradient's direction and length are formed once per
+// staged position, and the staging's loads are in flight together: 4032x3024
+// FP16 305 us (332 with atan2f for each of a site's interpolations and a loop
+// with divisions for the staging), FP32 1024x768 32 us (38).
 template <class S>
 __global__ void __launch_bounds__(256) k_demosaic(Plane<S, 1> raw, Plane<S, 2> grad, Plane<S, 4> out, DemosaicArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -728,11 +690,8 @@ __global__ void __launch_bounds__(256) k_demosaic(Plane<S, 1> raw, Plane<S, 2> g
             if (ty0 + 4 * k < DM_RH) sm.raw[ty0 + 4 * k][tx] = to_f(v[k]);
 #pragma unroll
         for (int k = 0; k < NG; k++)
-            if (tx < DM_GW && ty0 + 4 * k < DM_GH) {
-                const float2 gg = make_float2(fabsf(gv[k].x), fabsf(gv[k].y));
-                sm.grad[ty0 + 4 * k][tx] =
-                    make_float2(DmMath<S>::dir(gg.y, gg.x), DmMath<S>::root(gg.x * gg.x + gg.y * gg.y));
-            }
+            if (tx < DM_GW && ty0 + 4 * k < DM_GH)
+                sm.grad[ty0 + 4 * k][tx] = dm_direction(fabsf(gv[k].x), fabsf(gv[k].y));
     }
     __syncthreads();
 
@@ -746,14 +705,14 @@ __global__ void __launch_bounds__(256) k_demosaic(Plane<S, 1> raw, Plane<S, 2> g
             const int trb = tx0 + (((x0 - 5 + tx0) ^ py ^ rb_par) & 1);  // the pair's red/blue entry
             const int tg = tx0 + tx0 + 1 - trb;
             sm.green[ty][tg] = sm.raw[ty + 2][tg + 2];
-            sm.green[ty][trb] = dm_green<S>(sm, trb + 2, ty + 2, sm.grad[ty][trb], a, lowNoise);
+            sm.green[ty][trb] = dm_green(sm, trb + 2, ty + 2, sm.grad[ty][trb], a, lowNoise);
         }
     } else {
         for (int i = tid; i < DM_GW * DM_GH; i += nth) {
             const int ty = i / DM_GW, tx = i % DM_GW;
             const int px = clampi(x0 - 5 + tx, 0, W - 1), py = clampi(y0 - 5 + ty, 0, H - 1);
             const int lx = px - (x0 - 7), ly = py - (y0 - 7);  // raw-tile index of the clamped position
-            sm.green[ty][tx] = (st.red(px, py) || st.blue(px, py)) ? dm_green<S>(sm, lx, ly, sm.grad[ty][tx], a, lowNoise)
+            sm.green[ty][tx] = (st.red(px, py) || st.blue(px, py)) ? dm_green(sm, lx, ly, sm.grad[ty][tx], a, lowNoise)
                                                                    : sm.raw[ly][lx];
         }
     }
@@ -771,7 +730,7 @@ __global__ void __launch_bounds__(256) k_demosaic(Plane<S, 1> raw, Plane<S, 2> g
             sm.tmp[0][ty][tg] = 0.f;
             sm.tmp[1][ty][tg] = sm.green[ty + 2][tg + 2];
             sm.tmp[2][ty][tg] = 0.f;
-            const float c2 = dm_redblue<S>(sm, trb + 2, ty + 2, trb + 4, ty + 4, red, a);
+            const float c2 = dm_redblue(sm, trb + 2, ty + 2, trb + 4, ty + 4, red, a);
             const float c1 = sm.raw[ty + 4][trb + 4];
             sm.tmp[0][ty][trb] = red ? c1 : c2;
             sm.tmp[1][ty][trb] = sm.green[ty + 2][trb + 2];
@@ -790,7 +749,7 @@ __global__ void __launch_bounds__(256) k_demosaic(Plane<S, 1> raw, Plane<S, 2> g
                 o1 = sm.green[gy][gx];
                 o2 = 0.f;
             } else {
-                const float c2 = dm_redblue<S>(sm, gx, gy, lx, ly, red, a);
+                const float c2 = dm_redblue(sm, gx, gy, lx, ly, red, a);
                 const float c1 = sm.raw[ly][lx];
                 o0 = red ? c1 : c2;
                 o1 = sm.green[gy][gx];
@@ -823,7 +782,7 @@ __global__ void __launch_bounds__(256) k_demosaic(Plane<S, 1> raw, Plane<S, 2> g
                 rgb[1] = sm.tmp[1][cy][cx];
                 rgb[2] = sm.tmp[2][cy][cx];
             } else {
-                dm_rb_at_green<S>(sm, cx, cy, sm.grad[r + 5][c + 5], a, rgb);
+                dm_rb_at_green(sm, cx, cy, sm.grad[r + 5][c + 5], a, rgb);
             }
             st4<S>(out.px(x, y), dm_finish(rgb, a));
         }
