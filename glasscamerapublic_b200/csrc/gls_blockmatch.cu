@@ -31,20 +31,16 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
-// Per-pixel constants shared by both kernels.
+// Per-pixel constants of the matchers.
 struct BmConst {
-    float in_y, in_cb, in_cr;
     float s;       // luma distance scale
     float c1, c2;  // chroma scales (dm / chroma_boost)
 };
 
 template <class S>
 __device__ __forceinline__ BmConst bm_const(const BlockMatchArgs& a, Plane<S, 2> grad, int w, int h, int px, int py,
-                                            float y, float cb, float cr) {
+                                            float y) {
     BmConst k;
-    k.in_y = y;
-    k.in_cb = cb;
-    k.in_cr = cr;
     float ls = 1.f;
     if (a.lsc > 0.f) {  // lensShading, demosaic.metal:91-93, at the pixel
         const float cx = float(w / 2), cy = float(h / 2);
@@ -62,31 +58,6 @@ __device__ __forceinline__ BmConst bm_const(const BlockMatchArgs& a, Plane<S, 2>
     k.s = dm0 / (1.f + a.gradient_boost * edge);
     k.c1 = dm1 / a.chroma_boost;
     k.c2 = dm2 / a.chroma_boost;
-    return k;
-}
-
-// The same for the FP16-storage path: reciprocals and square roots by rsqrtf
-// and __fdividef (a few 2^-24 each, FP32 throughout), inv[c] = 1 / a.tm[c] and
-// ib = 1 / chroma_boost formed once per thread: about 50 instructions a pixel
-// where the IEEE sequences take 200.
-__device__ __forceinline__ BmConst bm_const_h(const BlockMatchArgs& a, const float (&inv)[3], float ib,
-                                              Plane<__half, 2> grad, int w, int h, int px, int py, float y) {
-    BmConst k{};
-    float ls = 1.f;
-    if (a.lsc > 0.f) {  // lensShading, demosaic.metal:91-93, at the pixel
-        const float cx = float(w / 2), cy = float(h / 2);
-        const float dx = float(px) - cx, dy = float(py) - cy;
-        ls = 1.f + a.lsc * __fdividef(dx * dx + dy * dy, cx * cx + cy * cy);
-    }
-    const float r0 = rsqrtf(a.var_a[0] + a.var_b[0] * ls * y);
-    const float r1 = rsqrtf(a.var_a[1] + a.var_b[1] * ls * y);
-    const float r2 = rsqrtf(a.var_a[2] + a.var_b[2] * ls * y);
-    const f2 g = ld2<__half>(grad.px(px, py));
-    const float mag = sqrtf(g.x * g.x + g.y * g.y);
-    const float t = clampf((a.gradient_threshold * mag * r0 - 2.f) * (1.f / 14.f), 0.f, 1.f);  // smoothstep(2, 16, .)
-    k.s = __fdividef(inv[0] * r0, 1.f + a.gradient_boost * (t * t * (3.f - 2.f * t)));
-    k.c1 = inv[1] * r1 * ib;
-    k.c2 = inv[2] * r2 * ib;
     return k;
 }
 
@@ -220,7 +191,7 @@ __global__ void __launch_bounds__(128, 3)
     for (int p = 0; p < NP; p++) {
         const int c = (NP * threadIdx.y + p + 10) * T::W + threadIdx.x + 10;
         const float4 in = sm.ycc[c];
-        const BmConst k = bm_const<float>(a, grad, img.w, img.h, min(x, img.w - 1), min(y + p, img.h - 1), in.z, in.x, in.y);
+        const BmConst k = bm_const<float>(a, grad, img.w, img.h, min(x, img.w - 1), min(y + p, img.h - 1), in.z);
         BmPlainPix& P = pix[p];
         const float4 p0 = *reinterpret_cast<const float4*>(&sm.pca0[c]), p1 = *reinterpret_cast<const float4*>(&sm.pca1[c]);
         P.n[0] = pk2(-p0.x, -p0.y);
@@ -607,7 +578,6 @@ __device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& 
     }
     __syncthreads();
     // the pixels' constants, once each
-    const float inv[3] = {1.f / a.tm[0], 1.f / a.tm[1], 1.f / a.tm[2]}, ib = 1.f / a.chroma_boost;
     float kmax = 0.f;
     for (int i = tid; i < T::ROWS * BX_TX; i += NT) {
         const int px = i % BX_TX, py = i / BX_TX;
@@ -615,7 +585,7 @@ __device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& 
         const float4 yb = sm.yb[c];
         const float cr = sm.cr[c].x;
         const BmConst k =
-            bm_const_h(a, inv, ib, grad, img.w, img.h, min(x0 + px, img.w - 1), min(y0 + py, img.h - 1), yb.x);
+            bm_const<__half>(a, grad, img.w, img.h, min(x0 + px, img.w - 1), min(y0 + py, img.h - 1), yb.x);
         const float kl = fmaxf(-2.f * kLog2e * k.s * k.s, -1e30f), sq = sqrtf(lk);
         const float c1 = sq * k.c1, c2 = sq * k.c2;
         sm.k[BK_KL][i] = kl;
@@ -899,7 +869,7 @@ __device__ __forceinline__ void bm_mma_tile(int x0, int y0, const Plane<__half, 
             const int pos = sy * BM_W + sx;
             const float in_y = __half2float(sm.y[pos]), in_cb = __half2float(sm.cb[pos]), in_cr = __half2float(sm.cr[pos]);
             const int ix = min(x0 + gx + pxl, img.w - 1), iy = min(y0 + gy + py[r], img.h - 1);
-            const BmConst k = bm_const<__half>(a, grad, img.w, img.h, ix, iy, in_y, in_cb, in_cr);
+            const BmConst k = bm_const<__half>(a, grad, img.w, img.h, ix, iy, in_y);
             const float kl = fmaxf(-2.f * kLog2e * k.s * k.s, -1e30f);
             const float base = fmaf(kl, sm.nn[pos], 0.5f * log2f(lk));
             const float sq = sqrtf(lk);

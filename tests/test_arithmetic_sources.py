@@ -13,3 +13,9 @@ def code(name):
 
 def test_the_raw_front_end_divides_and_takes_roots_in_full_precision():
     assert re.findall(APPROX, code("gls_front.cu")) == []
+
+
+def test_the_block_matchers_constants_are_formed_in_full_precision():
+    """Of the approximate forms only 1 / sqrt(2 log2 e), a constant of the weights' scale."""
+    found = re.findall(r"[^\n]*(?:" + APPROX + r")[^\n]*", code("gls_blockmatch.cu"))
+    assert found and all("isq = rsqrtf(lk);" in line for line in found)
