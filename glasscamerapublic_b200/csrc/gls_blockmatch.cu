@@ -229,17 +229,21 @@ __global__ void __launch_bounds__(128, 3)
 // a group of 4 x 2 pixels: the union of their windows is 24 x 22 positions, of
 // which each pixel's 21 x 21 window is 83.5%, walked as 33 tiles of 16
 // neighbours (2 rows x 8 columns). Per tile
-//   * S = |q'|^2 - 2 p'.q' for 16 neighbours x 8 pixels by one mma.sync
+//   * S = |q'|^2 / 2 - p'.q' for 16 neighbours x 8 pixels by one mma.sync
 //     m16n8k8: A holds the neighbours' centred coefficients (8 halves), B the
-//     pixels' times -2 (exact), C the neighbours' |q'|^2 in FP32. Products of
-//     halves are exact in FP32 and the sum is an FP32 sum, as the scalar form's;
-//     centring on the tile-centre pixel's coefficients keeps the cancellation
-//     error at FP32 rounding of the local variation of the coefficients;
+//     pixels' negated (any finite half stays one; twice them need not), C the
+//     neighbours' |q'|^2 / 2 in FP32. Products of
+//     halves are exact in FP32; the MMA's sum of nine terms does not round each
+//     addition to nearest, but rounds fewer times than a chain of FP32 FMAs: the
+//     exponents' error against float64 is 0.8 of the chain's (rms), the largest
+//     0.6 to 1.0 of it, for coefficients of 0 to 300 times their noise; centring on
+//     the tile-centre pixel's coefficients keeps the cancellation error at FP32
+//     rounding of the local variation of the coefficients;
 //   * a lane gets S of two horizontally adjacent pixels for each of two
 //     neighbours and evaluates both pixels' weights as packed FP32 pairs
 //     (fma/mul/add .rn.f32x2), the neighbour's values staged twice so that one
 //     load gives the broadcast pair: lw scaled by sqrt(2 log2 e) =
-//     exp2(kl S + base), chroma weight exp2(-(lw^2 + d1^2 + d2^2 - log2 sw)),
+//     exp2(2 kl S + base), chroma weight exp2(-(lw^2 + d1^2 + d2^2 - log2 sw)),
 //     both by ex2.approx.f32 (the reference uses half-precision exp under fast
 //     math here), then the five FP32 sums;
 //   * the spatial weight is separable. Its row part comes from a 23-entry table
@@ -296,14 +300,14 @@ struct BmTileSmem {
     uint4 q[T::H * BX_W];                  // q - c, 8 halves
     float4 yb[T::H * BX_W];                // (Y, Y, Cb, Cb)
     float2 cr[T::H * BX_W];                // (Cr, Cr)
-    float2 nn[T::H * BX_W];                // (|q - c|^2, the same)
+    float2 nn[T::H * BX_W];                // (|q - c|^2 / 2, the same)
     float4 wrow[24];                       // row part of the spatial weight, dy = -11 .. 11: (-log2, -log2, w / sqrt(lk) twice)
     float wcol[28];                        // column part, dx = -13 .. 13
     float cen[8];
     float bsm[25][8];
-    float k[BK_COUNT][T::ROWS * BX_TX];    // per pixel: kl, base, c1, c2, -c1 Cb, -c2 Cr
+    float k[BK_COUNT][T::ROWS * BX_TX];    // per pixel: 2 kl, base, c1, c2, -c1 Cb, -c2 Cr
     __half luma[2][T::LH * BX_LW];         // the luma tile, and the same shifted left by one
-    unsigned nn_max, kl_max;               // bits of the largest |q - c|^2 and |kl|
+    unsigned nn_max, kl_max;               // bits of the largest |q - c|^2 / 2 and |2 kl|
 };
 
 // a lane's view of a group: two adjacent pixels' constants as pairs
@@ -349,9 +353,9 @@ __device__ __forceinline__ void bm_group(const Sm& sm, int gx, int gy, u64 (&acc
         auto pair = [&](int c) { return as_u64(*reinterpret_cast<const float2*>(&sm.k[c][i])); };
         P = {pair(BK_KL), pair(BK_BASE), pair(BK_C1), pair(BK_C2), pair(BK_NO1), pair(BK_NO2)};
     }
-    // B: pixel g's coefficients 2t, 2t + 1 times -2
+    // B: minus pixel g's coefficients 2t, 2t + 1
     const uint32_t* q32 = reinterpret_cast<const uint32_t*>(sm.q);
-    const uint32_t bq = hmul2_u(q32[((gy + (g >> 2) + 10) * BX_W + gx + (g & 3) + 10) * 4 + t], 0xc000c000u);
+    const uint32_t bq = q32[((gy + (g >> 2) + 10) * BX_W + gx + (g & 3) + 10) * 4 + t] ^ 0x80008000u;
 #pragma unroll
     for (int k = 0; k < 15; k++) acc[k / 5][k % 5] = 0;
     // neighbour g of a tile's first row; ldmatrix: lanes 0-7 the first row's
@@ -565,6 +569,8 @@ __device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& 
         n0 += __shfl_xor_sync(0xffffffffu, n0, 2);
         n1 += __shfl_xor_sync(0xffffffffu, n1, 1);
         n1 += __shfl_xor_sync(0xffffffffu, n1, 2);
+        n0 *= 0.5f;
+        n1 *= 0.5f;
         if (t == 0) {
             sm.nn[m0] = make_float2(n0, n0);
             sm.nn[m1] = make_float2(n1, n1);
@@ -586,7 +592,7 @@ __device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& 
         const float cr = sm.cr[c].x;
         const BmConst k =
             bm_const<__half>(a, grad, img.w, img.h, min(x0 + px, img.w - 1), min(y0 + py, img.h - 1), yb.x);
-        const float kl = fmaxf(-2.f * kLog2e * k.s * k.s, -1e30f), sq = sqrtf(lk);
+        const float kl = 2.f * fmaxf(-2.f * kLog2e * k.s * k.s, -1e30f), sq = sqrtf(lk);
         const float c1 = sq * k.c1, c2 = sq * k.c2;
         sm.k[BK_KL][i] = kl;
         sm.k[BK_BASE][i] = fmaf(kl, sm.nn[c].x, 0.5f * log2f(lk));
