@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(128, 3)
 //     neighbours' |q'|^2 / 2 in FP32. Products of
 //     halves are exact in FP32; the MMA's sum of nine terms does not round each
 //     addition to nearest, but rounds fewer times than a chain of FP32 FMAs: the
-//     exponents' error against float64 is 0.8 of the chain's (rms), the largest
-//     0.6 to 1.0 of it, for coefficients of 0 to 300 times their noise; centring on
+//     exponents' error against float64 is 0.8 to 0.96 of the chain's (rms; the largest
+//     0.6 to 1.0 of it) for coefficients of 0 to 300 times their noise; centring on
 //     the tile-centre pixel's coefficients keeps the cancellation error at FP32
 //     rounding of the local variation of the coefficients;
 //   * a lane gets S of two horizontally adjacent pixels for each of two
@@ -342,7 +342,8 @@ __device__ __forceinline__ u64 as_u64(float2 v) { return pk2(v.x, v.y); }
 
 // The sums of one group (pixel origin gx, gy in the tile). SAFE: positions
 // outside a pixel's window are read as 0, so that a value that is not finite
-// reaches the pixels whose windows hold it and no others. CLAMP: the luma
+// reaches the pixels whose windows hold it (a luma: a patch that holds it, so
+// up to 12 positions away) and no others. CLAMP: the luma
 // exponents may round past their limit.
 template <bool SAFE, bool CLAMP, class Sm>
 __device__ __forceinline__ void bm_group(const Sm& sm, int gx, int gy, u64 (&acc)[3][5]) {
@@ -488,9 +489,14 @@ __device__ __forceinline__ void bm_tile(int x0, int y0, const Plane<__half, 4>& 
     if (tid < 8) {  // centring vector: the coefficients (FP32) of the centre pixel of the
                     // enclosing 32 x 32 tile, so that both tile heights centre and round alike
         const int cx = BX_TX / 2 + 12, cy = 16 + 12 - (y0 % 32);  // luma-tile coordinates
-        float c = 0.f;
-        for (int k = 0; k < 25; k++)
-            c += sm.bsm[k][tid] * __half2float(sm.luma[0][(cy + k / 5 - 2) * BX_LW + cx + k % 5 - 2]);
+        // (any finite centre will do: a luma that is not finite is taken as the one before it,
+        // so that it spoils the positions whose patches hold it and not the whole tile)
+        float c = 0.f, y = 0.f;
+        for (int k = 0; k < 25; k++) {
+            const float v = __half2float(sm.luma[0][(cy + k / 5 - 2) * BX_LW + cx + k % 5 - 2]);
+            y = fabsf(v) < inf ? v : y;
+            c += sm.bsm[k][tid] * y;
+        }
         sm.cen[tid] = c;
     }
     // pcaProjection (demosaic.metal:774-796) fused into the tile producer: the

@@ -23,3 +23,24 @@ def test_coefficients_up_to_the_largest_half(step):
     got = _denoise(ycc, grad, _params(h, w, a=1e4, b=0.0), True)
     assert np.isfinite(got[..., :3]).all() and (got[..., 3] >= 0.99).all()
     assert np.abs(got[..., 0] - level).max() < 400 + 8  # and the half's spacing
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("py,px", [(16, 48), (14, 46), (18, 50), (19, 44), (47, 48)])
+def test_a_luma_value_that_is_not_finite_reaches_twelve_positions(value, py, px):
+    """The patches of the window's positions hold it. Around the centre of a 32 x 32
+    region, (16, 48), it would enter the coefficients' common offset. No sampled
+    patch holds it (columns 43 on of a 55-wide image), so the basis is the clean image's.
+    Beyond its reach the matcher follows the FP32 one within 1.5e-3 (the bound of the
+    comparison with it) as the clean run does."""
+    h, w = 75, 55
+    ycc, grad = _image(h, w, 7)
+    p = _params(h, w)
+    clean = _denoise(ycc, grad, p, True)
+    ycc[py, px, 0] = value
+    got = _denoise(ycc, grad, p, True)
+    y, x = np.mgrid[0:h, 0:w]
+    outside = (np.abs(y - py) > 12) | (np.abs(x - px) > 12)
+    assert outside[(y // 32 == py // 32) & (x // 32 == px // 32)].any()
+    assert np.abs(got[..., :3] - clean[..., :3])[outside].max() < 3e-3
+    assert (np.abs(got[..., 3] - clean[..., 3])[outside] < 0.1 * clean[..., 3][outside]).all()
