@@ -87,16 +87,17 @@ __device__ __forceinline__ Rgb rgb_at(const float* p) {
     return {make_float2(v.x, v.y), v.z};
 }
 
-// Bilinear sample at texel position (sx, sy) in [0, iw - 1] x [0, ih - 1]
-// (iw, ih >= 2), which gives what clamp-to-edge reads give outside: the 2 x 2
-// texels lie inside the frame, the last ones with weight 1 at its far edges.
+// Bilinear sample at texel position (sx, sy) in [0, iw - 1] x [0, ih - 1],
+// which gives what clamp-to-edge reads give outside: on the last column and row
+// both texels are the last one.
 template <class S>
 __device__ __forceinline__ Rgb texel_mix(const FuseFrame& f, float sx, float sy) {
-    const int x0 = min(int(sx), f.iw - 2), y0 = min(int(sy), f.ih - 2);
+    const int x0 = int(sx), y0 = int(sy);
     const float ax = sx - float(x0), ay = sy - float(y0);
     const S* p0 = static_cast<const S*>(f.p) + size_t(unsigned(y0)) * unsigned(f.pitch) + 4 * unsigned(x0);
-    const S* p1 = p0 + unsigned(f.pitch);
-    return mix(mix(rgb_at(p0), rgb_at(p0 + 4), ax), mix(rgb_at(p1), rgb_at(p1 + 4), ax), ay);
+    const S* p1 = p0 + (y0 < f.ih - 1 ? unsigned(f.pitch) : 0u);
+    const unsigned dx = x0 < f.iw - 1 ? 4u : 0u;
+    return mix(mix(rgb_at(p0), rgb_at(p0 + dx), ax), mix(rgb_at(p1), rgb_at(p1 + dx), ax), ay);
 }
 
 // Frame f pull-warped at the N positions (x[k], y[k]) of the reference frame.
