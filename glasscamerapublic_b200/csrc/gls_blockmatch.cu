@@ -655,10 +655,13 @@ static void launch_pair(Plane<__half, 4> img, Plane<__half, 2> grad, const float
     // A level too small for the 296 blocks that fit the chip: each tile's groups
     // are dealt to up to 8 blocks, which stage it alike. 126x94 (24 tiles) 20 us,
     // 43 with a block a tile; 256x192 (96) 34 and 44 (41 over two blocks); taken
-    // further, past the blocks that fit, 52.
+    // further, past the blocks that fit, 52. A batch's streams share the chip, but
+    // seldom more than two are at such a level at once: twelve 256x192 frames on six
+    // streams 761 us, 849 if each level counts as alone, 826 with a block a tile,
+    // 793 if all six count; two frames 272, 272, 329, 286.
     if (split)
         for (const unsigned z : {2u, 3u, 4u, 8u})  // 4, 3, 2, 1 of a tile's 8 rounds of groups
-            if (g.x * g.y * z <= 296) g.z = z;
+            if (g.x * g.y * z * unsigned(a.streams) <= 296u * unsigned(a.streams > 2 ? 2 : a.streams)) g.z = z;
     k_block_match_pair<TY, NP><<<g, BxTile<TY, NP>::THREADS, smem, s>>>(img, grad, basis, out, a);
 }
 

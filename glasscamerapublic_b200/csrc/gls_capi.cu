@@ -375,7 +375,8 @@ static gls_status measure_ycc_nlf(gls_converter* cv, Plane<S, 4> img, float expo
 
 template <class S>
 static gls_status pyramid_run(gls_converter* cv, Pipeline<S>& P, Plane<S, 4> img0, Plane<S, 2> grad0,
-                              const gls_demosaic_params* p, uint32_t flags, cudaStream_t s, bool build_only = false) {
+                              const gls_demosaic_params* p, uint32_t flags, cudaStream_t s, bool build_only = false,
+                              int streams = 1) {
     const int L = p->levels;
     const int W = img0.w, H = img0.h;
     Plane<S, 4> img[GLS_MAX_LEVELS];
@@ -457,6 +458,7 @@ static gls_status pyramid_run(gls_converter* cv, Pipeline<S>& P, Plane<S, 4> img
         ba.gradient_threshold = dp.gradient_threshold;
         ba.lsc = p->lens_shading_correction;
         ba.tensor = flags & GLS_BM_TENSOR;
+        ba.streams = streams;
         if (!is_half<S>::value && cv->keep_nc) {
             GLS_TRY(P.nc[i].ensure(size_t(wi) * hi * sizeof(float)));
             ba.nc_out = static_cast<float*>(P.nc[i].p);
@@ -575,7 +577,7 @@ template <class S>
 static gls_status demosaic_run(gls_converter* cv, const uint16_t* raw, int w, int h, size_t stride_bytes,
                                const gls_demosaic_params* p, uint32_t flags, gls_image_view* out, cudaStream_t s,
                                int slot = 0, const SlotCopies* cp = nullptr, int stage = STAGE_ALL,
-                               Pipeline<S>* use = nullptr) {
+                               Pipeline<S>* use = nullptr, int streams = 1) {
     Pipeline<S>& P = use ? *use
                          : *reinterpret_cast<Pipeline<S>*>(is_half<S>::value ? (void*)&cv->p16s[slot]
                                                                             : (void*)&cv->p32s[slot]);
@@ -703,7 +705,7 @@ static gls_status demosaic_run(gls_converter* cv, const uint16_t* raw, int w, in
             KScope k(cv->prof, KC_DESPECKLE, s);
             launch_despeckle<S>(A, B, p->pyramid_nlf[0].a[0], p->pyramid_nlf[0].b[0], s);
         }
-        GLS_TRY(pyramid_run<S>(cv, P, B, grad, p, flags, s, stage == STAGE_FRONT));
+        GLS_TRY(pyramid_run<S>(cv, P, B, grad, p, flags, s, stage == STAGE_FRONT, streams));
         if (stage == STAGE_FRONT) return GLS_OK;
         final_src = plane<S, 4>(P.den[0], w, h);
         if (cv->calibrate)  // the post-processing reads the measured level-0 model
@@ -1235,9 +1237,9 @@ static gls_status enqueue_batch(gls_converter* conv, gls_frame_desc* frames, int
         const SlotCopies* cp = host_io ? &cps[k] : nullptr;
         result = (flags & GLS_FP16_STORAGE)
                      ? demosaic_run<__half>(conv, f.raw, f.width, f.height, f.raw_stride_bytes, f.params, flags,
-                                            &f.out, conv->slot_stream[k], k, cp)
+                                            &f.out, conv->slot_stream[k], k, cp, STAGE_ALL, nullptr, nslots)
                      : demosaic_run<float>(conv, f.raw, f.width, f.height, f.raw_stride_bytes, f.params, flags,
-                                           &f.out, conv->slot_stream[k], k, cp);
+                                           &f.out, conv->slot_stream[k], k, cp, STAGE_ALL, nullptr, nslots);
     }
     // join (also on error, so the caller's stream orders after whatever was
     // queued), downloads included

@@ -80,6 +80,7 @@ struct BlockMatchArgs {
     float lsc;                    // lens shading correction (0 = off)
     float* nc_out = nullptr;      // FP32 path: the chroma kernel norm per pixel, kept for the adjoint
     bool tensor = false;          // FP16 path: the tensor-core matcher (GLS_BM_TENSOR)
+    int streams = 1;              // slot streams of the call that launch levels side by side
 };
 
 struct SubtractArgs {

@@ -3,6 +3,8 @@ value, and a luma value that is not finite."""
 import numpy as np
 import pytest
 
+import glasscamerapublic_b200 as g
+from glasscamerapublic_b200 import scene
 from test_gpu_block_match import _denoise, _image, _params
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +46,27 @@ def test_a_luma_value_that_is_not_finite_reaches_twelve_positions(value, py, px)
     assert outside[(y // 32 == py // 32) & (x // 32 == px // 32)].any()
     assert np.abs(got[..., :3] - clean[..., :3])[outside].max() < 3e-3
     assert (np.abs(got[..., 3] - clean[..., 3])[outside] < 0.1 * clean[..., 3][outside]).all()
+
+
+@pytest.mark.parametrize("n", [2, 3, 6, 7])
+@pytest.mark.parametrize("w,h,levels", [(64, 48, 1), (256, 192, 3), (322, 250, 3)])
+def test_a_batch_that_splits_its_tiles_less_gives_the_same_bits(n, w, h, levels):
+    """24 to 96 tiles, over 8 to 1 blocks by the number of streams: a frame alone and in a batch."""
+    torch = pytest.importorskip("torch")
+    raws, ps = [], []
+    for k in range(n):
+        wl = scene.Workload("t", w, h, levels=levels, gain=0.8, read=3.0, iso=400, seed=k)
+        raws.append(torch.from_numpy(scene.make_raw(wl)[0].view(np.int16)).cuda())
+        ps.append(scene.make_params(wl))
+    conv = g.RawConverter(0)
+    try:
+        one = [conv.demosaic(r, p, noiseReduction=True, fp16=True, out_fp16=True,
+                             out=torch.empty((h, w, 4), dtype=torch.float16, device="cuda")).clone()
+               for r, p in zip(raws, ps)]
+        outs = [torch.empty((h, w, 4), dtype=torch.float16, device="cuda") for _ in raws]
+        conv.demosaic_batch(raws, ps, outs)
+        torch.cuda.synchronize()
+    finally:
+        conv.close()
+    for a, b in zip(one, outs):
+        assert torch.equal(a, b)
