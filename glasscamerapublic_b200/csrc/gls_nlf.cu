@@ -20,6 +20,8 @@
 // in the reference's order), so the FP32 path's statistics equal the CPU
 // oracle's bit for bit; the fits agree with the oracle's sequential FP64
 // sums to their last bits.
+#include <type_traits>
+
 #include <cmath>
 
 #include "../../include/glscam.h"
@@ -67,8 +69,8 @@ __device__ __forceinline__ float2 sums_of(u64 s) {
     return v;
 }
 
-constexpr int RS_TX = 32, RS_TY = 8, RS_P = 2, RS_ROWS = RS_TY * RS_P;  // half-resolution positions per block
-constexpr int RS_W = 2 * RS_TX + 10, RS_H = 2 * RS_ROWS + 10;             // full-resolution tile: 2x + [-4, 5]
+constexpr int RS_TX = 32, RS_TY = 8;                         // half-resolution positions per block
+constexpr int RS_W = 2 * RS_TX + 10, RS_H = 2 * RS_TY + 10;  // full-resolution tile: 2x + [-4, 5]
 
 // the block's class counts: 8 bits a class in two words, summed over the warp
 // (at most 4 positions a lane), one shared atomic per warp and class
@@ -101,9 +103,10 @@ __device__ __forceinline__ float div_const(float x) {
 
 // PATTERN: the Bayer pattern, so every channel's tap set is known at
 // compile time. Bound by the FMA pipe: 648 additions a position whose order is
-// fixed, in 324 packed instructions; values are staged with their squares, and
-// two vertically adjacent positions share 8 of their 10 rows. 2016x1512
-// positions: 119 us (132 with scalar additions, a position a thread).
+// fixed, in 324 packed instructions; values are staged with their squares.
+// 2016x1512 positions: 109 us (132 with scalar additions, 118 with two
+// vertically adjacent positions a thread, which also leaves small frames'
+// blocks too few: 128x96 positions 7.1 us, 10.1 with two).
 template <class S, int PATTERN>
 __global__ void __launch_bounds__(RS_TX* RS_TY) k_raw_stats(Plane<S, 1> raw, Plane<float, 4> mean,
                                                             Plane<float, 4> var, unsigned* __restrict__ hist) {
@@ -111,47 +114,42 @@ __global__ void __launch_bounds__(RS_TX* RS_TY) k_raw_stats(Plane<S, 1> raw, Pla
     constexpr int OY[4][4] = {{0, 0, 1, 1}, {1, 0, 0, 1}, {0, 1, 1, 0}, {1, 1, 0, 0}};
     __shared__ __align__(16) float2 tile[RS_H][RS_W];
     __shared__ unsigned cls[6];
-    const int X0 = blockIdx.x * RS_TX, Y0 = blockIdx.y * RS_ROWS;  // half-resolution origin
+    const int X0 = blockIdx.x * RS_TX, Y0 = blockIdx.y * RS_TY;  // half-resolution origin
     const int tid = threadIdx.y * RS_TX + threadIdx.x;
     if (tid < 6) cls[tid] = 0;
     for (int ty = threadIdx.y; ty < RS_H; ty += RS_TY)
         for (int tx = threadIdx.x; tx < RS_W; tx += RS_TX)
             tile[ty][tx] = with_square(to_f(*raw.pxc(2 * X0 - 4 + tx, 2 * Y0 - 4 + ty)));
     __syncthreads();
-    const int x = X0 + threadIdx.x, y0 = Y0 + RS_P * threadIdx.y;
+    const int x = X0 + threadIdx.x, y = Y0 + threadIdx.y;
     // the window steps one full-resolution pixel from 2 (x, y) - 4 and
     // reads each channel at its Bayer offset (readRAWQuad): channel c
     // reads the 10 x 10 block's 9 x 9 sub-block at its offset. Each
     // value is loaded once and added to the channels that read it, each
     // channel still in row-major order of its own taps.
-    u64 acc[RS_P][4] = {};
-    const int bx0 = 2 * threadIdx.x, by0 = 2 * RS_P * threadIdx.y;
+    u64 acc[4] = {};
+    const int bx0 = 2 * threadIdx.x, by0 = 2 * threadIdx.y;
 #pragma unroll
-    for (int r = 0; r < 2 * RS_P + 8; r++)
+    for (int r = 0; r < 10; r++)
 #pragma unroll
         for (int v = 0; v < 10; v += 2) {
             const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&tile[by0 + r][bx0 + v]);
 #pragma unroll
             for (int e = 0; e < 2; e++)
 #pragma unroll
-                for (int p = 0; p < RS_P; p++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const int j = r - 2 * p - OY[PATTERN][c], i = v + e - OX[PATTERN][c];
-                        if (j >= 0 && j < 9 && i >= 0 && i < 9) add_to(acc[p][c], e ? q.y : q.x);
-                    }
+                for (int c = 0; c < 4; c++) {
+                    const int j = r - OY[PATTERN][c], i = v + e - OX[PATTERN][c];
+                    if (j >= 0 && j < 9 && i >= 0 && i < 9) add_to(acc[c], e ? q.y : q.x);
+                }
         }
     ClassCount count;
-#pragma unroll
-    for (int p = 0; p < RS_P; p++) {
-        const int y = y0 + p;
-        if (x >= mean.w || y >= mean.h) continue;
+    if (x < mean.w && y < mean.h) {
         f4 m, vv;
         float* mp = &m.x;
         float* vp = &vv.x;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            const float2 t = sums_of(acc[p][c]);
+            const float2 t = sums_of(acc[c]);
             mp[c] = div_const<81>(t.x);
             vp[c] = div_const<81>(__fsub_rn(t.y, div_const<81>(__fmul_rn(t.x, t.x))));
         }
@@ -165,16 +163,16 @@ __global__ void __launch_bounds__(RS_TX* RS_TY) k_raw_stats(Plane<S, 1> raw, Pla
     if (tid < 6 && cls[tid]) atomicAdd(&hist[tid], cls[tid]);
 }
 
-// Four vertically adjacent positions a thread: a row's values, staged with their
-// squares, are read once for the up to four windows that take them. Bound by the FMA pipe
+// YS_P vertically adjacent positions a thread: a row's values, staged with their
+// squares, are read once for the up to YS_P windows that take them. Bound by the FMA pipe
 // (150 additions a position whose order is fixed) and 390 MB of traffic.
-// 4032x3024: 143 us (224 with one position a thread).
-constexpr int YS_TX = 32, YS_TY = 8, YS_P = 4, YS_ROWS = YS_TY * YS_P;
-constexpr int YS_W = YS_TX + 4, YS_H = YS_ROWS + 4;
+// 4032x3024: 143 us (224 with one position a thread and scalar squares).
+constexpr int YS_TX = 32, YS_TY = 8, YS_W = YS_TX + 4;
 
-template <class S>
+template <class S, int YS_P>
 __global__ void __launch_bounds__(YS_TX* YS_TY) k_ycc_stats(Plane<S, 4> img, Plane<float, 4> stats,
                                                             unsigned* __restrict__ hist) {
+    constexpr int YS_ROWS = YS_TY * YS_P, YS_H = YS_ROWS + 4;
     __shared__ float2 tile[3][YS_H][YS_W];
     __shared__ unsigned cls[6];
     const int x0 = blockIdx.x * YS_TX, y0 = blockIdx.y * YS_ROWS;
@@ -498,7 +496,7 @@ template <class S>
 int launch_measure_raw_nlf(Plane<S, 1> scaled, int pattern, Plane<float, 4> mean, Plane<float, 4> var,
                            float exposure, void* scratch, gls_raw_nlf* out, cudaStream_t s) {
     const FitScratch f = fit_scratch(scratch);
-    const dim3 g((mean.w + RS_TX - 1) / RS_TX, (mean.h + RS_ROWS - 1) / RS_ROWS);
+    const dim3 g((mean.w + RS_TX - 1) / RS_TX, (mean.h + RS_TY - 1) / RS_TY);
     const dim3 b(RS_TX, RS_TY);
     switch (pattern) {
         case 0: k_raw_stats<S, 0><<<g, b, 0, s>>>(scaled, mean, var, f.hist); break;
@@ -516,8 +514,19 @@ template <class S>
 int launch_measure_ycc_nlf(Plane<S, 4> img, Plane<float, 4> stats, float exposure, void* scratch,
                            gls_raw_nlf* out, cudaStream_t s) {
     const FitScratch f = fit_scratch(scratch);
-    const dim3 g((img.w + YS_TX - 1) / YS_TX, (img.h + YS_ROWS - 1) / YS_ROWS);
-    k_ycc_stats<S><<<g, dim3(YS_TX, YS_TY), 0, s>>>(img, stats, f.hist);
+    auto run = [&](auto positions) {
+        constexpr int P = decltype(positions)::value;
+        const dim3 g((img.w + YS_TX - 1) / YS_TX, (img.h + YS_TY * P - 1) / (YS_TY * P));
+        k_ycc_stats<S, P><<<g, dim3(YS_TX, YS_TY), 0, s>>>(img, stats, f.hist);
+    };
+    // four positions a thread, or two, where that leaves three blocks for each
+    // of the 148 SMs. us with 1, 2, 4: 256x192 (192 tiles of 32 x 8) 4.8 5.8 8.0,
+    // 400x300 (494) 6.2 6.6 7.9, 640x480 (1200) 10.0 8.9 10.1, 800x600 (1875)
+    // 13.6 11.9 11.8, 2016x1512 65 45 40.
+    const int tiles = ((img.w + YS_TX - 1) / YS_TX) * ((img.h + YS_TY - 1) / YS_TY);
+    if (tiles >= 4 * 444) run(std::integral_constant<int, 4>{});
+    else if (tiles >= 2 * 444) run(std::integral_constant<int, 2>{});
+    else run(std::integral_constant<int, 1>{});
     FitInput in{reinterpret_cast<const float4*>(stats.p), nullptr, stats.w, stats.h, stats.pitch / 4, 0,
                 double(img.w) * double(img.h), exposure};
     launch_fit<false>(in, f, out, s);
