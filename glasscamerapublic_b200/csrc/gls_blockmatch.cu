@@ -96,7 +96,8 @@ __device__ __forceinline__ u64 add2(u64 a, u64 b) {
 // same whatever the tile, so every tile gives the same bits. Differences and
 // chroma terms are packed FP32 (the same roundings in half the instructions),
 // the distance's sum stays a serial chain; ex2.approx.ftz where exp2f only
-// adds the scaling that keeps results below 2^-126.
+// adds the scaling that keeps results below 2^-126, which count for the pixels
+// of bmp_chroma_again alone.
 //
 // What bounds it: two pixels' tap takes 60 cycles of a sub-partition's FMA
 // pipe, 32 of its MUFU and 57 issue slots, and the SM's shared memory serves
@@ -161,6 +162,36 @@ __device__ __forceinline__ void bmp_row(const Smem& sm, int base, int r, const B
     }
 }
 
+// A pixel whose chroma weights are all so small that those below 2^-126, which
+// ex2.approx.ftz drops, count (scales at which the rounding of c times the pixel's
+// own chroma alone reaches the exponent's range): the chroma sums once more by
+// exp2f, which keeps them down to 2^-149.
+template <class Smem>
+__device__ __forceinline__ void bmp_chroma_again(const Smem& sm, int base, int pitch, const BmPlainPix& P,
+                                              float (&s)[5]) {
+    const float kLk = 2.f * 1.4426950408889634f;
+    s[1] = s[2] = s[4] = 0.f;
+#pragma unroll 1
+    for (int k = 0; k < 441; k++) {
+        const int j = k / 21, i = k % 21, q = base + j * pitch + i;
+        const ulonglong2 q0 = sm.pca0[q], q1 = sm.pca1[q];
+        const float4 y = sm.ycc[q];
+        float d[8], e1, e2;
+        upk2(add2(q0.x, P.n[0]), d[0], d[1]);
+        upk2(add2(q0.y, P.n[1]), d[2], d[3]);
+        upk2(add2(q1.x, P.n[2]), d[4], d[5]);
+        upk2(add2(q1.y, P.n[3]), d[6], d[7]);
+        float d2 = d[0] * d[0];
+        for (int c = 1; c < 8; c++) d2 = fmaf(d[c], d[c], d2);
+        const float lw = exp2f(P.kl * d2);
+        upk2(fma2(P.c, pk2(y.x, y.y), P.no), e1, e2);
+        const float wc = sm.spatial[j][i].x * exp2f(-fmaf(kLk * lw, lw, fmaf(e1, e1, e2 * e2)));
+        s[1] = fmaf(wc, y.x, s[1]);
+        s[2] = fmaf(wc, y.y, s[2]);
+        s[4] += wc;
+    }
+}
+
 template <int NP>
 __global__ void __launch_bounds__(128, 3)
     k_block_match_plain(Plane<float, 4> img, Plane<float, 2> grad, Plane<float, 8> pca, Plane<float, 4> out,
@@ -218,7 +249,8 @@ __global__ void __launch_bounds__(128, 3)
 #pragma unroll
     for (int p = 0; p < NP; p++) {
         if (y + p >= out.h) continue;
-        const float(&s)[5] = acc[p];
+        float(&s)[5] = acc[p];
+        if (s[4] < 0x1p-80f) bmp_chroma_again(sm, base + p * T::W, T::W, pix[p], s);
         st4<float>(out.px(x, y + p), f4{s[0] / s[3], s[1] / s[4], s[2] / s[4], s[3]});
         if (a.nc_out) a.nc_out[size_t(y + p) * out.w + x] = s[4];
     }
