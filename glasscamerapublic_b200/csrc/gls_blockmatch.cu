@@ -16,6 +16,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <shared_mutex>
 
 #include "gls_common.cuh"
 #include "gls_kernels.h"
@@ -1172,13 +1173,14 @@ void launch_pyramid_persistent(const PTask* tasks, int n, const PLevel* lv, PCou
 // 16 x 2 takes 2.26 ms a 2016x1512 denoise against 2.09, 48.5 ms a batch of six
 // 12 MP frames against 46.2, 0.385 ms a 256x192 frame against 0.314; 8 x 4 and
 // 4 x 4 hold half the warps (2.61 and 2.55 ms). GLS_BM_TILE=84, 44, 82 or 162
-// in the environment (or 8 / 4 for 84 / 44) fixes the variant. The choices are
-// listed by level size for gls_block_match_tiles.
-static std::mutex g_tile_mu;
+// in the environment (or 8 / 4 for 84 / 44) fixes the variant. The level sizes
+// met are listed for gls_block_match_tiles; host threads that drive converters
+// of their own share the lock.
+static std::shared_mutex g_tile_mu;
 static std::map<std::pair<int, int>, int> g_tile_choice;
 
 int bm_tile_list(int* whty, int max) {
-    std::lock_guard<std::mutex> lk(g_tile_mu);
+    std::shared_lock<std::shared_mutex> lk(g_tile_mu);
     int n = 0;
     for (const auto& kv : g_tile_choice) {
         if (n < max) {
@@ -1192,18 +1194,22 @@ int bm_tile_list(int* whty, int max) {
 }
 
 static int bm_tile_variant(int w, int h) {
-    static const int forced = [] {
+    static const int variant = [] {
         const char* e = std::getenv("GLS_BM_TILE");
         const int v = e ? std::atoi(e) : 0;
         if (v == 8) return 84;  // the thread-row counts of the two NP = 4 variants
         if (v == 4) return 44;
         for (int c : kBmVariants)
             if (v == c) return v;
-        return 0;
+        return 82;
     }();
-    if (forced) return forced;
-    std::lock_guard<std::mutex> lk(g_tile_mu);
-    return g_tile_choice.emplace(std::make_pair(w, h), 82).first->second;
+    {
+        std::shared_lock<std::shared_mutex> lk(g_tile_mu);
+        if (g_tile_choice.count({w, h})) return variant;
+    }
+    std::unique_lock<std::shared_mutex> lk(g_tile_mu);
+    g_tile_choice.emplace(std::make_pair(w, h), variant);
+    return variant;
 }
 
 template <int NP>
