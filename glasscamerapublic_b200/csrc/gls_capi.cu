@@ -441,9 +441,9 @@ static gls_status pyramid_run(gls_converter* cv, Pipeline<S>& P, Plane<S, 4> img
             launch_pca_eigen(part, n_blocks, n_patches, basis + i * 200, status + i, s);
         }
         Plane<S, 8> pcap = plane<S, 8>(P.pca, wi, hi);
-        if (!is_half<S>::value) {  // the FP16 path projects inside the block-matching kernel
+        if constexpr (!is_half<S>::value) {  // the FP16 path projects inside the block-matching kernel
             KScope k(cv->prof, KC_PCA_PROJECT, s);
-            launch_pca_project<S>(layer, basis + i * 200, pcap, s);
+            launch_pca_project(layer, basis + i * 200, pcap, s);
         }
         BlockMatchArgs ba;
         for (int c = 0; c < 3; c++) {
@@ -876,7 +876,7 @@ static gls_status adjoint_run(gls_converter* cv, const gls_demosaic_params* p, c
                                          plane<float, 4>(P.layer, wi, hi), ra, s);
             layer = static_cast<const float*>(P.layer.p);
         }
-        launch_pca_project<float>(Plane<float, 4>{const_cast<float*>(layer), wi, hi, size_t(wi) * 4}, basis,
+        launch_pca_project(Plane<float, 4>{const_cast<float*>(layer), wi, hi, size_t(wi) * 4}, basis,
                                   plane<float, 8>(P.pca, wi, hi), s);
         AdjointLevelArgs la{};
         la.w = wi;

@@ -116,8 +116,8 @@ void launch_pca_cov_rows(Plane<S, 4> img, double* part, int rows, cudaStream_t s
 constexpr int kPcaChunk = 64;
 void launch_pca_eigen(const double* part, int n_blocks, int n_patches, float* basis /*25x8*/, int* status,
                       cudaStream_t s);
-template <class S>
-void launch_pca_project(Plane<S, 4> img, const float* basis, Plane<S, 8> out, cudaStream_t s);
+// FP32 path (the FP16 matcher projects in its tile)
+void launch_pca_project(Plane<float, 4> img, const float* basis, Plane<float, 8> out, cudaStream_t s);
 // FP32 path: reads the projected `pca` plane; FP16 path: projects on tensor
 // cores inside the kernel from `basis` (the pca plane is not used)
 template <class S>

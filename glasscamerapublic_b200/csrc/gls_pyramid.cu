@@ -107,16 +107,15 @@ __global__ void __launch_bounds__(EJ_THREADS) k_pca_eigen(const double* __restri
 // every tap.
 constexpr int PP_W = 32, PP_H = 16;
 
-template <class S>
-__global__ void __launch_bounds__(PP_W* PP_H / 2) k_pca_project(Plane<S, 4> img, const float* __restrict__ basis,
-                                                                Plane<S, 8> out) {
+__global__ void __launch_bounds__(PP_W* PP_H / 2) k_pca_project(Plane<float, 4> img, const float* __restrict__ basis,
+                                                                Plane<float, 8> out) {
     __shared__ float4 b[25][2];
     __shared__ float luma[PP_H + 4][PP_W + 4];
     const int tid = threadIdx.y * PP_W + threadIdx.x;
     const int x0 = blockIdx.x * PP_W, y0 = blockIdx.y * PP_H;
     if (tid < 200) reinterpret_cast<float*>(b)[tid] = basis[tid];
     for (int k = tid; k < (PP_H + 4) * (PP_W + 4); k += PP_W * PP_H / 2)
-        luma[k / (PP_W + 4)][k % (PP_W + 4)] = to_f(*img.pxc(x0 - 2 + k % (PP_W + 4), y0 - 2 + k / (PP_W + 4)));
+        luma[k / (PP_W + 4)][k % (PP_W + 4)] = *img.pxc(x0 - 2 + k % (PP_W + 4), y0 - 2 + k / (PP_W + 4));
     __syncthreads();
     const int x = x0 + threadIdx.x, yt = 2 * threadIdx.y, y = y0 + yt;
     if (x >= img.w) return;
@@ -138,21 +137,9 @@ __global__ void __launch_bounds__(PP_W* PP_H / 2) k_pca_project(Plane<S, 4> img,
 #pragma unroll
     for (int p = 0; p < 2; p++) {
         if (y + p >= img.h) break;
-        S* o = out.px(x, y + p);
-        if constexpr (is_half<S>::value) {
-            uint4 u;
-            __half2 h0 = __floats2half2_rn(acc[p][0], acc[p][1]), h1 = __floats2half2_rn(acc[p][2], acc[p][3]);
-            __half2 h2 = __floats2half2_rn(acc[p][4], acc[p][5]), h3 = __floats2half2_rn(acc[p][6], acc[p][7]);
-            u.x = *reinterpret_cast<uint32_t*>(&h0);
-            u.y = *reinterpret_cast<uint32_t*>(&h1);
-            u.z = *reinterpret_cast<uint32_t*>(&h2);
-            u.w = *reinterpret_cast<uint32_t*>(&h3);
-            *reinterpret_cast<uint4*>(o) = u;
-        } else {
-            float4* o4 = reinterpret_cast<float4*>(o);
-            o4[0] = make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
-            o4[1] = make_float4(acc[p][4], acc[p][5], acc[p][6], acc[p][7]);
-        }
+        float4* o = reinterpret_cast<float4*>(out.px(x, y + p));
+        o[0] = make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
+        o[1] = make_float4(acc[p][4], acc[p][5], acc[p][6], acc[p][7]);
     }
 }
 
@@ -204,9 +191,8 @@ void launch_pca_eigen(const double* part, int n_blocks, int n_patches, float* ba
     k_pca_eigen<<<1, EJ_THREADS, 0, s>>>(part, n_blocks, n_patches, basis, status);
 }
 
-template <class S>
-void launch_pca_project(Plane<S, 4> img, const float* basis, Plane<S, 8> out, cudaStream_t s) {
-    k_pca_project<S><<<grid2(img.w, img.h, dim3(PP_W, PP_H)), dim3(PP_W, PP_H / 2), 0, s>>>(img, basis, out);
+void launch_pca_project(Plane<float, 4> img, const float* basis, Plane<float, 8> out, cudaStream_t s) {
+    k_pca_project<<<grid2(img.w, img.h, dim3(PP_W, PP_H)), dim3(PP_W, PP_H / 2), 0, s>>>(img, basis, out);
 }
 
 // Host FP64 eigen-solve of the same accumulators: the per-level host PCA of
@@ -286,8 +272,7 @@ void host_pca_basis(const double* part, int n_blocks, int n_patches, float* basi
     template void launch_downsample_pair<S>(Plane<S, 4>, Plane<S, 4>, Plane<S, 2>, Plane<S, 2>, cudaStream_t);  \
     template void launch_subtract_noise<S>(Plane<S, 4>, Plane<S, 4>, Plane<S, 4>, Plane<S, 2>, Plane<S, 4>,     \
                                            const SubtractArgs&, cudaStream_t);                                   \
-    template void launch_pca_cov<S>(Plane<S, 4>, double*, cudaStream_t);                                         \
-    template void launch_pca_project<S>(Plane<S, 4>, const float*, Plane<S, 8>, cudaStream_t);
+    template void launch_pca_cov<S>(Plane<S, 4>, double*, cudaStream_t);
 GLS_INST(float)
 GLS_INST(__half)
 #undef GLS_INST
