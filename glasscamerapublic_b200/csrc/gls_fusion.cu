@@ -110,15 +110,15 @@ __device__ __forceinline__ Rgb texel_mix(const FuseFrame& f, float sx, float sy)
 // two divisions' 24. All positions come before the first texel, so the
 // texels of all N samples are in flight together. Other frames (a single row
 // or column, a vanishing line through the image) take registerImage's form.
-// HALF: 1 FP16 frames, 0 FP32 frames, 2 by the frame's own flag.
-template <int N, int HALF>
+// HALF: FP16 frames all; else by the frame's own flag.
+template <int N, bool HALF>
 __device__ __forceinline__ void warp3(const FuseFrame& f, const int (&x)[N], const int (&y)[N], Rgb (&out)[N]) {
     using namespace glsm;
     if (!f.plain) {
 #pragma unroll
         for (int k = 0; k < N; k++) {
             const WarpPos q = warp_pos(f.H, x[k], y[k], f.iw, f.ih);
-            const float4 v = HALF == 1 || (HALF == 2 && f.half)
+            const float4 v = HALF || f.half
                                  ? warp_sample(static_cast<const __half*>(f.p), f.pitch, q)
                                  : warp_sample(static_cast<const float*>(f.p), f.pitch, q);
             out[k] = {make_float2(v.x, v.y), v.z};
@@ -141,7 +141,7 @@ __device__ __forceinline__ void warp3(const FuseFrame& f, const int (&x)[N], con
         sx[k] = fminf(fmaxf(sx[k], 0.f), float(f.iw - 1));
         sy[k] = fminf(fmaxf(sy[k], 0.f), float(f.ih - 1));
     }
-    if (HALF == 1 || (HALF == 2 && f.half)) {
+    if (HALF || f.half) {
 #pragma unroll
         for (int k = 0; k < N; k++) out[k] = texel_mix<__half>(f, sx[k], sy[k]);
     } else {
@@ -208,7 +208,7 @@ __device__ __forceinline__ void down_strip(float rx, float ry, int w, int h, int
 
 // Level 1 of the frames [first, first + gridDim.z) straight from the input
 // frames: the texels are warped as the strip reads them
-template <int HALF>
+template <bool HALF>
 __global__ void __launch_bounds__(256) k_fuse_level1(FuseFrames fr, int first, int W, int H, float4* __restrict__ out,
                                                      size_t out_stride, int w1, int h1, float rx, float ry, int rows) {
     const FuseFrame& f = fr.f[first + blockIdx.z];
@@ -259,7 +259,7 @@ struct FuseLevelArgs {
 // Four blocks an SM (64 registers): 1250 us a burst against 1404 with three
 // at level 0 and 1449 to 1812 with two or four frames unrolled, which cost
 // more occupancy than they add loads in flight.
-template <bool LEVEL0, int HALF, class O>
+template <bool LEVEL0, bool HALF, class O>
 __global__ void __launch_bounds__(256, 4) k_fuse_level(FuseLevelArgs a, FuseFrames fr) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = blockIdx.y * blockDim.y + threadIdx.y;
@@ -394,12 +394,11 @@ static gls_status fuse_frame(const gls_image_view& v, const float* H, int w, int
     return GLS_OK;
 }
 
-// fn(integral constant HALF) for a group's texel format (warp3)
+// fn(bool constant HALF) for a group's texel format (warp3)
 template <class Fn>
-static void by_format(int fmt, Fn&& fn) {
-    if (fmt == 0) fn(std::integral_constant<int, 0>{});
-    else if (fmt == 1) fn(std::integral_constant<int, 1>{});
-    else fn(std::integral_constant<int, 2>{});
+static void by_format(bool half, Fn&& fn) {
+    if (half) fn(std::true_type{});
+    else fn(std::false_type{});
 }
 
 static bool overlaps(const gls_image_view& a, const gls_image_view& b) {
@@ -441,9 +440,8 @@ gls_status fuse_pyramid_impl(FusionScratch* F, const gls_image_view* frames, int
             const int f = k == 0 ? 0 : f0 + k - 1;
             GLS_TRY(fuse_frame(frames[f], f == 0 ? I : H + size_t(f) * 9, W, Hh, fr.f[k]));
         }
-        int halves = 0;
-        for (int k = 0; k < cnt; k++) halves += fr.f[k].half;
-        const int fmt = halves == 0 ? 0 : halves == cnt ? 1 : 2;
+        bool halves = true;
+        for (int k = 0; k < cnt; k++) halves = halves && fr.f[k].half;
         const int k0 = grp == 0 ? 0 : 1;  // the reference's levels are built once
         for (int l = 1; l < levels; l++) {
             const int w = W >> (l - 1), h = Hh >> (l - 1), ow = W >> l, oh = Hh >> l;
@@ -455,7 +453,7 @@ gls_status fuse_pyramid_impl(FusionScratch* F, const gls_image_view* frames, int
             if (l > 1)
                 k_fuse_down<<<gs, blk, 0, s>>>(g(l - 1, k0), px(l - 1), w, h, g(l, k0), px(l), ow, oh, rx, ry, rows);
             else
-                by_format(fmt, [&](auto half) {
+                by_format(halves, [&](auto half) {
                     k_fuse_level1<half.value><<<gs, blk, 0, s>>>(fr, k0, W, Hh, g(1, k0), px(1), ow, oh, rx, ry, rows);
                 });
         }
@@ -483,9 +481,9 @@ gls_status fuse_pyramid_impl(FusionScratch* F, const gls_image_view* frames, int
             if (l > 0) {
                 a.g = g(l, 0);
                 a.g_stride = px(l);
-                k_fuse_level<false, 0, float><<<grid2(a.w, a.h), blk, 0, s>>>(a, fr);
+                k_fuse_level<false, false, float><<<grid2(a.w, a.h), blk, 0, s>>>(a, fr);
             } else {
-                by_format(fmt, [&](auto half) {
+                by_format(halves, [&](auto half) {
                     if (to_caller && out->dtype == GLS_F16)
                         k_fuse_level<true, half.value, __half><<<grid2(a.w, a.h), blk, 0, s>>>(a, fr);
                     else
