@@ -288,11 +288,11 @@ __global__ void __launch_bounds__(128, 3)
 // What bounds it: per tile and warp 8 ex2 (64 cycles of the sub-partition's
 // MUFU), 24 packed FP32 instructions (56 cycles of its FMA pipe) and about 46
 // issue slots, so the MUFU's 3.69 ms per 12 MP frame (5 levels) is the floor.
-// Measured: level 0 of a 2016x1512 image 1.25 ms (1.64 ms with the scalar
+// Measured: level 0 of a 2016x1512 image 1.24 ms (1.64 ms with the scalar
 // distance in packed FP32, four pixels a thread), 83 cycles a tile in the loop
 // (the mix of 8 ex2 and 24 packed FMA alone runs at about 70) and a quarter of
 // the time in staging, projection and the groups' ends; XU pipe 64% busy, issue
-// slots 59%. A 12 MP frame in a 6-frame batch: 8.35 -> 7.71 ms.
+// slots 60%. The five levels of a 12 MP frame: 7.23 -> 6.41 ms.
 constexpr int BX_TX = 32, BX_W = BX_TX + 20;
 // tile variants: TY warps of 32 NP pixels, tiles of 32 x (NP TY) = 32 x 32 or
 // 32 x 16 pixels (bm_tile_variant chooses).
@@ -1225,8 +1225,8 @@ template <class S>
 void launch_block_match(Plane<S, 4> img, Plane<S, 2> grad, Plane<S, 8> pca, const float* basis, Plane<S, 4> out,
                         const BlockMatchArgs& a, cudaStream_t s) {
     if constexpr (is_half<S>::value) {
-        // the packed-FP32 matcher unless the call asks for the tensor-core one
-        // (GLS_BM_TENSOR) or GLS_BM_KERNEL=mma selects it for the process
+        // the default matcher unless the call asks for the one with half-precision
+        // weights (GLS_BM_TENSOR) or GLS_BM_KERNEL=mma selects that for the process
         static const bool mma_env = [] {
             const char* e = std::getenv("GLS_BM_KERNEL");
             return e && std::strcmp(e, "mma") == 0;

@@ -38,7 +38,7 @@ namespace gls {
 // What bounds it, 8 x 4032x3024 FP16 frames, 5 levels, robust weights: the
 // warps' and samplings' arithmetic (issue slots), not HBM: the frames are read
 // twice and level 1 (49 MB a frame) is written once and read once. Measured:
-// 1.25 ms a burst (level 1 0.37 ms at 77% of the issue slots, level 0 0.6 ms,
+// 1.26 ms a burst (level 1 0.38 ms at 78% of the issue slots, level 0 0.6 at 67%,
 // the middle levels' passes 0.11 + 0.2 ms, near HBM / L2 rates), 3.28 ms with
 // a launch per frame and level and every warped image and sum in HBM.
 constexpr int kGroup = 8;

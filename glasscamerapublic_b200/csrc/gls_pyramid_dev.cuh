@@ -205,7 +205,9 @@ __device__ __forceinline__ void pca_cov_row(Plane<S, 4> img, double* __restrict_
 // completed as in select_pca_basis) are written as a row-major 25x8 FP32
 // basis. Every reduction has a fixed order, so the result is deterministic.
 // status receives the number of inverse-iteration solves per vector (2), or
-// -1 when a vector came out non-finite (the basis is then still written).
+// -1 when a vector came out non-finite (the basis is then still written). The
+// eigenvalues of a T that is not finite, or too small to scale, count as 0: the
+// basis is select_pca_basis's unit vectors.
 // Bound by the serial chain on one SM: 29 us (tridiagonalisation 14, Sturm 4.5,
 // inverse iteration to the basis 6, the launch and the row sums 4), 68 us with
 // block-wide phases for every step and the pivot form of the Sturm sequence.

@@ -1742,8 +1742,10 @@ gls_status run_match(gls_surf* s, const std::vector<std::pair<int, int>>& qt, cu
     const int cap = s->pair_cap;
     u64* keys = reinterpret_cast<u64*>(s->matches.p);
     GLS_CUDA(cudaMemsetAsync(keys, 0xff, size_t(J) * cap * sizeof(u64), st));
-    // the train set split so that the blocks fill about eight rounds of two
-    // per SM (148): the last round's idle share stays near a tenth
+    // the train set split so that the blocks of full slots fill about eight rounds
+    // of two per SM (148): the last round's idle share stays near a tenth. The counts
+    // are on the device: blocks past a slot's features leave at once (1076 by 1053
+    // features in slots of 64000: registration 0.54 ms, 0.87 in its former form)
     const int tiles = (s->capacity + MT - 1) / MT;
     const int split = std::clamp(8 * 296 / std::max(tiles * J, 1), 1, std::max(tiles, 1));
     k_match<<<dim3(tiles, J, split), 256, 0, st>>>(mj, cap, kOne2, keys);
