@@ -1014,7 +1014,7 @@ static void launch_mma(Plane<__half, 4> img, Plane<__half, 2> grad, const float*
 // bit-identical), and counts it done:
 //   SN (f, l)  waits for every BM tile of (f, l + 1)  (the coarse denoised image)
 //   COV (f, l) waits for every SN tile of (f, l)      (the layer)
-//   EIG (f, l) waits for every COV row of (f, l)
+//   EIG (f, l) waits for every COV row of (f, l)     (without patches, for its SN tiles)
 //   BM (f, l)  waits for EIG (f, l)                   (the basis; the layer before it)
 // Every task a block waits for comes earlier in the list and was taken by a
 // running block, so the earliest unfinished task can always run: the order
@@ -1094,9 +1094,9 @@ __global__ void __launch_bounds__(BM_THREADS, 2)
                     c = &cnt[tk.lev].sn;
                     target = L.n_sn;
                 }
-            } else if (type == PT_EIG) {
-                c = &cnt[tk.lev].cov;
-                target = L.n_cov;
+            } else if (type == PT_EIG) {  // a level without patches has no row: its layer has to be there for BM
+                c = L.n_cov > 0 || L.n_sn == 0 ? &cnt[tk.lev].cov : &cnt[tk.lev].sn;
+                target = L.n_cov > 0 || L.n_sn == 0 ? L.n_cov : L.n_sn;
             } else {
                 c = &cnt[tk.lev].eig;
                 target = 1;
